@@ -24,7 +24,7 @@ LIB = os.path.join(PKG, "libsilvan_b200.so")
 BIN = os.path.join(PKG, "bin", "silvan")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-SOURCES = ["graph_host.cpp", "gen.cpp", "graph_dev.cu", "sampler.cu", "counters.cu", "engine.cu",
+SOURCES = ["graph_host.cpp", "gen.cpp", "graph_dev.cu", "sampler.cu", "warp_sampler.cu", "counters.cu", "engine.cu",
            "server.cu", "noalloc.cu", "ingest.cu", "components.cu", "brandes.cu", "capi.cu"]
 
 

@@ -186,6 +186,7 @@ int silvan_graph_from_pairs(const uint32_t *pairs, uint64_t count, int directed,
     silvan_graph_s *G = new (std::nothrow) silvan_graph_s();
     if (!G) return SILVAN_E_OOM;
     build_csr(pv, directed != 0, G->g.host);
+    G->g.rows_match = true;
     return finish_graph(G, false, out);
 }
 
@@ -283,6 +284,7 @@ int silvan_graph_from_host(silvan_host_graph_t h, silvan_graph_t *out) {
     if (rc) return rc;
     silvan_graph_s *G = new (std::nothrow) silvan_graph_s();
     if (!G) return SILVAN_E_OOM;
+    G->g.rows_match = true;  // host graphs are built from edge lists
     G->g.host = h->host;
     G->g.cc = h->cc;
     G->g.ncomp = h->ncomp;

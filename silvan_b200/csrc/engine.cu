@@ -319,7 +319,7 @@ int DeviceGraph::upload_raw(uint32_t nn, bool dir, const uint64_t *out_off,
     cudaStream_t cs = nullptr, ks = nullptr;
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     uint64_t *tmp[2] = {nullptr, nullptr};
-    uint32_t *bad = nullptr;
+    uint32_t *bad = nullptr;  // the checks' words: [0] bad rows, [2..9] entry sums
     struct Cleanup {
         cudaStream_t *cs, *ks;
         cudaEvent_t *ev;
@@ -342,7 +342,8 @@ int DeviceGraph::upload_raw(uint32_t nn, bool dir, const uint64_t *out_off,
     CK(cudaStreamCreateWithFlags(&ks, cudaStreamNonBlocking));
     for (int i = 0; i < 4; i++) CK(cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming));
     RK(dmalloc(&tmp[0], (size_t)nn + 1));
-    RK(dmalloc(&bad, 1));
+    RK(dmalloc(&bad, 10));
+    unsigned long long *sums = reinterpret_cast<unsigned long long *>(bad + 2);
     RK(dmalloc(&d_cc, nn));
     RK(dmalloc(&d_out_off, (size_t)nn + 1));
     RK(dmalloc(&d_out_adj, m));
@@ -351,7 +352,7 @@ int DeviceGraph::upload_raw(uint32_t nn, bool dir, const uint64_t *out_off,
         RK(dmalloc(&d_in_off, (size_t)nn + 1));
         RK(dmalloc(&d_in_adj, m_in));
     }
-    CK(cudaMemsetAsync(bad, 0, sizeof(uint32_t), ks));
+    CK(cudaMemsetAsync(bad, 0, 10 * sizeof(uint32_t), ks));
     CK(cudaMemcpyAsync(tmp[0], out_off, sizeof(uint64_t) * (nn + 1), cudaMemcpyHostToDevice, cs));
     CK(cudaEventRecord(ev[0], cs));
     if (dir) {
@@ -379,16 +380,17 @@ int DeviceGraph::upload_raw(uint32_t nn, bool dir, const uint64_t *out_off,
     }
     RK(make_rows(ks));  // waits for the offsets only; the adjacency is still going up
     CK(cudaStreamWaitEvent(ks, ev[2], 0));
-    CK(validate_rows(d_out_off, d_out_adj, nn, bad, ks));
+    CK(validate_rows(d_out_off, d_out_adj, nn, bad, true, !dir, sums, ks));
     if (dir) {
         CK(cudaStreamWaitEvent(ks, ev[3], 0));
-        CK(validate_rows(d_in_off, d_in_adj, nn, bad, ks));
+        CK(validate_rows(d_in_off, d_in_adj, nn, bad, false, true, sums, ks));
     }
-    uint32_t hbad = 0;
-    CK(cudaMemcpyAsync(&hbad, bad, sizeof(uint32_t), cudaMemcpyDeviceToHost, ks));
+    uint32_t hbad[10];
+    CK(cudaMemcpyAsync(hbad, bad, sizeof(hbad), cudaMemcpyDeviceToHost, ks));
     CK(cudaStreamSynchronize(ks));
     CK(cudaStreamSynchronize(cs));
-    if (hbad) {
+    rows_match = std::memcmp(hbad + 2, hbad + 6, 4 * sizeof(uint32_t)) == 0;
+    if (hbad[0]) {
         set_error("CSR rows must hold ascending unique ids < n");
         return SILVAN_E_BADARG;
     }
@@ -447,6 +449,52 @@ void SlotPool::free_all() {
 }
 
 // ---------------------------------------------------------------------------
+// WarpPool
+// ---------------------------------------------------------------------------
+uint32_t WarpPool::cap_for(uint64_t n) { return (uint32_t)std::min<uint64_t>(n, 65536u); }
+
+uint64_t WarpPool::bytes_per_warp(uint64_t cap) {
+    return cap * (sizeof(BallRec) + sizeof(uint2) + 4) + (uint64_t)kWarpMeets * 16 +
+           2ull * kWarpLevels * sizeof(uint2);
+}
+
+int WarpPool::alloc(uint32_t w, uint32_t cap) {
+    free_all();
+    warps = w;
+    s.cap = cap;
+    const uint64_t tot = (uint64_t)w * cap;
+    RK(dmalloc(&s.ball, tot));
+    RK(dmalloc(&s.rows, tot));
+    RK(dmalloc(&s.touched, tot));
+    RK(dmalloc(&s.meet, (uint64_t)w * kWarpMeets));
+    RK(dmalloc(&s.mpre, (uint64_t)w * kWarpMeets));
+    RK(dmalloc(&s.lvl, (uint64_t)w * 2 * kWarpLevels));
+    return SILVAN_OK;
+}
+
+int WarpPool::ensure_list(uint32_t total) {
+    if (total <= list_cap) return SILVAN_OK;
+    uint32_t cap = std::max<uint32_t>(kRoundSamples, list_cap);
+    while (cap < total) cap *= 2;
+    dfree(list);
+    list_cap = 0;
+    RK(dmalloc(&list, (uint64_t)cap * kListClasses));
+    list_cap = cap;
+    return SILVAN_OK;
+}
+
+void WarpPool::free_all() {
+    dfree(s.ball);
+    dfree(s.rows);
+    dfree(s.touched);
+    dfree(s.meet);
+    dfree(s.mpre);
+    dfree(s.lvl);
+    dfree(list);
+    warps = list_cap = 0;
+}
+
+// ---------------------------------------------------------------------------
 // Engine
 // ---------------------------------------------------------------------------
 Engine::~Engine() {
@@ -461,6 +509,7 @@ Engine::~Engine() {
     for (auto &e : ev_)
         if (e) cudaEventDestroy(e);
     slots_.free_all();
+    warps_.free_all();
     device_free(board_mem_);
     if (stream_) cudaStreamDestroy(stream_);
 }
@@ -497,6 +546,18 @@ int Engine::init(uint64_t n_max, uint32_t slots, uint64_t mem_budget) {
         CK(cudaMemGetInfo(&fr, &tot));
         mem_budget = (fr + block_cache().idle_bytes(dev)) / 2;
     }
+    // the warp sampler's state: as many warps as stay resident, within an
+    // eighth of the budget
+    {
+        const uint32_t cap = WarpPool::cap_for(n_max);
+        const uint64_t per = WarpPool::bytes_per_warp(cap);
+        const uint64_t most = (uint64_t)sms * std::max(0, warp_sampler_per_sm());
+        const uint64_t w = std::min<uint64_t>(most, mem_budget / 8 / per);
+        if (w > 0) {
+            RK(warps_.alloc((uint32_t)w, cap));
+            mem_budget -= w * per;
+        }
+    }
     const uint64_t fit = mem_budget / std::max<uint64_t>(SlotPool::bytes_per_slot(n_max), 1);
     if (fit < slots) slots = (uint32_t)std::max<uint64_t>(fit, 1);
     RK(slots_.alloc(slots, n_max, stream_));
@@ -517,9 +578,9 @@ int Engine::ensure_segs(uint32_t nsegs) {
     hfree(h_segs_);
     hfree(h_cursors_);
     RK(dmalloc(&d_segs_, cap));
-    RK(dmalloc(&d_cursors_, cap));
+    RK(dmalloc(&d_cursors_, 2 * (size_t)cap));  // record cursors, then SegDesc::left
     RK(hmalloc(&h_segs_, cap));
-    RK(hmalloc(&h_cursors_, cap));
+    RK(hmalloc(&h_cursors_, 2 * (size_t)cap));
     max_segs_ = cap;
     drop_execs();
     return SILVAN_OK;
@@ -530,11 +591,12 @@ void Engine::drop_execs() {
     execs_.clear();
 }
 
-// The round's two kernels (round_begin + sampler) captured once per (CTA
-// size, grid) and replayed with new segments.
-int Engine::sampler_exec(int block, uint32_t grid, cudaGraphExec_t *out) {
+// The round's kernels (round_begin, the warp sampler when it is used, the CTA
+// sampler) captured once per (CTA size, grid, warp sampler) and replayed with
+// new segments.
+int Engine::sampler_exec(int block, uint32_t grid, bool warp, cudaGraphExec_t *out) {
     for (const Exec &x : execs_)
-        if (x.block == block && x.grid == grid) {
+        if (x.block == block && x.grid == grid && x.warp == warp) {
             *out = x.exec;
             return SILVAN_OK;
         }
@@ -544,11 +606,22 @@ int Engine::sampler_exec(int block, uint32_t grid, cudaGraphExec_t *out) {
     L.hdr = d_hdr_;
     L.segs = d_segs_;
     L.assist = board_;
+    WarpLaunch WL{};
+    if (warp) {
+        L.list = warps_.list;
+        L.list_cap = warps_.list_cap;
+        WL.slots = warps_.s;
+        WL.hdr = d_hdr_;
+        WL.segs = d_segs_;
+        WL.list = warps_.list;
+        WL.list_cap = warps_.list_cap;
+    }
     cudaGraph_t g = nullptr;
     std::lock_guard<std::mutex> cl(capture_mutex());
     CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     cudaError_t e1 = sampler_round_begin(L, max_segs_, stream_);
-    cudaError_t e2 = sampler_launch(L, grid, stream_, block);
+    cudaError_t e2 = warp ? warp_sampler_launch(WL, warps_.warps, stream_) : cudaSuccess;
+    if (e2 == cudaSuccess) e2 = sampler_launch(L, grid, stream_, block);
     cudaError_t e3 = cudaStreamEndCapture(stream_, &g);
     CK(e1);
     CK(e2);
@@ -558,7 +631,7 @@ int Engine::sampler_exec(int block, uint32_t grid, cudaGraphExec_t *out) {
     cudaGraphDestroy(g);
     CK(e4);
     if (execs_.size() >= 16) drop_execs();
-    execs_.push_back(Exec{block, grid, x});
+    execs_.push_back(Exec{block, grid, warp, x});
     *out = x;
     return SILVAN_OK;
 }
@@ -599,6 +672,15 @@ int Engine::choose_block(const std::vector<Job *> &jobs, const std::vector<JobRe
         }
     }
     return best;
+}
+
+// Whether a graph's samples are tried one warp each first: not when the last
+// launch of its class left more than half of them (a 384 x 384 grid leaves 92 %
+// and pays 16 % of the launch for trying; R-MAT 14 to 20 leave 23-31 %).
+bool Engine::try_warps(const DeviceGraph *G) const {
+    if (!G->rows_match) return false;
+    auto it = warp_stats_.find(G->tune_class());
+    return it == warp_stats_.end() || 2 * it->second.left <= it->second.drawn;
 }
 
 void Engine::fair_share(const std::vector<Job *> &jobs, std::vector<JobRequest> &reqs,
@@ -688,6 +770,8 @@ int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> 
             const uint32_t ai = job->params().assist_items;
             S.assist_items = ai == 0u ? kAssistItemsAuto : (ai == 0xffffffffu ? 0u : ai);
         }
+        S.compact = !try_warps(&G) ? 0u : kCompactOn | (G.directed ? 0u : kCompactWindow);
+        S.left = d_cursors_ + max_segs_ + s;
         S.first_sample = r.first_global;
         S.count = r.count;
         S.base = base;
@@ -732,8 +816,23 @@ int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> 
         return SILVAN_E_BADARG;
     }
     const uint32_t grid = std::min<uint32_t>(max_grid_[bi], total);
+    // Samples are first tried one warp each.  Not in the plain form (11 samples
+    // a launch), and not when a job sets its own help-board threshold, which
+    // asks for levels of the CTA sampler.
+    bool warp = false;
+    if (warps_.warps > 0 && jobs[idx[0]]->params().form != SILVAN_FORM_PLAIN) {
+        for (uint32_t i : idx) warp = warp || try_warps(jobs[i]->graph());
+        for (uint32_t i : idx) {
+            const uint32_t ai = jobs[i]->params().assist_items;
+            if (ai != 0u && ai != 0xffffffffu) warp = false;
+        }
+    }
+    if (warp && total > warps_.list_cap) {
+        RK(warps_.ensure_list(total));
+        drop_execs();
+    }
     cudaGraphExec_t exec = nullptr;
-    RK(sampler_exec(block, grid, &exec));
+    RK(sampler_exec(block, grid, warp, &exec));
     for (;;) {
         CK(cudaMemcpyAsync(d_segs_, h_segs_, sizeof(SegDesc) * idx.size(),
                            cudaMemcpyHostToDevice, stream_));
@@ -741,13 +840,17 @@ int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> 
         CK(cudaEventRecord(ev_[0], stream_));
         CK(cudaGraphLaunch(exec, stream_));
         CK(cudaEventRecord(ev_[1], stream_));
-        launches_ += 2;
+        launches_ += warp ? 3 : 2;
         sampler_launches_++;
         CK(cudaMemcpyAsync(h_cursors_, d_cursors_, sizeof(unsigned long long) * idx.size(),
                            cudaMemcpyDeviceToHost, stream_));
+        if (warp)
+            CK(cudaMemcpyAsync(h_cursors_ + max_segs_, d_cursors_ + max_segs_,
+                               sizeof(unsigned long long) * idx.size(), cudaMemcpyDeviceToHost,
+                               stream_));
         CK(cudaMemcpyAsync(h_hdr_, d_hdr_, sizeof(RoundHeader), cudaMemcpyDeviceToHost, stream_));
         CK(cudaStreamSynchronize(stream_));
-        if (h_hdr_->failed > 0 || h_hdr_->finished < total) {
+        if (h_hdr_->failed > 0 || h_hdr_->finished < list_total(h_hdr_->todo)) {
             // A shared level gave up a wait: its records may be left
             // non-neutral and the CTAs that owned them left the launch.  Every
             // slot is re-initialised (the launch has ended, so nothing writes
@@ -758,7 +861,7 @@ int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> 
                                   stream_));
             CK(cudaStreamSynchronize(stream_));
             slot_resets_++;
-            if (h_hdr_->finished < total) {
+            if (h_hdr_->finished < list_total(h_hdr_->todo)) {
                 set_error("sampler round ended with samples undrawn (waits between CTAs "
                           "that share a level gave up)");
                 return SILVAN_E_TIMEOUT;
@@ -774,8 +877,12 @@ int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> 
         // lasts about as long as its slowest sample, so the samples that fit
         // into that time on the other slots cost (almost) nothing extra
         if (h_hdr_->total > 0 && clock_khz_ > 0) {
-            const double cta_ms = (double)h_hdr_->cycles / clock_khz_ / h_hdr_->total;
-            const double tail_ms = (double)h_hdr_->max_cycles / clock_khz_;
+            // the warp sampler's time counts as every CTA's
+            const double warp_ms =
+                warp ? (double)h_hdr_->warp_cycles / clock_khz_ / warps_.warps : 0.0;
+            const double cta_ms =
+                ((double)h_hdr_->cycles / clock_khz_ + warp_ms * grid) / h_hdr_->total;
+            const double tail_ms = (double)h_hdr_->max_cycles / clock_khz_ + warp_ms;
             for (uint32_t i : idx)
                 last_[jobs[i]->graph()->tune_class()] = LastLaunch{cta_ms, tail_ms, ms, grid, total};
             for (uint32_t i : idx) {
@@ -789,6 +896,11 @@ int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> 
                 st.rounds++;
             }
         }
+        if (warp)
+            for (uint32_t s = 0; s < idx.size(); s++)
+                if (h_segs_[s].compact)
+                    warp_stats_[jobs[idx[s]]->graph()->tune_class()] =
+                        WarpStats{reqs[idx[s]].count, h_cursors_[max_segs_ + s]};
         bool redo = false;
         uint32_t base = 0;
         for (uint32_t s = 0; s < idx.size(); s++) {

@@ -22,6 +22,7 @@
 #include "counters.cuh"
 #include "graph_host.h"
 #include "sampler.cuh"
+#include "warp_sampler.cuh"
 #include "silvan.h"
 
 namespace silvan {
@@ -61,6 +62,10 @@ struct DeviceGraph {
     // (start, end) of every row, for the sampler: in_rows aliases out_rows
     // for undirected graphs
     uint2 *d_out_rows = nullptr, *d_in_rows = nullptr;
+    // every row entry has its counterpart in the other direction's rows (true
+    // by construction for graphs built here, checked for uploaded rows): the
+    // warp sampler may draw its samples
+    bool rows_match = false;
     int device = 0;
     // Class of the graph for the sampler's schedule statistics: graphs with
     // the same direction, node count and mean degree (both to a power of 2)
@@ -94,6 +99,20 @@ struct SlotPool {
     void free_all();
     static uint64_t bytes_per_slot(uint64_t n);
     ~SlotPool() { free_all(); }
+};
+
+// State of the warp sampler: per warp a ball of up to `cap` nodes.
+struct WarpPool {
+    WarpSlots s{};
+    uint32_t warps = 0;
+    uint32_t *list = nullptr;  // samples left to the CTA sampler
+    uint32_t list_cap = 0;
+    int alloc(uint32_t warps, uint32_t cap);
+    int ensure_list(uint32_t total);
+    void free_all();
+    static uint64_t bytes_per_warp(uint64_t cap);
+    static uint32_t cap_for(uint64_t n);
+    ~WarpPool() { free_all(); }
 };
 
 struct JobRequest {
@@ -170,17 +189,25 @@ class Engine {
         double cta_ms = 0, tail_ms = 0;
         uint32_t rounds = 0;
     };
+    // Samples of a class of graphs that went through the warp sampler, and those
+    // it left to the CTA sampler, in the last such launch.
+    struct WarpStats {
+        uint64_t drawn = 0, left = 0;
+    };
+    bool try_warps(const DeviceGraph *G) const;
     struct Exec {
         int block;
         uint32_t grid;
+        bool warp;  // the warp sampler first
         cudaGraphExec_t exec;
     };
     int ensure_segs(uint32_t nsegs);
     int choose_block(const std::vector<Job *> &jobs, const std::vector<JobRequest> &reqs,
                      const std::vector<uint32_t> &idx, uint32_t total) const;
-    int sampler_exec(int block, uint32_t grid, cudaGraphExec_t *out);
+    int sampler_exec(int block, uint32_t grid, bool warp, cudaGraphExec_t *out);
     void drop_execs();
     SlotPool slots_;
+    WarpPool warps_;
     void *board_mem_ = nullptr;  // help board of the sampler launches
     AssistBoard board_{};
     cudaStream_t stream_ = nullptr;
@@ -208,6 +235,7 @@ class Engine {
         uint32_t samples = 0;  // drawn by the launch
     };
     std::unordered_map<uint64_t, LastLaunch> last_;  // by tune_class()
+    std::unordered_map<uint64_t, WarpStats> warp_stats_;  // by tune_class()
     // by tune_class(): the samples of the last kHintJobs jobs (see job_hint)
     std::unordered_map<uint64_t, std::deque<uint64_t>> job_total_;
     static constexpr size_t kHintJobs = 8, kHintMin = 4;

@@ -386,6 +386,7 @@ int device_ingest(const char *path, bool directed, DeviceGraph &G, std::string &
     }
     G.m = m;
     G.m_in = m_in;
+    G.rows_match = true;
     CKI(cudaGetDevice(&G.device));
     RKI(G.make_rows(st));
     if (directed) {

@@ -32,7 +32,7 @@
 // is the first hit, t == |pred|-1 the last hit; any other t is resolved by
 // ranking the predecessors (reverse neighbours on the previous level of the
 // same side) by their own queue order.
-#include "sampler.cuh"
+#include "sampler_dev.cuh"
 
 namespace silvan {
 
@@ -44,7 +44,7 @@ constexpr int kItems = 4;        // scan items per lane per tile
 // samples (most of them on sparse directed graphs) cost a fraction of a
 // sample each.  Near the end of a round the CTAs take one at a time.
 constexpr uint32_t kScreen = 8;
-constexpr int kMaxLevels = 256;  // levels per side with recorded bounds
+constexpr int kMaxLevels = 64;  // levels per side with recorded bounds
 
 // Per-CTA-size constants: BLOCK threads serve one sample.  Smaller CTAs put
 // more samples in flight per SM (throughput on many short searches), larger
@@ -53,7 +53,8 @@ template <int BLOCK>
 struct Shape {
     static constexpr int kWarps = BLOCK / 32;
     static constexpr int kTile = BLOCK * kItems;                    // scan items per tile
-    static constexpr int kChunk = BLOCK * 4 < 2048 ? BLOCK * 4 : 2048;  // frontier nodes staged
+    static constexpr int kChunk = BLOCK * 2;                        // frontier nodes staged
+    static constexpr int kHash = 2 * kTile;                         // entries of the tile's table
     static constexpr int kPerThread = kChunk / BLOCK;
     static constexpr int kMinBlocks = 1024 / BLOCK;                 // 64 registers per thread
 };
@@ -63,13 +64,17 @@ struct SamplerSmem {
     static constexpr int kWarps = Shape<BLOCK>::kWarps;
     static constexpr int kChunk = Shape<BLOCK>::kChunk;
     uint32_t f_node[kChunk];
-    uint32_t f_off[kChunk];
+    uint32_t f_off[kChunk];  // a node's first adjacency entry minus its item prefix
     uint32_t f_pre[kChunk + 1];
     unsigned long long f_sig[kChunk];
+    // nodes first reached by the tile in progress, and the lowest item that
+    // reached each (expand_level)
+    uint32_t t_key[Shape<BLOCK>::kHash];
+    uint32_t t_item[Shape<BLOCK>::kHash];
     uint32_t warp_a[kItems * kWarps];  // per (item slot, warp): joins, then their offsets
     uint32_t warp_b[kItems * kWarps];  // per (item slot, warp): meeting edges, offsets
     uint32_t scan_tmp[kWarps + 1];
-    unsigned long long wsum[kWarps];
+    unsigned long long wsum[kWarps + 1];
     unsigned long long rec_base;
     uint32_t sum_new;
     uint32_t pred_hits;
@@ -100,24 +105,10 @@ struct SamplerSmem {
     uint32_t a_leave;   // a shared level of this CTA's sample failed: take no more samples
     // samples taken from the round in a chunk and screened in parallel: the
     // void ones are finished at once, the others wait here
-    uint32_t pend_w[kScreen];
+    // with their endpoints and the draws taken for them
+    uint32_t pend_w[kScreen], pend_u[kScreen], pend_v[kScreen], pend_d[kScreen];
     uint32_t pend_n, pend_i, scr_w0, scr_v;
 };
-
-__device__ __forceinline__ uint32_t lanemask_lt() {
-    uint32_t m;
-    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-    return m;
-}
-
-__device__ __forceinline__ uint32_t draw32(uint64_t seed, uint32_t sample, uint32_t d) {
-    return philox_lo32(seed, sample, kStreamSampler, d);
-}
-
-// x mod m for a 32-bit x and a non-zero 64-bit m: x itself when m >= 2^32.
-__device__ __forceinline__ uint32_t mod_u64(uint32_t x, unsigned long long m) {
-    return (m >> 32) ? x : x % (uint32_t)m;
-}
 
 // Exclusive block scan of one value per thread; returns the block total.
 // tmp needs kWarps + 1 entries.
@@ -151,28 +142,57 @@ __device__ uint32_t block_exclusive_scan(uint32_t v, uint32_t &excl, uint32_t *t
     return total;
 }
 
+// The same of 64-bit values; tmp needs kWarps + 1 entries.
+template <int BLOCK>
+__device__ unsigned long long block_exclusive_scan64(unsigned long long v,
+                                                     unsigned long long &excl,
+                                                     unsigned long long *tmp) {
+    constexpr int kWarps = Shape<BLOCK>::kWarps;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned long long incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    if (lane == 31) tmp[warp] = incl;
+    __syncthreads();
+    // every warp scans the warps' sums itself
+    unsigned long long w = lane < kWarps ? tmp[lane] : 0ull;
+    const unsigned long long own = w;
+#pragma unroll
+    for (int o = 1; o < kWarps; o <<= 1) {
+        const unsigned long long t = __shfl_up_sync(0xffffffffu, w, o);
+        if (lane >= o) w += t;
+    }
+    excl = __shfl_sync(0xffffffffu, w - own, warp) + incl - v;
+    const unsigned long long total = __shfl_sync(0xffffffffu, w, kWarps - 1);
+    return total;
+}
+
+constexpr uint32_t kNoNode = 0xffffffffu;
+
+// The slot of y in the tile's table, inserted when absent.  A tile inserts at
+// most half as many nodes as the table has entries.
+template <int BLOCK>
+__device__ __forceinline__ uint32_t tile_slot(uint32_t *keys, uint32_t y) {
+    constexpr int kLog = BLOCK == 128 ? 10 : BLOCK == 256 ? 11 : BLOCK == 512 ? 12 : 13;
+    static_assert((1 << kLog) == Shape<BLOCK>::kHash, "table size");
+    uint32_t h = (y * 2654435769u) >> (32 - kLog);
+    for (int i = 0; i < Shape<BLOCK>::kHash; i++) {
+        uint32_t k = *reinterpret_cast<volatile uint32_t *>(&keys[h]);
+        if (k == kNoNode) k = atomicCAS(&keys[h], kNoNode, y);
+        if (k == kNoNode || k == y) break;
+        h = (h + 1u) & (uint32_t)(Shape<BLOCK>::kHash - 1);
+    }
+    return h;
+}
+
 // The neutral record (st, cnt, sigma = 0; first = ~0; last = 0) in one
 // 32-byte store: a node record is one sector, written by one transaction.
 __device__ __forceinline__ void rec_reset(NodeRec *r) {
     asm volatile("st.global.v8.b32 [%0], {%1, %1, %1, %1, %2, %2, %1, %1};" ::"l"(r), "r"(0u),
                  "r"(0xffffffffu)
-                 : "memory");
-}
-
-// A whole record in one 32-byte store.
-__device__ __forceinline__ void rec_store(NodeRec *r, uint4 lo, uint4 hi) {
-    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(r), "r"(lo.x),
-                 "r"(lo.y), "r"(lo.z), "r"(lo.w), "r"(hi.x), "r"(hi.y), "r"(hi.z), "r"(hi.w)
-                 : "memory");
-}
-
-// A whole record in one 32-byte load through L2 (the slot is written by this
-// CTA and, for shared levels, by others): words 0-3 and 4-7.
-__device__ __forceinline__ void rec_load(const NodeRec *r, uint4 &lo, uint4 &hi) {
-    asm volatile("ld.global.cg.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(lo.x), "=r"(lo.y), "=r"(lo.z), "=r"(lo.w), "=r"(hi.x), "=r"(hi.y),
-                   "=r"(hi.z), "=r"(hi.w)
-                 : "l"(r)
                  : "memory");
 }
 
@@ -303,6 +323,16 @@ __device__ uint32_t weighted_pred(const SegDesc &A, const NodeRec *rec, uint32_t
     return last;
 }
 
+// A further hit, item g from the predecessor x with sigma sg, on a node of the
+// level in progress whose record is written.
+__device__ __forceinline__ void record_hit(NodeRec *r, uint32_t g, uint32_t x,
+                                           unsigned long long sg) {
+    atomicAdd(&r->cnt, 1u);
+    atomicMax(reinterpret_cast<unsigned long long *>(&r->last),
+              ((unsigned long long)g << 32) | x);
+    atomicAdd(reinterpret_cast<unsigned long long *>(&r->sigma), sg);
+}
+
 // Expands one BFS level of `side` (silvan/src/Sp_sampler.cpp:89-143).
 //
 // The level is latency-bound on deep, narrow searches (a grid's ~200 levels
@@ -331,7 +361,8 @@ __device__ void expand_level(const SegDesc &A, SamplerSmem<BLOCK> &s, NodeRec *r
     uint32_t qend = s.end_q, mend = s.nmeet;
     for (uint32_t c0 = lo; c0 < hi; c0 += kChunk) {
         const uint32_t nc = min((uint32_t)kChunk, hi - c0);
-        // stage the chunk: row starts, degrees (prefix), sigma
+        // stage the chunk: row starts, degrees (prefix), sigma; nodes without
+        // entries are left out (their number is the scan's high word)
         uint32_t xq[kPer], o0[kPer], o1[kPer];
         unsigned long long sg[kPer];
 #pragma unroll
@@ -351,107 +382,113 @@ __device__ void expand_level(const SegDesc &A, SamplerSmem<BLOCK> &s, NodeRec *r
                 sg[i] = __ldcg(&rec[xq[i]].sigma);
             }
         }
-        uint32_t tsum = 0;
+        unsigned long long tsum = 0ull, excl;
+#pragma unroll
+        for (int i = 0; i < kPer; i++)
+            tsum += (unsigned long long)(o1[i] - o0[i]) + (o1[i] != o0[i] ? 1ull << 32 : 0ull);
+        const unsigned long long total = block_exclusive_scan64<BLOCK>(tsum, excl, s.wsum);
+        const uint32_t G = (uint32_t)total, nz = (uint32_t)(total >> 32);
 #pragma unroll
         for (int i = 0; i < kPer; i++) {
-            const uint32_t p = threadIdx.x * kPer + i;
-            if (p < nc) {
-                s.f_node[p] = xq[i];
-                s.f_off[p] = o0[i];
-                s.f_sig[p] = sg[i];
-            }
-            tsum += o1[i] - o0[i];
+            if (o1[i] == o0[i]) continue;
+            const uint32_t p = (uint32_t)(excl >> 32), pre = (uint32_t)excl;
+            s.f_node[p] = xq[i];
+            s.f_off[p] = o0[i] - pre;
+            s.f_pre[p] = pre;
+            s.f_sig[p] = sg[i];
+            excl += (unsigned long long)(o1[i] - o0[i]) + (1ull << 32);
         }
-        uint32_t excl;
-        uint32_t total = block_exclusive_scan<BLOCK>(tsum, excl, s.scan_tmp);
-#pragma unroll
-        for (int i = 0; i < kPer; i++) {
-            const uint32_t p = threadIdx.x * kPer + i;
-            if (p < nc) s.f_pre[p] = excl;
-            excl += o1[i] - o0[i];
-        }
-        if (threadIdx.x == 0) s.f_pre[nc] = total;
         __syncthreads();
-        const uint32_t G = total;
+        uint32_t top = 1u;  // the highest power of two below nz
+        while (top * 2u < nz) top *= 2u;
         for (uint32_t t0 = 0; t0 < G; t0 += kTile) {
             // ---- phase 1 ------------------------------------------------------
             // item slot k of thread tid is item t0 + k * BLOCK + tid: a narrow
-            // level spreads over every warp, and the item order is (k, warp, lane)
-            uint32_t ys[kItems], xs[kItems], code[kItems], li[kItems];
+            // level spreads over every warp, and the item order is (k, warp,
+            // lane).  A warp's 32 items of a slot are consecutive: the node of
+            // the first one is searched by the whole warp (one address, no bank
+            // conflicts), the others follow from the nodes that start within
+            // the 32 items, one bit each.
+            uint32_t ys[kItems], code[kItems], li[kItems];
 #pragma unroll
-            for (int k = 0; k < kItems; k++) {
-                const uint32_t it = t0 + (uint32_t)(k * BLOCK) + threadIdx.x;
-                code[k] = 0;
-                ys[k] = 0;
-                xs[k] = 0;
-                li[k] = 0;
-                if (it < G) {
-                    uint32_t l = 0, h = nc;
-                    while (h - l > 1) {
-                        const uint32_t mid = (l + h) >> 1;
-                        if (s.f_pre[mid] <= it) l = mid;
-                        else h = mid;
-                    }
-                    li[k] = l;
-                    xs[k] = s.f_node[l];
-                    ys[k] = __ldg(&adj[s.f_off[l] + (it - s.f_pre[l])]);
-                    code[k] = 3;  // valid, state not read yet
+            for (int k = 0; k < kItems; k++) li[k] = 0u;
+            for (uint32_t step = top; step > 0u; step >>= 1) {
+#pragma unroll
+                for (int k = 0; k < kItems; k++) {
+                    const uint32_t first = t0 + (uint32_t)(k * BLOCK + warp * 32);
+                    const uint32_t n = li[k] + step;
+                    if (n < nz && s.f_pre[n] <= first) li[k] = n;
                 }
             }
-            // the neighbour's state, and its row (needed only if it joins; loaded
-            // now so that the join does not wait for it)
-            uint32_t sty[kItems], dg[kItems];
 #pragma unroll
             for (int k = 0; k < kItems; k++) {
-                sty[k] = code[k] ? __ldcg(&rec[ys[k]].st) : 0u;
-                const uint2 r = code[k] ? __ldg(&rows[ys[k]]) : make_uint2(0u, 0u);
-                dg[k] = r.y - r.x;
+                const uint32_t first = t0 + (uint32_t)(k * BLOCK + warp * 32);
+                const uint32_t n = li[k] + 1u + (uint32_t)lane;
+                const uint32_t at = n < nz ? s.f_pre[n] - first : 32u;
+                const uint32_t m = __reduce_or_sync(0xffffffffu, at < 32u ? 1u << at : 0u);
+                li[k] += __popc(m & (lanemask_lt() * 2u + 1u));
+                const uint32_t it = first + (uint32_t)lane;
+                code[k] = it < G ? 3u : 0u;  // valid, state not read yet
+                ys[k] = it < G ? __ldg(&adj[s.f_off[li[k]] + it]) : 0u;
             }
+            uint32_t sty[kItems], dg[kItems];
+#pragma unroll
+            for (int k = 0; k < kItems; k++) sty[k] = code[k] ? __ldcg(&rec[ys[k]].st) : 0u;
 #pragma unroll
             for (int k = 0; k < kItems; k++) {
                 if (!code[k]) continue;
-                // unvisited, or joined earlier in this level: a new-level hit
-                // (the joining hit marks the node in phase 2)
-                if (sty[k] == 0u || sty[k] == new_st) code[k] = 1;
+                // unvisited; joined earlier in this level; of the other side
+                if (sty[k] == 0u) code[k] = 1;
+                else if (sty[k] == new_st) code[k] = 4;
                 else if (st_side(sty[k]) != side) code[k] = 2;
                 else code[k] = 0;
             }
-            // Phase 1 records only the hit count and the smallest key.  Most
-            // new nodes of a level have a single hit (about 1.2 hits per node
-            // on R-MAT); their whole record is then written by the joining
-            // hit with one store in phase 2, and only nodes with several hits
-            // get the sigma and last-key atomics.  The tiles of a level run
-            // one after another on this CTA, separated by a barrier after
-            // each tile's stores, so a later tile's hits find the record
-            // complete and add to it.
+            // the rows of the unvisited ones (needed by the hits that join)
 #pragma unroll
             for (int k = 0; k < kItems; k++) {
-                if (code[k] != 1) continue;
-                const uint32_t it = t0 + (uint32_t)(k * BLOCK) + threadIdx.x;
-                const unsigned long long key = ((unsigned long long)(gbase + it) << 32) | xs[k];
-                NodeRec *r = &rec[ys[k]];
-                atomicMin(reinterpret_cast<unsigned long long *>(&r->first), key);
-                atomicAdd(&r->cnt, 1u);
+                dg[k] = 0u;
+                if (code[k] == 1) {
+                    const uint2 r = __ldg(&rows[ys[k]]);
+                    dg[k] = r.y - r.x;
+                }
+            }
+            // The nodes that this tile reaches first go through a table in
+            // shared memory, which finds the lowest item of each: the joining
+            // hit, which writes the whole record with one store.  Nodes joined
+            // by an earlier tile have their record (a barrier separates the
+            // tiles' stores), and take every other hit as three additions.
+            // Scattered accesses are what the level pays for (one a cycle and
+            // SM; L1TEX was 78 % busy): per hit one probe, and per joined node
+            // one row and one store here, where a minimum, a count and a second
+            // look at the record per hit made it five.  R-MAT 14 top-10: the
+            // sampler takes 10.3 ms instead of 11.4; a 256 x 256 grid 33.3 ms
+            // instead of 36.0 per 65,536 samples (ncu).
+            uint32_t ts[kItems];
+#pragma unroll
+            for (int k = 0; k < kItems; k++) {
+                ts[k] = 0u;
+                if (code[k] == 1) {
+                    ts[k] = tile_slot<BLOCK>(s.t_key, ys[k]);
+                    atomicMin(&s.t_item[ts[k]], (uint32_t)(k * BLOCK) + threadIdx.x);
+                } else if (code[k] == 4) {
+                    const uint32_t it = t0 + (uint32_t)(k * BLOCK) + threadIdx.x;
+                    record_hit(&rec[ys[k]], gbase + it, s.f_node[li[k]], s.f_sig[li[k]]);
+                    hits_local++;
+                    code[k] = 0;
+                }
+                __syncwarp();
             }
             __syncthreads();
             // ---- phase 2: ordered compaction of joins and meeting edges -------
-            uint32_t single = 0;  // bit k: item k is the node's only hit so far
+            bool again = false;  // a hit on a node that another item joins
 #pragma unroll
             for (int k = 0; k < kItems; k++) {
                 if (code[k] != 1) continue;
-                uint4 lo4, hi4;
-                rec_load(&rec[ys[k]], lo4, hi4);
-                const uint32_t it = t0 + (uint32_t)(k * BLOCK) + threadIdx.x;
-                const unsigned long long key = ((unsigned long long)(gbase + it) << 32) | xs[k];
                 hits_local++;
-                if (lo4.y > 1u) {  // several hits: sigma and the last key by atomics
-                    NodeRec *r = &rec[ys[k]];
-                    atomicMax(reinterpret_cast<unsigned long long *>(&r->last), key);
-                    atomicAdd(reinterpret_cast<unsigned long long *>(&r->sigma), s.f_sig[li[k]]);
-                } else {
-                    single |= 1u << k;
+                if (s.t_item[ts[k]] != (uint32_t)(k * BLOCK) + threadIdx.x) {
+                    code[k] = 4;
+                    again = true;
                 }
-                if (hi4.y != gbase + it) code[k] = 0;  // not the joining hit
             }
             uint32_t rn[kItems], rm[kItems];
 #pragma unroll
@@ -465,7 +502,8 @@ __device__ void expand_level(const SegDesc &A, SamplerSmem<BLOCK> &s, NodeRec *r
                     s.warp_b[k * kWarps + warp] = __popc(bm);
                 }
             }
-            __syncthreads();
+            __syncwarp();
+            const bool shared_nodes = __syncthreads_or(again) != 0;
             // Every warp turns the counts into exclusive offsets over
             // (k, warp) in item order (the same sums in every warp) and picks
             // its own kItems of them by shuffles; no second barrier.  The next
@@ -531,26 +569,35 @@ __device__ void expand_level(const SegDesc &A, SamplerSmem<BLOCK> &s, NodeRec *r
                 if (code[k] == 1) {
                     const uint32_t y = ys[k];
                     queue[oa[k] + rn[k]] = y;
-                    if (single & (1u << k)) {
-                        // the only hit: st, cnt = 1, sigma, first = last = key
-                        const uint32_t it = t0 + (uint32_t)(k * BLOCK) + threadIdx.x;
-                        const unsigned long long sg = s.f_sig[li[k]];
-                        rec_store(&rec[y], make_uint4(new_st, 1u, (uint32_t)sg, (uint32_t)(sg >> 32)),
-                                  make_uint4(xs[k], gbase + it, xs[k], gbase + it));
-                    } else {
-                        rec[y].st = new_st;
-                    }
+                    // the joining hit: st, cnt = 1, sigma, first = last = key
+                    const uint32_t it = t0 + (uint32_t)(k * BLOCK) + threadIdx.x;
+                    const uint32_t x = s.f_node[li[k]];
+                    const unsigned long long sg = s.f_sig[li[k]];
+                    rec_store(&rec[y],
+                              make_uint4(new_st, 1u, (uint32_t)sg, (uint32_t)(sg >> 32)),
+                              make_uint4(x, gbase + it, x, gbase + it));
                     sum_local += dg[k];
+                    // its table entry is free for the next tile
+                    s.t_key[ts[k]] = kNoNode;
+                    s.t_item[ts[k]] = 0xffffffffu;
                 } else if (code[k] == 2) {
                     const uint32_t pos = ob[k] + rm[k];
-                    if (pos < kMeetCap) meet[pos] = make_uint2(xs[k], ys[k]);
+                    if (pos < kMeetCap) meet[pos] = make_uint2(s.f_node[li[k]], ys[k]);
                 }
             }
-            // A single-hit record is written whole by its joining hit; a hit
-            // of the next tile on the same node must find it written and add
-            // to it, not be overwritten by it (the chunk's last tile has the
-            // barrier below).
-            if (t0 + (uint32_t)kTile < G) __syncthreads();
+            // A record is written whole by its joining hit; the other hits, of
+            // this tile and of the next, must find it written and add to it
+            // (the chunk's last tile has the barrier below).
+            __syncwarp();
+            if (shared_nodes || t0 + (uint32_t)kTile < G) __syncthreads();
+            if (shared_nodes) {
+#pragma unroll
+                for (int k = 0; k < kItems; k++)
+                    if (code[k] == 4)
+                        record_hit(&rec[ys[k]], gbase + t0 + (uint32_t)(k * BLOCK) + threadIdx.x,
+                                   s.f_node[li[k]], s.f_sig[li[k]]);
+                __syncwarp();
+            }
         }
         if (threadIdx.x == 0) s.vis += G;
         gbase += G;
@@ -609,12 +656,6 @@ __device__ void expand_level(const SegDesc &A, SamplerSmem<BLOCK> &s, NodeRec *r
 // ---------------------------------------------------------------------------
 constexpr uint32_t kAssistPolls = 1u << 18;  // board polls of a CTA without samples
 constexpr unsigned long long kCntMask = (1ull << 31) - 1u;
-
-__device__ __forceinline__ uint32_t ld_acquire_u32(const uint32_t *p) {
-    uint32_t v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
 
 __device__ __forceinline__ void st_release_u32(uint32_t *p, uint32_t v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
@@ -793,7 +834,8 @@ __device__ __forceinline__ int32_t post_level(const SamplerLaunch &L, SamplerSme
     // and the last samples' levels are what the launch waits for.
     uint32_t thr = A.assist_items;
     if (thr == kAssistItemsAuto) {
-        const bool draining = ld_acquire_u32(&L.hdr->work) >= L.hdr->total;
+        if (items < 16u * (uint32_t)Shape<BLOCK>::kTile) return -1;
+        const bool draining = ld_acquire_u32(&L.hdr->work) >= list_total(L.hdr->todo);
         thr = (draining ? 16u : 32u) * (uint32_t)Shape<BLOCK>::kTile;
     }
     if (items < thr || F > L.assist.node_cap ||
@@ -1208,29 +1250,19 @@ __device__ void help_entry(const SamplerLaunch &L, SamplerSmem<BLOCK> &s, uint32
     }
 }
 
-// Segment owning work index w: the last segment whose base is <= w.
-__device__ __forceinline__ uint32_t segment_of(const SegDesc *segs, uint32_t nsegs, uint32_t w) {
-    uint32_t l = 0, h = nsegs;
-    while (h - l > 1) {
-        const uint32_t mid = (l + h) >> 1;
-        if (segs[mid].base <= w) l = mid;
-        else h = mid;
-    }
-    return l;
-}
-
 // Takes the next kScreen work indices of the round (one while few are left)
 // and screens them, one thread each: endpoints (Sp_sampler.cpp:46,58-60)
 // and the void test (:62-74).  A void sample's outputs are written here; the
-// others are queued in s.pend_w for the full sampler.  Sets s.a_drained when
-// the round has no sample left.
+// others are queued in s.pend_w for the full sampler.  The samples the warp
+// sampler left are taken one at a time (they are the long ones) and have been
+// screened.  Sets s.a_drained when the round has no sample left.
 template <int BLOCK>
 __device__ __noinline__ void screen_chunk(const SamplerLaunch &L, SamplerSmem<BLOCK> &s,
                                           uint32_t total, uint32_t nsegs) {
     if (threadIdx.x == 0) {
         const uint32_t taken = ld_acquire_u32(&L.hdr->work);
         const uint32_t left = taken < total ? total - taken : 0u;
-        const uint32_t v = left > 2u * kScreen * gridDim.x ? kScreen : 1u;
+        const uint32_t v = !L.list && left > 2u * kScreen * gridDim.x ? kScreen : 1u;
         const uint32_t w0 = atomicAdd(&L.hdr->work, v);
         s.scr_w0 = w0;
         s.scr_v = v;
@@ -1243,15 +1275,21 @@ __device__ __noinline__ void screen_chunk(const SamplerLaunch &L, SamplerSmem<BL
     bool is_void = false;
     if (threadIdx.x < s.scr_v && w < total) {
         const long long t0 = clock64();
-        const SegDesc &A = L.segs[segment_of(L.segs, nsegs, w)];
-        const uint32_t gidx = A.first_sample + (w - A.base);
+        uint32_t wi = w;
+        if (L.list) {  // work index w counts through the classes
+            uint32_t c = 0;
+            while (c < kListClasses - 1 && wi >= L.hdr->todo[c]) wi -= L.hdr->todo[c++];
+            wi = __ldcg(&L.list[(uint64_t)c * L.list_cap + wi]);
+        }
+        const SegDesc &A = L.segs[segment_of(L.segs, nsegs, wi)];
+        const uint32_t gidx = A.first_sample + (wi - A.base);
         uint32_t d = 0;
         uint32_t v = draw32(A.seed, gidx, d++) % A.n;
         const uint32_t u = draw32(A.seed, gidx, d++) % A.n;
         while (u == v) v = draw32(A.seed, gidx, d++) % A.n;
-        is_void = A.directed ? (A.cc[u] < A.cc[v]) : (A.cc[u] != A.cc[v]);
+        is_void = !L.list && (A.directed ? (A.cc[u] < A.cc[v]) : (A.cc[u] != A.cc[v]));
         if (is_void) {
-            const uint32_t sl = w - A.base;
+            const uint32_t sl = wi - A.base;
             A.out_pl[sl] = 0;
             A.out_np[sl] = 0;
             A.out_vis[sl] = 0;
@@ -1260,21 +1298,24 @@ __device__ __noinline__ void screen_chunk(const SamplerLaunch &L, SamplerSmem<BL
             A.out_pred[sl] = 0;
             atomicAdd(&L.hdr->cycles, (unsigned long long)(clock64() - t0));
         } else {
-            s.pend_w[atomicAdd(&s.pend_n, 1u)] = w;
+            const uint32_t i = atomicAdd(&s.pend_n, 1u);
+            s.pend_w[i] = wi;
+            s.pend_u[i] = u;
+            s.pend_v[i] = v;
+            s.pend_d[i] = d;
         }
     }
+    __syncwarp();
     const uint32_t nv = __syncthreads_count(is_void);
-    if (threadIdx.x == 0 && nv) {
-        __threadfence();
-        atomicAdd(&L.hdr->finished, nv);
-    }
+    if (threadIdx.x == 0 && nv) atomicAdd(&L.hdr->finished, nv);
     __syncthreads();
 }
 
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK, Shape<BLOCK>::kMinBlocks) sampler_kernel(SamplerLaunch L) {
     constexpr int kWarps = Shape<BLOCK>::kWarps;
-    __shared__ SamplerSmem<BLOCK> s;
+    extern __shared__ __align__(16) unsigned char sampler_smem[];
+    SamplerSmem<BLOCK> &s = *reinterpret_cast<SamplerSmem<BLOCK> *>(sampler_smem);
     const uint32_t slot = blockIdx.x;
     const uint64_t base = (uint64_t)slot * L.slots.stride;
     NodeRec *rec = L.slots.rec + base;
@@ -1283,7 +1324,7 @@ __global__ void __launch_bounds__(BLOCK, Shape<BLOCK>::kMinBlocks) sampler_kerne
     uint32_t *touched = L.slots.touched + base;
     uint2 *meet = L.slots.meet + (uint64_t)slot * kMeetCap;
     uint64_t *mpre = L.slots.meet_pre + (uint64_t)slot * kMeetCap;
-    const uint32_t total = L.hdr->total;
+    const uint32_t total = list_total(L.hdr->todo);
     const uint32_t nsegs = L.hdr->nsegs;
     const SegDesc &A = s.seg;
 
@@ -1300,15 +1341,30 @@ __global__ void __launch_bounds__(BLOCK, Shape<BLOCK>::kMinBlocks) sampler_kerne
         s.a_leave = 0;
     }
     if (threadIdx.x == 0) s.pend_n = s.pend_i = 0;
+    for (uint32_t i = threadIdx.x; i < (uint32_t)Shape<BLOCK>::kHash; i += BLOCK) {
+        s.t_key[i] = kNoNode;
+        s.t_item[i] = 0xffffffffu;
+    }
+    uint32_t seg = 0xffffffffu;
     for (;;) {
         if (threadIdx.x == 0) {
             int32_t pick = L.assist.entries != nullptr && !s.a_leave
                                ? join_entry<BLOCK>(L, s, blockIdx.x)
                                : -1;
             if (pick < 0 && !s.a_leave && s.pend_i < s.pend_n) {
-                const uint32_t w = s.pend_w[s.pend_i++];
+                const uint32_t i = s.pend_i++;
+                const uint32_t w = s.pend_w[i];
                 s.work = w;
                 s.sample = segment_of(L.segs, nsegs, w);
+                s.u = s.pend_u[i];
+                s.v = s.pend_v[i];
+                s.draw_base = s.pend_d[i];
+                s.status = 0;
+                s.vis = 0;
+                s.nmeet = 0;
+                s.ntouched = 0;
+                s.nonmono = 0;
+                s.pred_hits = 0;
                 pick = -3;  // a sample
             } else if (pick < 0 && !s.a_drained && !s.a_leave) {
                 pick = -4;  // take the next chunk of the round
@@ -1361,52 +1417,20 @@ __global__ void __launch_bounds__(BLOCK, Shape<BLOCK>::kMinBlocks) sampler_kerne
             screen_chunk<BLOCK>(L, s, total, nsegs);
             continue;
         }
-        {
-            const uint32_t *src = reinterpret_cast<const uint32_t *>(&L.segs[s.sample]);
+        if (s.sample != seg) {  // the segment in s.seg is another one
+            seg = s.sample;
+            __syncthreads();
+            const uint32_t *src = reinterpret_cast<const uint32_t *>(&L.segs[seg]);
             uint32_t *dst = reinterpret_cast<uint32_t *>(&s.seg);
             for (uint32_t i = threadIdx.x; i < sizeof(SegDesc) / 4; i += BLOCK)
                 dst[i] = src[i];
+            __syncthreads();
         }
-        __syncthreads();
         const uint32_t sl = s.work - A.base;
         const uint32_t gidx = A.first_sample + sl;
         const long long t_sample0 = clock64();
-
-        // ---- endpoints (Sp_sampler.cpp:46,58-60) and void test (:62-74) -------
-        if (threadIdx.x == 0) {
-            uint32_t d = 0;
-            uint32_t v = draw32(A.seed, gidx, d++) % A.n;
-            uint32_t u = draw32(A.seed, gidx, d++) % A.n;
-            while (u == v) v = draw32(A.seed, gidx, d++) % A.n;
-            s.u = u;
-            s.v = v;
-            s.draw_base = d;
-            s.status = 0;
-            s.vis = 0;
-            s.nmeet = 0;
-            s.ntouched = 0;
-            s.nonmono = 0;
-            s.pred_hits = 0;
-        }
-        __syncthreads();
+        // endpoints drawn and screened (screen_chunk)
         const uint32_t u = s.u, v = s.v;
-        const bool void_cc = A.directed ? (A.cc[u] < A.cc[v]) : (A.cc[u] != A.cc[v]);
-        if (void_cc) {
-            if (threadIdx.x == 0) {
-                A.out_pl[sl] = 0;
-                A.out_np[sl] = 0;
-                A.out_vis[sl] = 0;
-                A.out_status[sl] = 0;
-                A.out_ball[sl] = 0;
-                A.out_pred[sl] = 0;
-                const unsigned long long dc = (unsigned long long)(clock64() - t_sample0);
-                atomicAdd(&L.hdr->cycles, dc);
-                atomicMax(&L.hdr->max_cycles, dc);
-                atomicAdd(&L.hdr->finished, 1u);
-            }
-            __syncthreads();
-            continue;
-        }
         if (threadIdx.x == 0) {
             rec[u].st = st_make(kSideU, 0);
             rec[u].sigma = 1;
@@ -1688,7 +1712,6 @@ __global__ void __launch_bounds__(BLOCK, Shape<BLOCK>::kMinBlocks) sampler_kerne
             atomicAdd(&L.hdr->cycles, dc);
             atomicMax(&L.hdr->max_cycles, dc);
             if (s.a_leave) atomicAdd(&L.hdr->failed, 1u);
-            __threadfence();
             atomicAdd(&L.hdr->finished, 1u);
         }
         __syncthreads();
@@ -1697,9 +1720,16 @@ __global__ void __launch_bounds__(BLOCK, Shape<BLOCK>::kMinBlocks) sampler_kerne
 
 __global__ void round_begin_kernel(SamplerLaunch L, uint32_t max_segs) {
     const uint32_t ns = min(L.hdr->nsegs, max_segs);
-    for (uint32_t i = threadIdx.x; i < ns; i += blockDim.x) *L.segs[i].rec_cursor = 0ull;
+    for (uint32_t i = threadIdx.x; i < ns; i += blockDim.x) {
+        *L.segs[i].rec_cursor = 0ull;
+        if (L.segs[i].left) *L.segs[i].left = 0ull;
+    }
     if (threadIdx.x == 0) {
         L.hdr->work = 0;
+        for (int c = 0; c < kListClasses; c++)
+            L.hdr->todo[c] = L.list || c < kListClasses - 1 ? 0u : L.hdr->total;
+        L.hdr->warp_work = 0;
+        L.hdr->warp_cycles = 0;
         L.hdr->finished = 0;
         L.hdr->open_mask = 0;
         L.hdr->assisted = 0;
@@ -1774,27 +1804,46 @@ cudaError_t sampler_round_begin(const SamplerLaunch &L, uint32_t max_segs, cudaS
     return cudaGetLastError();
 }
 
-cudaError_t sampler_launch(const SamplerLaunch &L, uint32_t grid, cudaStream_t stream, int block) {
-    if (grid == 0) return cudaSuccess;
+namespace {
+// The kernel of a CTA size, its shared memory opted into on the current
+// device (the attribute is per device; setting it again is harmless).
+struct SizedKernel {
+    const void *fn;
+    size_t smem;
+};
+
+template <int BLOCK>
+cudaError_t sized_kernel(SizedKernel *k) {
+    *k = {reinterpret_cast<const void *>(sampler_kernel<BLOCK>), sizeof(SamplerSmem<BLOCK>)};
+    return cudaFuncSetAttribute(sampler_kernel<BLOCK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)k->smem);
+}
+
+cudaError_t sized_kernel(int block, SizedKernel *k) {
     switch (block) {
-    case 128: sampler_kernel<128><<<grid, 128, 0, stream>>>(L); break;
-    case 256: sampler_kernel<256><<<grid, 256, 0, stream>>>(L); break;
-    case 512: sampler_kernel<512><<<grid, 512, 0, stream>>>(L); break;
-    case 1024: sampler_kernel<1024><<<grid, 1024, 0, stream>>>(L); break;
+    case 128: return sized_kernel<128>(k);
+    case 256: return sized_kernel<256>(k);
+    case 512: return sized_kernel<512>(k);
+    case 1024: return sized_kernel<1024>(k);
     default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
+}
+}  // namespace
+
+cudaError_t sampler_launch(const SamplerLaunch &L, uint32_t grid, cudaStream_t stream, int block) {
+    if (grid == 0) return cudaSuccess;
+    SizedKernel k{};
+    const cudaError_t e = sized_kernel(block, &k);
+    if (e != cudaSuccess) return e;
+    void *args[] = {const_cast<SamplerLaunch *>(&L)};
+    return cudaLaunchKernel(k.fn, dim3(grid), dim3((unsigned)block), args, k.smem, stream);
 }
 
 int sampler_max_ctas_per_sm(int block) {
     int n = 0;
-    switch (block) {
-    case 128: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, sampler_kernel<128>, 128, 0); break;
-    case 256: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, sampler_kernel<256>, 256, 0); break;
-    case 512: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, sampler_kernel<512>, 512, 0); break;
-    case 1024: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, sampler_kernel<1024>, 1024, 0); break;
-    default: break;
-    }
+    SizedKernel k{};
+    if (sized_kernel(block, &k) != cudaSuccess) return 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k.fn, block, k.smem);
     return n;
 }
 

@@ -50,8 +50,15 @@ struct SegDesc {
     // BFS levels of at least this many adjacency entries are posted on the
     // launch's help board (0 = never, kAssistItemsAuto = the default threshold)
     uint32_t assist_items;
-    uint32_t pad;
+    uint32_t compact;  // kCompactOn, kCompactWindow
+    unsigned long long *left;  // samples the warp sampler left (nullptr: not counted)
 };
+
+// SegDesc::compact.  On: the samples may be drawn one warp each
+// (warp_sampler.cuh); the rows of the two directions must match (u -> v on a
+// forward row exactly when u is on v's reverse row).  Window: the graph is
+// undirected, so such a search may forget its older levels.
+constexpr uint32_t kCompactOn = 1u, kCompactWindow = 2u;
 
 // Launch-invariant description of a sampler round; the segments live in
 // device memory so that the launch can be captured in a CUDA graph once and
@@ -71,8 +78,20 @@ struct RoundHeader {
     // to its slot, and the host re-initialises every slot after the launch
     uint32_t failed;
     uint32_t wait_polls;  // polls of each bounded help-board wait (set by the host)
-    uint32_t pad;
+    uint32_t warp_work;   // next work index of the warp sampler (zeroed by round_begin)
+    // samples the CTA sampler draws: all of them (in the last class), or those
+    // the warp sampler listed, by class (set by round_begin, raised by the
+    // warp sampler)
+    uint32_t todo[4];
+    unsigned long long warp_cycles;  // SM cycles of its warps (zeroed by round_begin)
 };
+
+// Classes of the samples the warp sampler lists, the largest first: a launch
+// lasts until its longest samples are done, so they start first.
+constexpr int kListClasses = 4;
+SILVAN_HD uint32_t list_total(const uint32_t *todo) {
+    return todo[0] + todo[1] + todo[2] + todo[3];
+}
 
 // Polls of a bounded help-board wait unless the caller asks otherwise
 // (silvan_params_t::wait_polls): at >= 64 ns per poll well above any real
@@ -137,6 +156,9 @@ struct SamplerLaunch {
     RoundHeader *hdr;
     const SegDesc *segs;
     AssistBoard assist;  // zero: every level is expanded by its own CTA
+    // work indices left by the warp sampler, list_cap per class (nullptr: all)
+    const uint32_t *list;
+    uint32_t list_cap;
 };
 
 // Neutral records for `slots` slots of n nodes.

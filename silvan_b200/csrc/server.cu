@@ -190,6 +190,7 @@ struct Server {
             }
             const double t_adm = now_seconds();
             r->graph.reset(new DeviceGraph());
+            r->graph->rows_match = true;  // host graphs are built from edge lists
             r->graph->host = std::move(r->host);
             r->graph->cc = std::move(r->cc);
             r->graph->ncomp = r->ncomp;
