@@ -264,7 +264,26 @@ int DeviceGraph::upload() {
     }
     RK(dmalloc(&d_cc, n));
     CK(cudaMemcpy(d_cc, cc.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice));
+    if (!rows_match) RK(check_rows(cudaStreamLegacy));
     return make_rows(cudaStreamLegacy);
+}
+
+int DeviceGraph::check_rows(cudaStream_t stream) {
+    uint32_t *w = nullptr;  // [0] bad rows, [2..9] entry sums
+    uint32_t h[10];
+    RK(dmalloc(&w, 10));
+    unsigned long long *sums = reinterpret_cast<unsigned long long *>(w + 2);
+    cudaError_t e = cudaMemsetAsync(w, 0, sizeof(h), stream);
+    if (e == cudaSuccess)
+        e = validate_rows(d_out_off, d_out_adj, n, w, true, !directed, sums, stream);
+    if (e == cudaSuccess && directed)
+        e = validate_rows(d_in_off, d_in_adj, n, w, false, true, sums, stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h, w, sizeof(h), cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    dfree(w);
+    CK(e);
+    rows_match = h[0] == 0 && std::memcmp(h + 2, h + 6, 4 * sizeof(uint32_t)) == 0;
+    return SILVAN_OK;
 }
 
 int DeviceGraph::make_rows(cudaStream_t stream) {

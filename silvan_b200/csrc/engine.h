@@ -81,6 +81,8 @@ struct DeviceGraph {
     // d_out_rows / d_in_rows from the device offsets (every upload path ends
     // with it)
     int make_rows(cudaStream_t stream);
+    // rows_match of the device rows
+    int check_rows(cudaStream_t stream);
     // Components and diameter bound on the host copy, then the component
     // ids to the device (after a device ingest filled d_* and `host`).
     int finish_from_host_copy();
