@@ -6,13 +6,13 @@
 //   approx[u] += x;  emp_wimpy_vars[u] += x * x;
 //   mcrade[u][j] = (int64)((double)mcrade[u][j] + sign_j * x)   (truncation)
 // With num_paths > 1 the additions are not associative, so a node's updates
-// must be applied in sample order.  A round's records are grouped by node
-// (count, bucket space, scatter), each node's group is put in sample order
-// (by rank: compares for groups of <= 32, a bitmap of the sub-round's samples
-// otherwise) and the group is folded sequentially by one warp: lanes 0..24
-// each carry one Monte Carlo trial, lane 25 approx, lane 26 the wimpy
-// variance.  Different nodes are independent, so the only serial work is per
-// node.
+// must be applied in sample order.  A draw's records are grouped by node once
+// (count, bucket space, scatter) and each node's group put in sample order (by
+// rank: compares for groups of <= 32, a bitmap of the draw's samples
+// otherwise).  A commit round then folds each group's entries of its sample
+// range sequentially, one warp a node: lanes 0..24 each carry one Monte Carlo
+// trial, lane 25 approx, lane 26 the wimpy variance.  Different nodes are
+// independent, so the only serial work is per node.
 #include <algorithm>
 #include <cstddef>
 #include <cfloat>
@@ -27,20 +27,23 @@ namespace silvan {
 namespace {
 
 // ---------------------------------------------------------------------------
-// One commit round as a single cooperative kernel.  Its phases are separated
-// by grid-wide barriers (every CTA is resident: cooperative launch):
-//   A  per sample the Rademacher signs (pass 2) and 1 / num_paths; records
-//      counted per node and the touched nodes listed
+// A draw's records by node as a single cooperative kernel.  Its phases are
+// separated by grid-wide barriers (every CTA is resident: cooperative launch):
+//   A  per sample the Rademacher signs and 1 / num_paths; records counted per
+//      node and the touched nodes listed
 //   B  bucket space of every touched node taken from a cursor (warp
 //      aggregated), the scatter cursors, the list of buckets of more than
 //      32 entries
 //   C  records scattered into their nodes' buckets
-//   D  the sub-round's 1 / num_paths and signs staged in shared memory;
-//      the large buckets on warp 0 of each CTA (claimed from a cursor), the
-//      small ones on the other warps (fixed assignment); the round's scalar
-//      sums; cursors zeroed
+//   D  each bucket put in sample order, its entries with their factor and
+//      signs: the huge buckets by whole CTAs (claimed from a cursor), then the
+//      others one warp each (fixed assignment); cursors zeroed
 // Each barrier is bounded: a CTA that waits longer than kBarrierPolls polls
 // records SILVAN_E_TIMEOUT in the job's error word and leaves the kernel.
+//
+// Once per draw, not per commit round: an estimation commits a draw in about
+// ten rounds, and the three barriers and their phases were more than half of
+// each (R-MAT 20, a million nodes: 14 of 31-35 us; a round is now 27 and the draw 55 once).
 // ---------------------------------------------------------------------------
 constexpr int kCommitThreads = 1024;
 constexpr uint32_t kBarrierPolls = 1u << 22;  // far above any real wait (microseconds)
@@ -88,18 +91,16 @@ __device__ bool grid_barrier(uint32_t *bar) {
 __device__ void bucket_count(const RoundBuffers &rb, const ApplyArgs &a) {
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
     const uint32_t lane = threadIdx.x & 31;
-    // per sample, one warp: the Rademacher signs (pass 2; lane j draws trial
-    // j, as rademacher_mask does) and 1 / num_paths, the factor every record
-    // of the sample is multiplied by (Probabilistic.cpp:502)
-    for (uint32_t s = a.lo + (tid >> 5); s < a.hi; s += nth >> 5) {
-        if (a.pass == 2) {
-            bool plus = false;
-            if (lane < (uint32_t)kTrials)
-                plus = philox_lo32(a.seed, a.first_sample + s, kStreamRademacher, lane) %
-                           100000000u >= 50000000u;
-            const uint32_t m = __ballot_sync(0xffffffffu, plus);
-            if (lane == 0) rb.signs[s] = m;
-        }
+    // per sample, one warp: the Rademacher signs (read in pass 2; lane j draws
+    // trial j, as rademacher_mask does) and 1 / num_paths, the factor every
+    // record of the sample is multiplied by (Probabilistic.cpp:502)
+    for (uint32_t s = tid >> 5; s < a.count; s += nth >> 5) {
+        bool plus = false;
+        if (lane < (uint32_t)kTrials)
+            plus = philox_lo32(a.seed, a.first_sample + s, kStreamRademacher, lane) %
+                       100000000u >= 50000000u;
+        const uint32_t m = __ballot_sync(0xffffffffu, plus);
+        if (lane == 0) rb.signs[s] = m;
         if (lane == 31) rb.inv_np[s] = __ddiv_rn(1.0, (double)rb.np[s]);
     }
     const uint32_t R = round_records(rb, a);
@@ -113,8 +114,7 @@ __device__ void bucket_count(const RoundBuffers &rb, const ApplyArgs &a) {
         if (i < R) {
             const PathRec r = rb.recs[i];
             node = r.node;
-            if (r.sample >= a.lo && r.sample < a.hi)
-                first = atomicAdd(&rb.node_cnt[r.node], 1u) == 0u;
+            first = atomicAdd(&rb.node_cnt[r.node], 1u) == 0u;
         }
         const uint32_t m = __ballot_sync(0xffffffffu, first);
         if (m) {
@@ -159,6 +159,7 @@ __device__ void bucket_alloc(const RoundBuffers &rb, uint32_t T) {
             rb.bucket_len[t] = b;
             rb.node_cnt[node] = off;  // becomes the scatter cursor
             if (large) rb.large[lbase + __popc(lm & ((1u << lane) - 1u))] = t;
+            if (b > kHugeBucket) rb.huge[atomicAdd(rb.n_touched + 7, 1u)] = t;
         }
     }
 }
@@ -168,19 +169,225 @@ __device__ void bucket_scatter(const RoundBuffers &rb, const ApplyArgs &a) {
     const uint32_t R = round_records(rb, a);
     for (uint32_t i = tid; i < R; i += nth) {
         PathRec r = rb.recs[i];
-        if (r.sample < a.lo || r.sample >= a.hi) continue;
         uint32_t pos = atomicAdd(&rb.node_cnt[r.node], 1u);
         rb.entries[pos] = ((unsigned long long)r.sample << 32) | r.count;
     }
 }
+
+// An entry of a bucket as the rounds read it.  inv_np and signs were written by
+// other CTAs before the last grid barrier.
+__device__ __forceinline__ DrawEntry draw_entry(const RoundBuffers &rb, unsigned long long e) {
+    const uint32_t sl = (uint32_t)(e >> 32);
+    DrawEntry d;
+    d.x = __dmul_rn((double)(uint32_t)e, __ldcg(&rb.inv_np[sl]));
+    d.signs = __ldcg(&rb.signs[sl]);
+    d.sample = sl;
+    return d;
+}
+
+// Shared memory of phase D: the samples of the CTA's huge bucket and the set
+// bits before each word; then each warp's bucket.
+struct OrderSmem {
+    union {
+        struct {
+            uint32_t bits[kDrawSamples / 32];
+            uint32_t wpre[kDrawSamples / 32];
+        } h;
+        uint32_t sample[kCommitThreads / 32][kHugeBucket];
+    };
+    uint32_t scan[33];
+    uint32_t li;
+};
+
+// Buckets of more than kHugeBucket entries, by whole CTAs.  The entries of a
+// bucket are distinct samples of the draw (a node is on a sample's path map
+// once), so their order is the rank of each sample in a bitmap of the draw:
+// set one bit per entry, prefix-count the bits per word, and each entry goes
+// to its rank (linear in the bucket; no comparison sort).  (One warp a bucket
+// took 400 us for a hub's 60,000 entries.)
+__device__ void order_huge(const RoundBuffers &rb, const JobCounters &jc, uint32_t S,
+                           OrderSmem &sm) {
+    constexpr uint32_t kWords = kDrawSamples / 32, kPer = kWords / kCommitThreads;
+    const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const uint32_t NH = __ldcg(rb.n_touched + 7);
+    for (;;) {
+        if (threadIdx.x == 0) sm.li = atomicAdd(rb.n_touched + 5, 1u);
+        for (uint32_t w = threadIdx.x; w < kWords; w += kCommitThreads) sm.h.bits[w] = 0u;
+        __syncthreads();
+        const uint32_t li = sm.li;
+        if (li >= NH) break;
+        const uint32_t t = __ldcg(&rb.huge[li]);
+        const uint32_t b0 = __ldcg(&rb.bucket_off[t]), b = __ldcg(&rb.bucket_len[t]);
+        if (b > S) {  // more entries than samples: not a bucket of distinct samples
+            if (threadIdx.x == 0) {
+                atomicCAS(&jc.sc->error, 0, SILVAN_E_STATE);
+                rb.bucket_span[t] = make_uint2(0u, 0u);
+            }
+            __syncthreads();
+            continue;
+        }
+        for (uint32_t i = threadIdx.x; i < b; i += kCommitThreads) {
+            const uint32_t sidx = (uint32_t)(__ldcg(&rb.entries[b0 + i]) >> 32);
+            if (sidx < S) atomicOr(&sm.h.bits[sidx >> 5], 1u << (sidx & 31));
+            else atomicCAS(&jc.sc->error, 0, SILVAN_E_STATE);
+        }
+        __syncwarp();
+        __syncthreads();
+        // exclusive prefix of the words' bit counts (thread L owns words
+        // [L kPer, (L + 1) kPer))
+        uint32_t c = 0;
+#pragma unroll
+        for (uint32_t w = 0; w < kPer; w++) c += __popc(sm.h.bits[threadIdx.x * kPer + w]);
+        uint32_t incl = c;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
+            if ((int)lane >= o) incl += u;
+        }
+        if (lane == 31) sm.scan[wib] = incl;
+        __syncthreads();
+        uint32_t ws = sm.scan[lane];
+        const uint32_t own = ws;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, ws, o);
+            if ((int)lane >= o) ws += u;
+        }
+        uint32_t run = __shfl_sync(0xffffffffu, ws - own, (int)wib) + incl - c;
+#pragma unroll
+        for (uint32_t w = 0; w < kPer; w++) {
+            sm.h.wpre[threadIdx.x * kPer + w] = run;
+            run += __popc(sm.h.bits[threadIdx.x * kPer + w]);
+        }
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < b; i += kCommitThreads) {
+            const unsigned long long e = __ldcg(&rb.entries[b0 + i]);
+            const uint32_t sidx = (uint32_t)(e >> 32);
+            if (sidx >= S) continue;
+            const uint32_t w = sidx >> 5;
+            const uint32_t r = sm.h.wpre[w] + __popc(sm.h.bits[w] & ((1u << (sidx & 31)) - 1u));
+            rb.sorted[b0 + r] = draw_entry(rb, e);
+            uint32_t *span = reinterpret_cast<uint32_t *>(&rb.bucket_span[t]);
+            if (r == 0u) span[0] = sidx;
+            if (r == b - 1u) span[1] = sidx;
+        }
+        __syncwarp();
+        __syncthreads();
+    }
+    __syncthreads();
+}
+
+// The other buckets, touched node t on warp t mod (warps of the grid), no
+// cursor.  A bucket holds distinct samples, so each entry's position in sample
+// order is the number of entries with a smaller sample: compares across the
+// warp up to 32 entries, over a copy in shared memory up to kHugeBucket.
+__device__ void order_others(const RoundBuffers &rb, uint32_t T, OrderSmem &sm) {
+    constexpr uint32_t kKeys = kHugeBucket / 32;
+    const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const uint32_t stride = gridDim.x * (kCommitThreads / 32);
+    uint32_t *mine = sm.sample[wib];
+    for (uint32_t t = blockIdx.x * (kCommitThreads / 32) + wib; t < T; t += stride) {
+        const uint32_t b = __ldcg(&rb.bucket_len[t]);
+        if (b > kHugeBucket) continue;
+        const uint32_t off = __ldcg(&rb.bucket_off[t]);
+        uint32_t *span = reinterpret_cast<uint32_t *>(&rb.bucket_span[t]);
+        if (b <= 32u) {
+            const unsigned long long key = lane < b ? __ldcg(&rb.entries[off + lane]) : ~0ull;
+            uint32_t rank = 0;
+            for (uint32_t j = 0; j < b; j++)
+                rank += __shfl_sync(0xffffffffu, key, (int)j) < key;
+            if (lane < b) {
+                rb.sorted[off + rank] = draw_entry(rb, key);
+                if (rank == 0u) span[0] = (uint32_t)(key >> 32);
+                if (rank == b - 1u) span[1] = (uint32_t)(key >> 32);
+            }
+        } else {
+            unsigned long long key[kKeys];
+            uint32_t rank[kKeys];
+#pragma unroll
+            for (uint32_t r = 0; r < kKeys; r++) {
+                const uint32_t i = r * 32u + lane;
+                key[r] = i < b ? __ldcg(&rb.entries[off + i]) : ~0ull;
+                mine[i] = (uint32_t)(key[r] >> 32);
+                rank[r] = 0u;
+            }
+            __syncwarp();
+            for (uint32_t j = 0; j < b; j++) {
+                const uint32_t o = mine[j];
+#pragma unroll
+                for (uint32_t r = 0; r < kKeys; r++) rank[r] += o < (uint32_t)(key[r] >> 32);
+            }
+#pragma unroll
+            for (uint32_t r = 0; r < kKeys; r++) {
+                if (r * 32u + lane >= b) continue;
+                rb.sorted[off + rank[r]] = draw_entry(rb, key[r]);
+                if (rank[r] == 0u) span[0] = (uint32_t)(key[r] >> 32);
+                if (rank[r] == b - 1u) span[1] = (uint32_t)(key[r] >> 32);
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// The last CTA out keeps the draw's counts and zeroes the control words.
+__device__ void prepare_exit(const RoundBuffers &rb) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(rb.n_touched + 6, 1u) == gridDim.x - 1) {
+            rb.n_touched[8] = __ldcg(&rb.n_touched[0]);
+            rb.n_touched[9] = __ldcg(&rb.n_touched[1]);
+            rb.n_touched[0] = 0u;
+            rb.n_touched[1] = 0u;
+            rb.n_touched[4] = 0u;
+            rb.n_touched[5] = 0u;
+            rb.n_touched[6] = 0u;
+            rb.n_touched[7] = 0u;
+            __threadfence();
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kCommitThreads, 1) prepare_draw_kernel(const ApplyState st) {
+    __shared__ OrderSmem sm;
+    const RoundBuffers &rb = st.rb;
+    const JobCounters &jc = st.jc;
+    const ApplyArgs &a = st.a;
+    uint32_t *bar = rb.n_touched + 2;
+    bucket_count(rb, a);
+    if (!grid_barrier(bar)) goto timeout;
+    {
+        const uint32_t T = __ldcg(rb.n_touched);
+        bucket_alloc(rb, T);
+        if (!grid_barrier(bar)) goto timeout;
+        bucket_scatter(rb, a);
+        if (!grid_barrier(bar)) goto timeout;
+        order_huge(rb, jc, a.count, sm);
+        order_others(rb, T, sm);
+        // the scatter cursors back to zero for the next draw
+        for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < T;
+             t += gridDim.x * blockDim.x)
+            rb.node_cnt[rb.touched[t]] = 0;
+    }
+    prepare_exit(rb);
+    return;
+timeout:
+    if (threadIdx.x == 0) atomicCAS(&jc.sc->error, 0, SILVAN_E_TIMEOUT);
+    prepare_exit(rb);
+}
+
+// ---------------------------------------------------------------------------
+// A commit round.
+// ---------------------------------------------------------------------------
+
 // Sequential fold of one node's contributions in sample order.  Every lane
 // runs the same instruction stream and carries one chain: lane j < 25 trial j
 // of mcrade, lane 25 approx (and the top-k crossing), lane 26 the wimpy
-// variance; lanes 27..31 repeat lane 25's chain and store nothing.  The chains
-// advance together, one entry per step.  The entries are staged 32 at a time
-// in the warp's scratch: x = count * (1 / num_paths), the sample's signs and
-// its round-local index.
-struct FoldScratch {
+// variance; lanes 27..31 repeat lane 25's chain and store nothing.  The entries
+// are staged 32 at a time in the warp's scratch: x = count * (1 / num_paths),
+// the sample's signs and its round-local index.  A hub's chain bounds a round:
+// the sums advance one dependent addition (8 cycles) per entry; the trials,
+// whose chain (add, truncate) takes 24, advance four entries a step where 32
+// are there (fold_full): R-MAT 14, 60,000 entries of one node: 740 -> 540 us.
+struct alignas(16) FoldScratch {
     double x[32];
     uint32_t signs[32];
     uint32_t sample[32];
@@ -229,258 +436,313 @@ __device__ __forceinline__ void fold_flush(const JobCounters &jc, FoldScratch &f
     __syncwarp();
 }
 
-// A node's counters as its fold starts, loaded before its entries are put in
-// order so that the loads overlap that work.
+// A node's counters as its fold starts.
 struct NodeState {
     double v;         // this lane's chain
     uint32_t lu0;     // last_upd before the round
+    uint32_t lu;      // and after the entries so far (0: no addition)
     bool crossed;     // lane 25: approx reached 3 in an earlier round (top-k pass 1)
 };
 
-// A journaled round also saves them at the node's touched position t.
-__device__ __forceinline__ NodeState fold_load(const JobCounters &jc, const RoundJournal &jr,
-                                               const ApplyArgs &a, uint32_t node, uint32_t t) {
+__device__ __forceinline__ NodeState fold_load(const JobCounters &jc, const ApplyArgs &a,
+                                               uint32_t node) {
     const int lane = threadIdx.x & 31;
-    NodeState s{0.0, 0u, true};
+    NodeState s{0.0, 0u, 0u, true};
     if (lane < kTrials) {
-        if (a.pass == 2) {
-            const long long m = jc.mcrade[(uint64_t)node * kTrials + lane];
-            if (a.journal) jr.mcrade[(uint64_t)t * kTrials + lane] = m;
-            s.v = (double)m;
-        }
+        if (a.pass == 2) s.v = (double)jc.mcrade[(uint64_t)node * kTrials + lane];
     } else if (lane == 26) {
         s.v = jc.wimpy[node];
-        if (a.journal) jr.wimpy[t] = s.v;
     } else {
         s.v = jc.approx[node];
         if (lane == 25) {
             s.lu0 = jc.last_upd[node];
             if (a.track_cross) s.crossed = jc.cross_flag[node] != 0;
-            if (a.journal) {
-                jr.approx[t] = s.v;
-                jr.last_upd[t] = s.lu0;
-            }
         }
     }
     return s;
 }
 
-// Folds the node's b entries; fill(r0) has lane i stage entry r0 + i (when
-// below b) in the scratch.
-template <typename Fill>
-__device__ void fold_node(const JobCounters &jc, const ApplyArgs &a, uint32_t node, uint32_t b,
-                          NodeState st, Fill fill, FoldScratch &fs) {
+// A journaled round saves them at the node's touched position t.
+__device__ __forceinline__ void fold_journal(const RoundJournal &jr, const ApplyArgs &a,
+                                             uint32_t t, const NodeState &s) {
+    const int lane = threadIdx.x & 31;
+    if (lane < kTrials) {
+        if (a.pass == 2) jr.mcrade[(uint64_t)t * kTrials + lane] = (long long)s.v;
+    } else if (lane == 25) {
+        jr.approx[t] = s.v;
+        jr.last_upd[t] = s.lu0;
+    } else if (lane == 26) {
+        jr.wimpy[t] = s.v;
+    } else if (lane == 27) {
+        jr.stamp[t] = a.stamp;
+    }
+}
+
+// One entry of a trial: m + s x for an integer m, truncated towards zero, where
+// x is 1 (c) or far enough from 0 and 1 that m + s x is no integer after
+// rounding.  With x == 1 the entry moves m by its sign.  With 0 < x < 1, m + x
+// is m for m >= 0 and m + 1 for m < 0, and m - x is m for m <= 0 and m - 1 for
+// m > 0: a step towards zero or none.
+__host__ __device__ constexpr int32_t trial_step(int32_t m, bool plus, bool c) {
+    if (plus) return c || m < 0 ? m + 1 : m;
+    return c || m > 0 ? m - 1 : m;
+}
+
+// Four entries at once: what they add to m depends on their c and plus bits and
+// on m only from -4 to 4 (further out no step reaches zero before the last),
+// so the additions for these nine m are four bits each of one word.
+struct TrialSteps {
+    unsigned long long v[256];  // c bits << 4 | plus bits
+};
+constexpr TrialSteps make_trial_steps() {
+    TrialSteps t{};
+    for (int i = 0; i < 256; i++) {
+        unsigned long long w = 0;
+        for (int s = -4; s <= 4; s++) {
+            int32_t m = s;
+            for (int k = 0; k < 4; k++) m = trial_step(m, (i >> k) & 1, (i >> (4 + k)) & 1);
+            w |= (unsigned long long)((m - s) & 15) << (4 * (s + 4));
+        }
+        t.v[i] = w;
+    }
+    return t;
+}
+__device__ const TrialSteps g_trial_steps = make_trial_steps();
+
+// Folds 32 staged entries, each x either 1 (its bit in c) or at least 2^-25 away
+// from 0 and 1, with fewer than 2^26 samples so far: m + s x then lies at least
+// 2^-26 from an integer, more than it can be rounded by, and trial_step holds.
+// All loads come before the two chains, which every lane runs side by side:
+// 32 additions of 8 cycles, 8 steps of the trials of about 30.
+__device__ __forceinline__ void fold_full(const JobCounters &jc, const ApplyArgs &a,
+                                          uint32_t node, uint32_t c, NodeState &st,
+                                          const FoldScratch &fs) {
     const int lane = threadIdx.x & 31;
     const bool mc = lane < kTrials, wv = lane == 26;
-    double v = st.v;
-    uint32_t lu = 0;
-    for (uint32_t r0 = 0; r0 < b; r0 += 32) {
-        fill(r0);
-        __syncwarp();
-        const bool pos = r0 + lane < b && fs.x[lane] > 0.;
-        const uint32_t pm = __ballot_sync(0xffffffffu, pos);
-        // 1 + global index of the last sample that adds to approx
-        if (pm) lu = a.first_sample + fs.sample[31 - __clz(pm)] + 1u;
-        const uint32_t kmax = min(32u, b - r0);
-        int kc = -1;
-#pragma unroll 4
-        for (uint32_t k = 0; k < kmax; k++) {
-            const double x = fs.x[k];
-            const bool plus = (fs.signs[k] >> lane) & 1u;
-            // mcrade: (int64)((double)m + s x), m kept as an integer-valued
-            // double (|m| is at most the sample count, far below 2^53, so the
-            // conversions are exact and truncating in double is the same);
-            // approx and the wimpy variance add x and x * x when x > 0
-            const double add = x > 0. ? (wv ? __dmul_rn(x, x) : x) : 0.0;
-            const double y = mc ? (plus ? x : -x) : add;
-            const double t = __dadd_rn(v, y);
-            if (!st.crossed && kc < 0 && t >= 3.0) kc = (int)k;
-            v = mc ? trunc(t) : t;
+    st.lu = a.first_sample + fs.sample[31] + 1u;
+    int32_t m = 0;
+    if (a.pass == 2) {
+        unsigned long long w[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const uint4 g = *reinterpret_cast<const uint4 *>(&fs.signs[4 * i]);
+            const uint32_t plus = ((g.x >> lane) & 1u) | ((g.y >> lane) & 1u) << 1 |
+                                  ((g.z >> lane) & 1u) << 2 | ((g.w >> lane) & 1u) << 3;
+            w[i] = __ldg(&g_trial_steps.v[((c >> (4 * i)) & 15u) << 4 | plus]);
         }
-        if (kc >= 0) {  // lane 25 only: approx reached 3 at entry kc
-            st.crossed = true;
-            jc.cross_flag[node] = 1;
-            const uint32_t q = atomicAdd(&jc.sc->n_cross, 1u);
-            jc.cross_sample[q] = a.first_sample + fs.sample[kc];
+        m = mc ? (int32_t)st.v : 0;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int32_t near = max(-4, min(4, m));
+            m += (int32_t)((uint32_t)(w[i] >> (4 * (near + 4))) << 28) >> 28;
         }
-        __syncwarp();
     }
-    if (mc) {
-        if (a.pass == 2) jc.mcrade[(uint64_t)node * kTrials + lane] = (long long)v;
+    double v = st.v;
+#pragma unroll
+    for (int k = 0; k < 32; k += 2) {
+        const double2 x = *reinterpret_cast<const double2 *>(&fs.x[k]);
+        v = __dadd_rn(v, wv ? __dmul_rn(x.x, x.x) : x.x);
+        v = __dadd_rn(v, wv ? __dmul_rn(x.y, x.y) : x.y);
+    }
+    if (lane == 25 && !st.crossed && v >= 3.0) {  // approx reached 3 at entry k
+        double t = st.v;
+        int k = 0;
+        while ((t = __dadd_rn(t, fs.x[k])) < 3.0) k++;
+        st.crossed = true;
+        jc.cross_flag[node] = 1;
+        const uint32_t q = atomicAdd(&jc.sc->n_cross, 1u);
+        jc.cross_sample[q] = a.first_sample + fs.sample[k];
+    }
+    if (!mc)
+        st.v = v;
+    else if (a.pass == 2)
+        st.v = (double)m;
+    __syncwarp();
+}
+
+// Folds the kmax entries staged in the scratch.
+__device__ __forceinline__ void fold_entries(const JobCounters &jc, const ApplyArgs &a,
+                                             uint32_t node, uint32_t kmax, NodeState &st,
+                                             const FoldScratch &fs) {
+    const int lane = threadIdx.x & 31;
+    const bool mc = lane < kTrials, wv = lane == 26;
+    const bool in = (uint32_t)lane < kmax;
+    const uint32_t pm = __ballot_sync(0xffffffffu, in && fs.x[lane] > 0.);
+    // 1 + global index of the last sample that adds to approx
+    if (pm) st.lu = a.first_sample + fs.sample[31 - __clz(pm)] + 1u;
+    int kc = -1;
+    double v = st.v;
+#pragma unroll 4
+    for (uint32_t k = 0; k < kmax; k++) {
+        const double x = fs.x[k];
+        const bool plus = (fs.signs[k] >> lane) & 1u;
+        // mcrade: (int64)((double)m + s x), m kept as an integer-valued
+        // double (|m| is at most the sample count, far below 2^53, so the
+        // conversions are exact and truncating in double is the same);
+        // approx and the wimpy variance add x and x * x when x > 0
+        const double add = x > 0. ? (wv ? __dmul_rn(x, x) : x) : 0.0;
+        const double y = mc ? (plus ? x : -x) : add;
+        const double t = __dadd_rn(v, y);
+        if (!st.crossed && kc < 0 && t >= 3.0) kc = (int)k;
+        v = mc ? trunc(t) : t;
+    }
+    st.v = v;
+    if (kc >= 0) {  // lane 25 only: approx reached 3 at entry kc
+        st.crossed = true;
+        jc.cross_flag[node] = 1;
+        const uint32_t q = atomicAdd(&jc.sc->n_cross, 1u);
+        jc.cross_sample[q] = a.first_sample + fs.sample[kc];
+    }
+    __syncwarp();
+}
+
+__device__ __forceinline__ void fold_store(const JobCounters &jc, const ApplyArgs &a,
+                                           uint32_t node, const NodeState &st, FoldScratch &fs) {
+    const int lane = threadIdx.x & 31;
+    if (lane < kTrials) {
+        if (a.pass == 2) jc.mcrade[(uint64_t)node * kTrials + lane] = (long long)st.v;
     } else if (lane == 25) {
-        jc.approx[node] = v;
-        if (lu) {
+        jc.approx[node] = st.v;
+        if (st.lu) {
             if (st.lu0 == 0) fs.upd[fs.nupd++] = node;
-            jc.last_upd[node] = lu;
+            jc.last_upd[node] = st.lu;
         }
-        fs.sup_a = fmax(fs.sup_a, v);
-    } else if (wv) {
-        jc.wimpy[node] = v;
-        fs.sup_w = fmax(fs.sup_w, v);
+        fs.sup_a = fmax(fs.sup_a, st.v);
+    } else if (lane == 26) {
+        jc.wimpy[node] = st.v;
+        fs.sup_w = fmax(fs.sup_w, st.v);
     }
     __syncwarp();
     if (fs.nupd == 32) upd_flush(jc, fs);
 }
 
-// Shared memory of phase D: the sub-round's per-sample factors (read by every
-// fold in place of global gathers), warp 0's large bucket in sample order, and
-// one fold scratch per warp.  s_inv holds samples from lo & ~1 on, s_sgn
-// from lo & ~3 on (inv_base / sgn_base).
-struct CommitSmem {
-    double s_inv[kLargeBucket + 2];         // 1 / num_paths of the sub-round's samples
-    uint32_t s_sgn[kLargeBucket + 4];       // their Rademacher signs (pass 2)
-    unsigned long long sbuf[kLargeBucket];  // warp 0's bucket, in sample order
-    uint32_t bits[kLargeBucket / 32];       // samples of that bucket
-    uint32_t wpre[kLargeBucket / 32];       // set bits before each word
-    FoldScratch fsc[kCommitThreads / 32];
-};
-constexpr size_t kCommitSmem = sizeof(CommitSmem);
-__device__ __forceinline__ uint32_t inv_base(const ApplyArgs &a) { return a.lo & ~1u; }
-__device__ __forceinline__ uint32_t sgn_base(const ApplyArgs &a) { return a.lo & ~3u; }
-
-// The sub-round's 1 / num_paths and signs into shared memory, read with
-// L2-coherent loads: phase A wrote them from other CTAs, ordered before this
-// read by the grid barrier.
-__device__ void stage_factors(const RoundBuffers &rb, const ApplyArgs &a, CommitSmem &sm) {
-    const uint32_t i0 = inv_base(a), i1 = min((a.hi + 1u) & ~1u, rb.max_samples);
-    const uint32_t s0 = sgn_base(a), s1 = min((a.hi + 3u) & ~3u, rb.max_samples);
-    for (uint32_t i = threadIdx.x; i < i1 - i0; i += blockDim.x)
-        sm.s_inv[i] = __ldcg(&rb.inv_np[i0 + i]);
-    for (uint32_t i = threadIdx.x; i < s1 - s0; i += blockDim.x)
-        sm.s_sgn[i] = a.pass == 2 ? __ldcg(&rb.signs[s0 + i]) : 0u;
-    __syncthreads();
-}
-constexpr int kLoads = 8;  // bucket entries a lane of warp 0 loads at once
-constexpr uint32_t kSmallWarps = kCommitThreads / 32 - 1;  // warps 1.. of each CTA
-
-// Buckets of at most 32 entries, on warps 1.. of every CTA: touched node t
-// goes to warp t mod (CTAs x kSmallWarps), no cursor.  A bucket holds
-// distinct samples, so each entry's position in sample order is the number
-// of entries with a smaller sample (32 compares per lane, no sort).
-__device__ void apply_small(const RoundBuffers &rb, const JobCounters &jc, const RoundJournal &jr,
-                            const ApplyArgs &a, uint32_t T, CommitSmem &sm) {
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    FoldScratch &fs = sm.fsc[wib];
-    fold_begin(fs);
-    const uint32_t stride = gridDim.x * kSmallWarps;
-    for (uint32_t t = blockIdx.x * kSmallWarps + (uint32_t)(wib - 1); t < T; t += stride) {
-        const uint32_t b = __ldcg(&rb.bucket_len[t]);
-        if (b > 32) continue;
-        const uint32_t node = __ldcg(&rb.touched[t]);
-        const NodeState st = fold_load(jc, jr, a, node, t);
-        const unsigned long long key =
-            (uint32_t)lane < b ? __ldcg(&rb.entries[__ldcg(&rb.bucket_off[t]) + lane]) : ~0ull;
-        uint32_t rank = 0;
-        for (uint32_t j = 0; j < b; j++) rank += __shfl_sync(0xffffffffu, key, (int)j) < key;
-        fold_node(jc, a, node, b, st,
-                  [&](uint32_t) {
-                      if ((uint32_t)lane < b) {
-                          const uint32_t sl = (uint32_t)(key >> 32);
-                          fs.x[rank] = __dmul_rn((double)(uint32_t)key, sm.s_inv[sl - inv_base(a)]);
-                          fs.signs[rank] = sm.s_sgn[sl - sgn_base(a)];
-                          fs.sample[rank] = sl;
-                      }
-                  },
-                  fs);
-    }
-    fold_flush(jc, fs);
+__device__ __forceinline__ void fold_stage(FoldScratch &fs, uint32_t i, const DrawEntry &e) {
+    fs.x[i] = e.x;
+    fs.signs[i] = e.signs;
+    fs.sample[i] = e.sample;
 }
 
-// Buckets of more than 32 entries, on warp 0 of every CTA, claimed from a
-// cursor.  The entries of a bucket are distinct samples of the sub-round (a
-// node is on a sample's path map once), so their order is the rank of each
-// sample in a bitmap of the sub-round: set one bit per entry, prefix-count
-// the bits per word, and each entry goes to its rank (linear in the bucket;
-// no comparison sort).
-__device__ void apply_large(const RoundBuffers &rb, const JobCounters &jc, const RoundJournal &jr,
-                            const ApplyArgs &a, CommitSmem &sm) {
-    const int lane = threadIdx.x & 31;
-    FoldScratch &fs = sm.fsc[0];
-    fold_begin(fs);
-    const uint32_t NL = __ldcg(rb.n_large);
-    const uint32_t S = a.hi - a.lo;
-    const uint32_t nwords = (S + 31) / 32, per = (nwords + 31) / 32;
-    const uint32_t w0 = min(nwords, lane * per), w1 = min(nwords, w0 + per);
-    for (;;) {
-        uint32_t li = 0;
-        if (lane == 0) li = atomicAdd(rb.n_touched + 5, 1u);
-        li = __shfl_sync(0xffffffffu, li, 0);
-        if (li >= NL) break;
+__device__ __forceinline__ DrawEntry entry_load(const DrawEntry *p) {
+    const uint4 w = __ldcg(reinterpret_cast<const uint4 *>(p));
+    DrawEntry e;
+    e.x = __hiloint2double((int)w.y, (int)w.x);
+    e.signs = w.z;
+    e.sample = w.w;
+    return e;
+}
+
+constexpr int kRoundThreads = 512;
+constexpr int kRoundCtas = 2;     // per SM
+constexpr uint32_t kAhead = 3;    // sets of 32 entries on their way in a large bucket
+constexpr uint32_t kBatch = 8;    // small buckets a warp looks at together
+
+// Buckets of more than 32 entries, one warp each: the first entry of the round
+// by a 32-way search, then 32 entries at a time, the next sets on their
+// way while one is folded.
+__device__ void fold_large(const RoundBuffers &rb, const JobCounters &jc, const RoundJournal &jr,
+                           const ApplyArgs &a, uint32_t w, uint32_t nw, FoldScratch &fs) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t NL = __ldcg(rb.n_touched + 9);
+    for (uint32_t li = w; li < NL; li += nw) {
         const uint32_t t = __ldcg(&rb.large[li]);
-        const uint32_t b0 = __ldcg(&rb.bucket_off[t]), b = __ldcg(&rb.bucket_len[t]);
-        if (b > S) {  // more entries than samples: not a bucket of distinct samples
-            if (lane == 0) atomicCAS(&jc.sc->error, 0, SILVAN_E_STATE);
-            continue;
-        }
+        const uint32_t off = __ldcg(&rb.bucket_off[t]), b = __ldcg(&rb.bucket_len[t]);
+        const uint2 span = __ldcg(&rb.bucket_span[t]);
         const uint32_t node = __ldcg(&rb.touched[t]);
-        const NodeState st = fold_load(jc, jr, a, node, t);
-        for (uint32_t w = w0; w < w1; w++) sm.bits[w] = 0u;
-        __syncwarp();
-        // the bucket's entries kLoads at a time per lane, all loads in
-        // flight before their uses
-        for (uint32_t i0 = 0; i0 < b; i0 += 32 * kLoads) {
-            unsigned long long e[kLoads];
-#pragma unroll
-            for (int j = 0; j < kLoads; j++) {
-                const uint32_t i = i0 + (uint32_t)j * 32 + lane;
-                e[j] = i < b ? __ldcg(&rb.entries[b0 + i]) : 0ull;
-            }
-#pragma unroll
-            for (int j = 0; j < kLoads; j++) {
-                if (i0 + (uint32_t)j * 32 + lane >= b) continue;
-                const uint32_t sidx = (uint32_t)(e[j] >> 32) - a.lo;
-                if (sidx < S) atomicOr(&sm.bits[sidx >> 5], 1u << (sidx & 31));
-                else atomicCAS(&jc.sc->error, 0, SILVAN_E_STATE);
-            }
+        if (span.x >= a.hi || span.y < a.lo) continue;
+        NodeState st = fold_load(jc, a, node);
+        const DrawEntry *E = rb.sorted + off;
+        uint32_t l = 0, h = span.x >= a.lo ? 0u : b;  // first entry at or beyond lo in [l, h]
+        while (h > l) {
+            const uint32_t step = (h - l + 31u) / 32u;
+            const uint32_t i = l + lane * step;
+            const bool below = i < h && __ldcg(&E[i].sample) < a.lo;
+            const uint32_t k = (uint32_t)__popc(__ballot_sync(0xffffffffu, below));
+            if (k == 0u) break;
+            h = min(h, l + k * step);
+            l = l + (k - 1u) * step + 1u;
         }
-        __syncwarp();
-        // exclusive prefix of the words' bit counts (lane L owns words
-        // [L per, (L + 1) per))
-        uint32_t c = 0;
-        for (uint32_t w = w0; w < w1; w++) c += __popc(sm.bits[w]);
-        uint32_t incl = c;
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += u;
-        }
-        uint32_t run = incl - c;
-        for (uint32_t w = w0; w < w1; w++) {
-            sm.wpre[w] = run;
-            run += __popc(sm.bits[w]);
-        }
-        __syncwarp();
-        for (uint32_t i0 = 0; i0 < b; i0 += 32 * kLoads) {
-            unsigned long long e[kLoads];
+        DrawEntry e{0.0, 0u, 0xffffffffu}, next[kAhead];
 #pragma unroll
-            for (int j = 0; j < kLoads; j++) {
-                const uint32_t i = i0 + (uint32_t)j * 32 + lane;
-                e[j] = i < b ? __ldcg(&rb.entries[b0 + i]) : 0ull;
-            }
+        for (uint32_t p = 0; p < kAhead; p++)
+            if (l + p * 32u + lane < b) next[p] = entry_load(&E[l + p * 32u + lane]);
+        const bool few = (uint64_t)a.first_sample + a.hi < (1ull << 26);
+        bool first = true;
+        for (uint32_t i = l;; i += 32u) {
+            e = next[0];
 #pragma unroll
-            for (int j = 0; j < kLoads; j++) {
-                if (i0 + (uint32_t)j * 32 + lane >= b) continue;
-                const uint32_t sidx = (uint32_t)(e[j] >> 32) - a.lo;
-                if (sidx < S) {
-                    const uint32_t w = sidx >> 5;
-                    sm.sbuf[sm.wpre[w] + __popc(sm.bits[w] & ((1u << (sidx & 31)) - 1u))] = e[j];
-                }
-            }
+            for (uint32_t p = 0; p + 1 < kAhead; p++) next[p] = next[p + 1];
+            const uint32_t k =
+                (uint32_t)__popc(__ballot_sync(0xffffffffu, i + lane < b && e.sample < a.hi));
+            if (k == 0u) break;
+            if (first && a.journal) fold_journal(jr, a, t, st);
+            first = false;
+            if (lane < k) fold_stage(fs, lane, e);
+            const uint32_t far = i + kAhead * 32u + lane;
+            if (far < b) next[kAhead - 1] = entry_load(&E[far]);
+            __syncwarp();
+            const bool one = e.x == 1.0;
+            const bool plain = one || (e.x >= 0x1p-25 && e.x <= 1.0 - 0x1p-25);
+            if (k == 32u && few && __all_sync(0xffffffffu, plain))
+                fold_full(jc, a, node, __ballot_sync(0xffffffffu, one), st, fs);
+            else
+                fold_entries(jc, a, node, k, st, fs);
+            if (k < 32u) break;
         }
-        __syncwarp();
-        fold_node(jc, a, node, b, st,
-                  [&](uint32_t r0) {
-                      const uint32_t r = r0 + lane;
-                      if (r < b) {
-                          const unsigned long long e = sm.sbuf[r];
-                          const uint32_t sl = (uint32_t)(e >> 32);
-                          fs.x[lane] = __dmul_rn((double)(uint32_t)e, sm.s_inv[sl - inv_base(a)]);
-                          fs.signs[lane] = sm.s_sgn[sl - sgn_base(a)];
-                          fs.sample[lane] = sl;
-                      }
-                  },
-                  fs);
+        if (!first) fold_store(jc, a, node, st, fs);
     }
-    fold_flush(jc, fs);
+}
+
+// Buckets of at most 32 entries: a warp looks at kBatch of them, leaves out
+// those without samples of the round by their span, and folds the others one
+// after another, the next one's entries and counters loaded meanwhile.
+__device__ void fold_small(const RoundBuffers &rb, const JobCounters &jc, const RoundJournal &jr,
+                           const ApplyArgs &a, uint32_t w, uint32_t nw, FoldScratch &fs) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t T = __ldcg(rb.n_touched + 8);
+    for (uint32_t t0 = w * kBatch; t0 < T; t0 += nw * kBatch) {
+        const uint32_t t = t0 + lane;
+        uint32_t off = 0, len = 33, node = 0;
+        uint2 span = make_uint2(0u, 0u);
+        if (lane < kBatch && t < T) {
+            off = __ldcg(&rb.bucket_off[t]);
+            len = __ldcg(&rb.bucket_len[t]);
+            span = __ldcg(&rb.bucket_span[t]);
+            node = __ldcg(&rb.touched[t]);
+        }
+        uint32_t m = __ballot_sync(0xffffffffu, len <= 32u && span.x < a.hi && span.y >= a.lo);
+        int i = m ? __ffs(m) - 1 : 0;
+        uint32_t o_n = __shfl_sync(0xffffffffu, off, i), l_n = __shfl_sync(0xffffffffu, len, i);
+        uint32_t v_n = __shfl_sync(0xffffffffu, node, i);
+        DrawEntry e_n{0.0, 0u, 0xffffffffu};
+        NodeState s_n{0.0, 0u, 0u, true};
+        if (m) {
+            if (lane < l_n) e_n = entry_load(&rb.sorted[o_n + lane]);
+            s_n = fold_load(jc, a, v_n);
+        }
+        while (m) {
+            const uint32_t at = t0 + (uint32_t)i, v = v_n, l = l_n;
+            const DrawEntry e = e_n;
+            NodeState st = s_n;
+            m &= m - 1u;
+            if (m) {
+                i = __ffs(m) - 1;
+                o_n = __shfl_sync(0xffffffffu, off, i);
+                l_n = __shfl_sync(0xffffffffu, len, i);
+                v_n = __shfl_sync(0xffffffffu, node, i);
+                e_n.sample = 0xffffffffu;
+                if (lane < l_n) e_n = entry_load(&rb.sorted[o_n + lane]);
+                s_n = fold_load(jc, a, v_n);
+            }
+            const bool in = lane < l && e.sample >= a.lo && e.sample < a.hi;
+            const uint32_t im = __ballot_sync(0xffffffffu, in);
+            if (!im) continue;
+            if (a.journal) fold_journal(jr, a, at, st);
+            if (in) fold_stage(fs, (uint32_t)__popc(im & ((1u << lane) - 1u)), e);
+            __syncwarp();
+            fold_entries(jc, a, v, (uint32_t)__popc(im), st, fs);
+            fold_store(jc, a, v, st, fs);
+        }
+    }
 }
 
 __device__ void commit_sums(const RoundBuffers &rb, const JobCounters &jc, const ApplyArgs &a) {
@@ -534,95 +796,51 @@ __device__ void commit_sums(const RoundBuffers &rb, const JobCounters &jc, const
 }
 
 
-// The last CTA out zeroes the round's control words for the next round
-// (word 7, the touched count, stays for undo_round).
-__device__ void commit_exit(const RoundBuffers &rb) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(rb.n_touched + 6, 1u) == gridDim.x - 1) {
-            rb.n_touched[0] = 0u;
-            rb.n_touched[1] = 0u;
-            rb.n_touched[4] = 0u;
-            rb.n_touched[5] = 0u;
-            rb.n_touched[6] = 0u;
-            __threadfence();
-        }
-    }
-}
-
-__global__ void __launch_bounds__(kCommitThreads, 1) commit_round_kernel(const ApplyState st) {
-    extern __shared__ __align__(16) unsigned char commit_smem[];
+__global__ void __launch_bounds__(kRoundThreads, kRoundCtas) commit_round_kernel(
+    const ApplyState st) {
+    __shared__ FoldScratch fsc[kRoundThreads / 32];
     const RoundBuffers &rb = st.rb;
     const JobCounters &jc = st.jc;
     const RoundJournal &jr = st.jr;
     const ApplyArgs &a = st.a;
-    uint32_t *bar = rb.n_touched + 2;
-    if (a.journal && blockIdx.x == 0) {
-        // the scalars and path-length counts as the round starts (phase D
-        // is the first to change them)
-        const unsigned long long *src = reinterpret_cast<const unsigned long long *>(jc.sc);
-        unsigned long long *dst = reinterpret_cast<unsigned long long *>(jr.sc);
-        for (uint32_t i = threadIdx.x; i < sizeof(JobScalars) / 8; i += blockDim.x) dst[i] = src[i];
-        for (uint32_t i = threadIdx.x; i <= a.D; i += blockDim.x) jr.sp_lengths[i] = jc.sp_lengths[i];
-    }
-    bucket_count(rb, a);
-    if (!grid_barrier(bar)) goto timeout;
-    {
-        const uint32_t T = __ldcg(rb.n_touched);
-        if (blockIdx.x == 0 && threadIdx.x == 0) rb.n_touched[7] = T;
-        bucket_alloc(rb, T);
-        if (!grid_barrier(bar)) goto timeout;
-        bucket_scatter(rb, a);
-        if (!grid_barrier(bar)) goto timeout;
-        CommitSmem &sm = *reinterpret_cast<CommitSmem *>(commit_smem);
-        // the sub-round's factors into shared memory, then warp 0 folds the
-        // large buckets while the other warps fold the small ones
-        stage_factors(rb, a, sm);
-        if (threadIdx.x < 32) apply_large(rb, jc, jr, a, sm);
-        else apply_small(rb, jc, jr, a, T, sm);
-        __syncthreads();
-        commit_sums(rb, jc, a);
-        // the scatter cursors back to zero for the next round
-        for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < T;
-             t += gridDim.x * blockDim.x)
-            rb.node_cnt[rb.touched[t]] = 0;
-    }
-    commit_exit(rb);
-    return;
-timeout:
-    if (threadIdx.x == 0) atomicCAS(&jc.sc->error, 0, SILVAN_E_TIMEOUT);
-    commit_exit(rb);
+    const uint32_t wib = threadIdx.x >> 5, nw = gridDim.x * (kRoundThreads / 32);
+    FoldScratch &fs = fsc[wib];
+    fold_begin(fs);
+    // the long buckets first, spread over the CTAs
+    fold_large(rb, jc, jr, a, wib * gridDim.x + blockIdx.x, nw, fs);
+    fold_small(rb, jc, jr, a, blockIdx.x * (kRoundThreads / 32) + wib, nw, fs);
+    fold_flush(jc, fs);
+    commit_sums(rb, jc, a);
 }
 
-int g_commit_grid = 0;  // resident CTAs of commit_round_kernel (apply_init)
+int g_commit_grid = 0;  // resident CTAs of prepare_draw_kernel (apply_init)
+int g_sms = 0;
 
 }  // namespace
 
 cudaError_t apply_init() {
-    cudaError_t e = cudaFuncSetAttribute(commit_round_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kCommitSmem);
-    if (e != cudaSuccess) return e;
-    int dev = 0, sms = 0, per_sm = 0;
+    int dev = 0, per_sm = 0;
+    cudaError_t e;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
+    if ((e = cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
         return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, commit_round_kernel,
-                                                      kCommitThreads, kCommitSmem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, prepare_draw_kernel,
+                                                      kCommitThreads, 0);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorLaunchOutOfResources;
-    g_commit_grid = sms * per_sm;
+    g_commit_grid = g_sms;
     return cudaSuccess;
 }
 
-// One warp per node of the round's touched list, lanes as in the fold.
+// One warp per node of the draw's touched list that the round saved, lanes as
+// in the fold.
 __global__ void undo_round_kernel(RoundBuffers rb, JobCounters jc, RoundJournal jr, int pass,
-                                  uint32_t D) {
-    const uint32_t T = __ldcg(rb.n_touched + 7);
+                                  uint32_t D, uint32_t stamp) {
+    const uint32_t T = __ldcg(rb.n_touched + 8);
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < T; t += nw) {
+        if (jr.stamp[t] != stamp) continue;
         const uint32_t node = rb.touched[t];
         if (lane < kTrials) {
             if (pass == 2)
@@ -642,19 +860,25 @@ __global__ void undo_round_kernel(RoundBuffers rb, JobCounters jc, RoundJournal 
     }
 }
 
-cudaError_t apply_round(const ApplyState &st, cudaStream_t stream) {
+cudaError_t prepare_draw(const ApplyState &st, cudaStream_t stream) {
     if (g_commit_grid <= 0) return cudaErrorNotReady;
+    if (st.a.count > kDrawSamples) return cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)g_commit_grid);
     cfg.blockDim = dim3(kCommitThreads);
-    cfg.dynamicSmemBytes = kCommitSmem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, commit_round_kernel, st);
+    return cudaLaunchKernelEx(&cfg, prepare_draw_kernel, st);
+}
+
+cudaError_t apply_round(const ApplyState &st, cudaStream_t stream) {
+    if (g_sms <= 0) return cudaErrorNotReady;
+    commit_round_kernel<<<g_sms * kRoundCtas, kRoundThreads, 0, stream>>>(st);
+    return cudaGetLastError();
 }
 
 namespace {
@@ -680,7 +904,7 @@ __global__ void stop_init_kernel(StopReduction *acc) {
 // readback and leaves the accumulator neutral for the next check.
 __global__ void __launch_bounds__(512) stop_reduce_kernel(JobCounters jc, int nparts, uint32_t D,
                                                           StopReduction *acc, uint32_t *ticket,
-                                                          StopReadback rb) {
+                                                          StopReadback rb, RoundJournal jr) {
     __shared__ long long smc[kMaxPartitions * kTrials];
     __shared__ unsigned long long sw[kMaxPartitions];
     __shared__ uint32_t st[kMaxPartitions];
@@ -783,9 +1007,17 @@ __global__ void __launch_bounds__(512) stop_reduce_kernel(JobCounters jc, int np
     }
     const unsigned long long *src = reinterpret_cast<const unsigned long long *>(jc.sc);
     unsigned long long *dst = reinterpret_cast<unsigned long long *>(rb.sc);
-    for (uint32_t i = threadIdx.x; i < sizeof(JobScalars) / 8; i += blockDim.x) dst[i] = __ldcg(&src[i]);
-    if (rb.sp)
-        for (uint32_t i = threadIdx.x; i <= D; i += blockDim.x) rb.sp[i] = __ldcg(&jc.sp_lengths[i]);
+    unsigned long long *keep = reinterpret_cast<unsigned long long *>(jr.sc);
+    for (uint32_t i = threadIdx.x; i < sizeof(JobScalars) / 8; i += blockDim.x) {
+        const unsigned long long x = __ldcg(&src[i]);
+        dst[i] = x;
+        if (keep) keep[i] = x;
+    }
+    for (uint32_t i = threadIdx.x; i <= D; i += blockDim.x) {
+        const uint64_t x = __ldcg(&jc.sp_lengths[i]);
+        if (rb.sp) rb.sp[i] = x;
+        if (jr.sp_lengths) jr.sp_lengths[i] = x;
+    }
 }
 
 // Peeling index of node v (Probabilistic.cpp:855-862), stored in peel_idx.
@@ -908,8 +1140,8 @@ __global__ void divide_kernel(const double *approx, double m, double *out, uint3
 }
 
 cudaError_t undo_round(const RoundBuffers &rb, const JobCounters &jc, const RoundJournal &jr,
-                       int pass, uint32_t D, cudaStream_t stream) {
-    undo_round_kernel<<<296, 512, 0, stream>>>(rb, jc, jr, pass, D);
+                       int pass, uint32_t D, uint32_t stamp, cudaStream_t stream) {
+    undo_round_kernel<<<296, 512, 0, stream>>>(rb, jc, jr, pass, D, stamp);
     return cudaGetLastError();
 }
 
@@ -927,8 +1159,9 @@ cudaError_t stop_reduce_init(StopReduction *acc, uint32_t *ticket, cudaStream_t 
 }
 
 cudaError_t stop_reduce(const JobCounters &jc, int nparts, uint32_t D, StopReduction *acc,
-                        uint32_t *ticket, const StopReadback &out, cudaStream_t stream) {
-    stop_reduce_kernel<<<296, 512, 0, stream>>>(jc, nparts, D, acc, ticket, out);
+                        uint32_t *ticket, const StopReadback &out, const RoundJournal &jr,
+                        cudaStream_t stream) {
+    stop_reduce_kernel<<<296, 512, 0, stream>>>(jc, nparts, D, acc, ticket, out, jr);
     return cudaGetLastError();
 }
 

@@ -10,7 +10,8 @@
 
 namespace silvan {
 
-constexpr uint32_t kLargeBucket = 8192;  // samples per apply sub-round (bucket bound)
+constexpr uint32_t kDrawSamples = 65536;  // samples of a draw at most
+constexpr uint32_t kHugeBucket = 256;     // larger buckets are ordered by a whole CTA
 constexpr int kMaxPartitions = 128;
 
 // Job-level scalars kept on the device.
@@ -31,6 +32,13 @@ struct JobScalars {
 
 static_assert(sizeof(JobScalars) % 8 == 0, "JobScalars is copied in 8-byte words");
 
+// One contribution to a node, as a commit round reads it.
+struct __align__(16) DrawEntry {
+    double x;         // count * (1 / num_paths)
+    uint32_t signs;   // the sample's Rademacher signs
+    uint32_t sample;  // round-local index
+};
+
 struct RoundBuffers {
     // per round-local sample
     int32_t *pl;
@@ -40,7 +48,7 @@ struct RoundBuffers {
     uint32_t *signs;
     uint32_t *ball;
     uint32_t *pred;
-    double *inv_np;  // 1 / num_paths of each sample (set by the commit)
+    double *inv_np;  // 1 / num_paths of each sample (set by prepare_draw)
     uint32_t max_samples;
     // path-map records
     PathRec *recs;
@@ -49,16 +57,19 @@ struct RoundBuffers {
     // bucketing by node
     uint32_t *node_cnt;      // n, zero between rounds
     uint32_t *touched;       // distinct nodes of the round
-    // control words of the commit rounds (zero when allocated; each round
-    // leaves them as it found them): [0] touched nodes, [1] large buckets,
-    // [2..3] grid barrier, [4] bucket-space cursor, [5] large-bucket claims,
-    // [6] CTAs done; [7] touched nodes of the last round (read by undo_round)
+    // control words (zero when allocated; prepare_draw leaves [0..7] zero):
+    // [0] touched nodes, [1] large buckets, [2..3] grid barrier, [4]
+    // bucket-space cursor, [5] claims of the huge ones, [6] CTAs done, [7] huge
+    // buckets; of the prepared draw: [8] touched nodes, [9] large buckets
     uint32_t *n_touched;
     uint32_t *bucket_off;    // start of each touched node's bucket
     uint32_t *bucket_len;    // its number of entries
+    uint2 *bucket_span;      // its first and last sample
     uint32_t *large;         // buckets of more than 32 entries (listed by bucket_alloc)
     uint32_t *n_large;       // = n_touched + 1 (both zeroed together)
+    uint32_t *huge;          // buckets of more than kHugeBucket entries
     unsigned long long *entries;  // sample << 32 | count, grouped by node
+    DrawEntry *sorted;            // the same, each bucket in sample order
     uint32_t *work_counter;  // sampler work counter
 };
 
@@ -78,7 +89,8 @@ struct JobCounters {
 
 struct ApplyArgs {
     uint32_t n;
-    uint32_t n_records;      // path-map records of the round
+    uint32_t n_records;      // path-map records of the draw
+    uint32_t count;          // samples of the draw
     uint64_t seed;
     uint32_t first_sample;   // global index of round-local sample 0
     uint32_t lo, hi;         // round-local sample range committed by this call
@@ -86,18 +98,21 @@ struct ApplyArgs {
     int32_t track_cross;     // pass 1 of top-k mode
     uint32_t D;
     int32_t journal;         // save what the round changes (RoundJournal) so it can be undone
+    uint32_t stamp;          // of a journaled round: distinct from every earlier one's
 };
 
 // What a journaled commit round overwrites: the old counters of each node it
-// folds (indexed by the node's position on the round's touched list), the
-// job's scalars and the shortest-path length counts.  undo_round puts them
-// back, which leaves the counters as they were before the round.  Sized for
-// every node of the graph (a round touches each node at most once).
+// folds (indexed by the node's position on the draw's touched list), and, saved
+// by the check before it (stop_reduce), the job's scalars and the
+// shortest-path length counts.  undo_round puts them back, which leaves the
+// counters as they were before the round.  Sized for every node of the graph
+// (a round touches each node at most once).
 struct RoundJournal {
     long long *mcrade;     // n x 25 (pass 2 only)
     double *approx;        // n
     double *wimpy;         // n
     uint32_t *last_upd;    // n
+    uint32_t *stamp;       // n: the journaled round that saved the entry
     JobScalars *sc;        // 1
     uint64_t *sp_lengths;  // D + 1
 };
@@ -110,21 +125,21 @@ struct ApplyState {
     ApplyArgs a;
 };
 
-// Kernels apply_round launches: one cooperative kernel.
-constexpr int kApplyRoundKernels = 1;
-
-// Commits round-local samples [a.lo, a.hi) of the round buffers to the job
-// counters: one cooperative kernel whose phases are separated by grid-wide
-// barriers, with st as its argument.
+// Groups the records of a draw (samples [0, a.count), a.n_records records) by
+// node, each node's in sample order, for the commit rounds that follow: one
+// cooperative kernel whose phases are separated by grid-wide barriers.
+cudaError_t prepare_draw(const ApplyState &st, cudaStream_t stream);
+// Commits round-local samples [a.lo, a.hi) of the prepared draw to the job
+// counters.
 cudaError_t apply_round(const ApplyState &st, cudaStream_t stream);
-// Function attributes and resident grid of the commit kernel on the current
-// device (call before capturing).
+// Resident grid of the prepare kernel on the current device (call before
+// capturing).
 cudaError_t apply_init();
-// Restores what the last commit round (journaled, and the last round on
-// rb) changed: the nodes of rb's touched list, the scalars, the path-length
-// counts.
+// Restores what the last commit round (journaled with `stamp`) changed: the
+// nodes it folded, and the scalars and path-length counts as the check before
+// it saved them.
 cudaError_t undo_round(const RoundBuffers &rb, const JobCounters &jc, const RoundJournal &jr,
-                       int pass, uint32_t D, cudaStream_t stream);
+                       int pass, uint32_t D, uint32_t stamp, cudaStream_t stream);
 
 // Reduction for one stopping-rule evaluation: per partition and trial the
 // maximum of mcrade (LLONG_MIN when no node of the partition was updated;
@@ -156,9 +171,11 @@ struct StopReadback {
 // (stop_reduce leaves them neutral).
 cudaError_t stop_reduce_init(StopReduction *acc, uint32_t *ticket, cudaStream_t stream);
 // One kernel: the reduction over upd_list plus the scalars and path-length
-// counts, written to `out`.
+// counts, written to `out`; these two also to the journal (where its pointers
+// are not null), for a journaled round after the check.
 cudaError_t stop_reduce(const JobCounters &jc, int nparts, uint32_t D, StopReduction *acc,
-                        uint32_t *ticket, const StopReadback &out, cudaStream_t stream);
+                        uint32_t *ticket, const StopReadback &out, const RoundJournal &jr,
+                        cudaStream_t stream);
 
 cudaError_t peel_map(const JobCounters &jc, uint32_t n, const int32_t *lut, int32_t idx_min,
                      int32_t lut_size, uint32_t *hist, cudaStream_t stream);

@@ -1098,6 +1098,9 @@ Job::~Job() {
     dfree(r.bucket_off);
     dfree(r.bucket_len);
     dfree(r.entries);
+    dfree(r.sorted);
+    dfree(r.bucket_span);
+    dfree(r.huge);
     dfree(jc_.approx);
     dfree(jc_.wimpy);
     dfree(jc_.mcrade);
@@ -1122,6 +1125,7 @@ Job::~Job() {
     dfree(jr_.approx);
     dfree(jr_.wimpy);
     dfree(jr_.last_upd);
+    dfree(jr_.stamp);
     dfree(jr_.sc);
     dfree(jr_.sp_lengths);
     if (ev_chk_) cudaEventDestroy(ev_chk_);
@@ -1150,8 +1154,8 @@ int Job::alloc_round(uint32_t max_samples, uint64_t rec_cap) {
     RK(dmalloc(&r.ball, max_samples));
     RK(dmalloc(&r.pred, max_samples));
     RK(dmalloc(&r.node_cnt, n_));
-    RK(dmalloc(&r.n_touched, 8));
-    CK(cudaMemset(r.n_touched, 0, 8 * sizeof(uint32_t)));
+    RK(dmalloc(&r.n_touched, 16));
+    CK(cudaMemset(r.n_touched, 0, 16 * sizeof(uint32_t)));
     RK(dmalloc(&r.inv_np, max_samples));
     r.n_large = r.n_touched + 1;
     r.rec_cursor = nullptr;
@@ -1169,6 +1173,9 @@ int Job::grow_records(uint64_t cap) {
     dfree(r.bucket_off);
     dfree(r.bucket_len);
     dfree(r.entries);
+    dfree(r.sorted);
+    dfree(r.bucket_span);
+    dfree(r.huge);
     r.rec_cap = cap;
     const uint64_t tcap = std::min<uint64_t>(cap, n_) + 1;
     RK(dmalloc(&r.recs, cap));
@@ -1177,15 +1184,18 @@ int Job::grow_records(uint64_t cap) {
     RK(dmalloc(&r.bucket_off, tcap + 1));
     RK(dmalloc(&r.bucket_len, tcap));
     RK(dmalloc(&r.entries, cap));
+    RK(dmalloc(&r.sorted, cap));
+    RK(dmalloc(&r.bucket_span, tcap));
+    RK(dmalloc(&r.huge, cap / kHugeBucket + 1));
     return SILVAN_OK;
 }
 
 uint64_t Job::device_bytes() const {
     const uint64_t n = n_;
     uint64_t b = n * (8 + 8 + 8 * kTrials + 4 + 1 + 4 + 4 + 4 + 4);
-    if (p_.k == 0) b += n * (8 * kTrials + 8 + 8 + 4);  // the round journal
-    b += (uint64_t)kRoundSamples * 36 + rb_.rec_cap * (12 + 8) +
-         std::min<uint64_t>(rb_.rec_cap, n) * 8;
+    if (p_.k == 0) b += n * (8 * kTrials + 8 + 8 + 4 + 4);  // the round journal
+    b += (uint64_t)kRoundSamples * 36 + rb_.rec_cap * (12 + 8 + sizeof(DrawEntry)) +
+         std::min<uint64_t>(rb_.rec_cap, n) * 16;
     return b;
 }
 
@@ -1226,6 +1236,8 @@ int Job::init() {
         RK(dmalloc(&jr_.approx, n));
         RK(dmalloc(&jr_.wimpy, n));
         RK(dmalloc(&jr_.last_upd, n));
+        RK(dmalloc(&jr_.stamp, n));
+        CK(cudaMemset(jr_.stamp, 0, sizeof(uint32_t) * n));
         RK(dmalloc(&jr_.sc, 1));
         RK(dmalloc(&jr_.sp_lengths, (uint64_t)g_->diameter + 1));
         CK(cudaEventCreateWithFlags(&ev_chk_, cudaEventDisableTiming));
@@ -1258,33 +1270,47 @@ int Job::init() {
     return SILVAN_OK;
 }
 
-// Commits samples [lo, hi) (indices into the drawn range r) whose raw outputs
-// the engine left in rb_, in apply sub-rounds of at most kLargeBucket samples.
-int Job::apply_range(const JobRequest &r, uint32_t lo, uint32_t hi, uint64_t n_records,
-                     bool journal) {
-    if (journal && (hi - lo > kLargeBucket || !jr_.approx)) {
-        set_error("a journaled commit round must be a single sub-round");
+ApplyState Job::apply_state(const JobRequest &r) {
+    ApplyState st{};
+    st.rb = rb_;
+    st.jc = jc_;
+    st.jr = jr_;
+    ApplyArgs &a = st.a;
+    a.n = n_;
+    a.count = r.count;
+    a.seed = p_.seed;
+    a.first_sample = r.first_global;
+    a.pass = r.pass;
+    a.track_cross = r.track_cross ? 1 : 0;
+    a.D = g_->diameter;
+    return st;
+}
+
+// Groups the raw outputs that the engine left in rb_ for the drawn range r, for
+// the commits of its parts.
+int Job::prepare_range(const JobRequest &r, uint64_t n_records) {
+    static_assert(kRoundSamples <= kDrawSamples, "a draw fits the bitmap of its samples");
+    ApplyState st = apply_state(r);
+    st.a.n_records = (uint32_t)n_records;
+    CK(prepare_draw(st, stream_));
+    launches += 1;
+    return SILVAN_OK;
+}
+
+// Commits samples [lo, hi) (indices into the drawn range r, prepared).
+int Job::apply_range(const JobRequest &r, uint32_t lo, uint32_t hi, bool journal) {
+    if (journal && !jr_.approx) {
+        set_error("no round journal");
         return SILVAN_E_STATE;
     }
-    for (uint32_t a0 = lo; a0 < hi; a0 += kLargeBucket) {
-        ApplyState st{};
-        st.rb = rb_;
-        st.jc = jc_;
-        st.jr = jr_;
-        ApplyArgs &a = st.a;
-        a.journal = journal ? 1 : 0;
-        a.n = n_;
-        a.n_records = (uint32_t)n_records;
-        a.seed = p_.seed;
-        a.first_sample = r.first_global;
-        a.lo = a0;
-        a.hi = std::min<uint32_t>(hi, a0 + kLargeBucket);
-        a.pass = r.pass;
-        a.track_cross = r.track_cross ? 1 : 0;
-        a.D = g_->diameter;
-        CK(apply_round(st, stream_));
-        launches += kApplyRoundKernels;
-    }
+    if (lo >= hi) return SILVAN_OK;
+    ApplyState st = apply_state(r);
+    st.a.journal = journal ? 1 : 0;
+    st.a.stamp = journal ? ++stamp_ : 0u;
+    st.a.lo = lo;
+    st.a.hi = hi;
+    CK(apply_round(st, stream_));
+    launches += 1;
     return SILVAN_OK;
 }
 
@@ -1600,7 +1626,8 @@ bool Job::check_topk(std::string &outs) {
 int Job::stop_check_enqueue() {
     StopReadback out = readback_;
     if (!absolute_) out.sp = nullptr;
-    CK(stop_reduce(jc_, nparts_, g_->diameter, d_red_, d_ticket_, out, stream_));
+    // the scalars as they are now also into the journal (null in top-k mode)
+    CK(stop_reduce(jc_, nparts_, g_->diameter, d_red_, d_ticket_, out, jr_, stream_));
     launches += 1;
     if (ev_chk_) CK(cudaEventRecord(ev_chk_, stream_));
     return SILVAN_OK;
@@ -1929,6 +1956,7 @@ int Job::on_drawn(const JobRequest &r, uint64_t n_records) {
     }
     const uint64_t save_apply = launches;
     CK(cudaEventRecord(ev_commit_[0], stream_));
+    RK(prepare_range(r, n_records));
     for (;;) {
         JobRequest rc = r;
         rc.pass = phase_ == kPass1 ? 1 : 2;
@@ -1936,7 +1964,7 @@ int Job::on_drawn(const JobRequest &r, uint64_t n_records) {
         const uint64_t cur = base_global_ + pass_samples_;
         const uint64_t c_hi = std::min(base_global_ + target_, g1);
         if (c_hi > cur) {
-            RK(apply_range(rc, (uint32_t)(cur - g0), (uint32_t)(c_hi - g0), n_records));
+            RK(apply_range(rc, (uint32_t)(cur - g0), (uint32_t)(c_hi - g0)));
             pass_samples_ += c_hi - cur;
         }
         if (pass_samples_ < target_) break;  // the next point lies beyond the drawn range
@@ -1945,7 +1973,6 @@ int Job::on_drawn(const JobRequest &r, uint64_t n_records) {
         ov_.rc = rc;
         ov_.g0 = g0;
         ov_.g1 = g1;
-        ov_.n_records = n_records;
         const int ev = evaluate();
         ov_.on = false;
         RK(ev);
@@ -1976,7 +2003,7 @@ int Job::on_drawn(const JobRequest &r, uint64_t n_records) {
 // size where they are, with a journal (ov_ records the round).  The host
 // evaluates the check meanwhile; evaluate() keeps the round if the point
 // comes out the same and undoes it otherwise.  The samples must be in the
-// drawn range and fit one commit sub-round.
+// drawn range.
 int Job::speculate() {
     ov_.spec_lo = ov_.spec_hi = 0;
     if (!ov_.on || !absolute_ || !jr_.approx || p_.serial_checks || phase_ != kPass2 ||
@@ -1984,17 +2011,17 @@ int Job::speculate() {
         return SILVAN_OK;
     const uint64_t ns = (uint64_t)(next_stop_ * 1.2);
     const uint64_t t = pass2_target(pass_samples_, p_.m_hat != 0, omega_, ns, last_stop_);
-    if (t <= pass_samples_ || t - pass_samples_ > kLargeBucket) return SILVAN_OK;
+    if (t <= pass_samples_) return SILVAN_OK;
     const uint64_t cur = base_global_ + pass_samples_, hi = base_global_ + t;
     if (cur < ov_.g0 || hi > ov_.g1) return SILVAN_OK;
-    RK(apply_range(ov_.rc, (uint32_t)(cur - ov_.g0), (uint32_t)(hi - ov_.g0), ov_.n_records, true));
+    RK(apply_range(ov_.rc, (uint32_t)(cur - ov_.g0), (uint32_t)(hi - ov_.g0), true));
     ov_.spec_lo = pass_samples_;
     ov_.spec_hi = t;
     return SILVAN_OK;
 }
 
 int Job::undo_speculation() {
-    CK(undo_round(rb_, jc_, jr_, 2, g_->diameter, stream_));
+    CK(undo_round(rb_, jc_, jr_, 2, g_->diameter, stamp_, stream_));
     launches += 1;
     ov_.spec_lo = ov_.spec_hi = 0;
     return SILVAN_OK;

@@ -299,8 +299,9 @@ class Job {
   private:
     enum Phase { kInit, kPass1, kPass2, kDone };
     int alloc_round(uint32_t max_samples, uint64_t rec_cap);
-    int apply_range(const JobRequest &r, uint32_t lo, uint32_t hi, uint64_t n_records,
-                    bool journal = false);
+    int prepare_range(const JobRequest &r, uint64_t n_records);
+    int apply_range(const JobRequest &r, uint32_t lo, uint32_t hi, bool journal = false);
+    ApplyState apply_state(const JobRequest &r);
     int evaluate();
     int speculate();
     int undo_speculation();
@@ -344,11 +345,12 @@ class Job {
     // while the host evaluates the check, and undone if the check stops the
     // run or moves the next schedule point
     RoundJournal jr_{};
+    uint32_t stamp_ = 0;  // of the last journaled round
     cudaEvent_t ev_chk_ = nullptr;  // the check's reads have landed
     struct Overlap {
         bool on = false;      // on_drawn is committing a drawn range
         JobRequest rc{};      // that range, as pass 2 commits it
-        uint64_t g0 = 0, g1 = 0, n_records = 0;
+        uint64_t g0 = 0, g1 = 0;
         uint64_t spec_lo = 0, spec_hi = 0;  // pass samples of the journaled round (0, 0: none)
     } ov_;
     cudaEvent_t ev_run_[2] = {nullptr, nullptr};
