@@ -8,6 +8,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <iomanip>
 #include <map>
 #include <mutex>
@@ -946,14 +947,40 @@ int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> 
     return SILVAN_OK;
 }
 
-// Samples the first launch of the next job of this class draws.  Seeds stop
+// Jobs that stop after about as many samples: the same class of graphs and the
+// same accuracy, confidence, mode and sampling rate.  The class alone is too
+// wide: a top-k job's 227,000 samples on a 384 x 384 lattice had the next
+// absolute job on a 511 x 511 one (the same class) draw 65,536 samples where
+// it uses 1,900: 158 ms, against 7 alone.
+uint64_t Engine::job_kind(const DeviceGraph *G, const silvan_params_t &p) {
+    uint64_t h = G->tune_class();
+    auto mix = [&](uint64_t v) {  // 64-bit FNV-1a over words, then a shift
+        h = (h ^ v) * 0x100000001b3ull;
+        h ^= h >> 29;
+    };
+    auto bits = [](double d) {
+        uint64_t u;
+        memcpy(&u, &d, sizeof(u));
+        return u;
+    };
+    mix(bits(p.eps));
+    mix(bits(p.delta));
+    mix(bits(p.alpha));
+    mix(bits(p.a));
+    mix((uint64_t)p.k << 32 | p.threads);
+    mix((p.m_hat ? 1u : 0u) | (p.alpha_given ? 2u : 0u) | (uint64_t)p.form << 8 |
+        (uint64_t)p.backtrack << 32);
+    return h;
+}
+
+// Samples the first launch of the next job of this kind draws.  Seeds stop
 // at different schedule points (on R-MAT scale 20 the totals of 60 seeds
 // spread over +-13 % of their mean), so one earlier total is a noisy guess:
 // with fewer than kHintMin totals recorded, 25 % above the last one; with
 // more, 3 % above the largest of the last kHintJobs, which about one job in
 // kHintJobs + 1 exceeds (it then draws its rest in a second launch).
-uint64_t Engine::job_hint(const DeviceGraph *G) const {
-    auto it = job_total_.find(G->tune_class());
+uint64_t Engine::job_hint(const DeviceGraph *G, const silvan_params_t &p) const {
+    auto it = job_total_.find(job_kind(G, p));
     if (it == job_total_.end() || it->second.empty()) return 0;
     const std::deque<uint64_t> &h = it->second;
     if (h.size() < kHintMin) return h.back() + h.back() / 4;
@@ -961,14 +988,17 @@ uint64_t Engine::job_hint(const DeviceGraph *G) const {
     return mx + mx / 32;
 }
 
-void Engine::note_job(const DeviceGraph *G, uint64_t used, bool alpha_kept) {
+void Engine::note_job(const DeviceGraph *G, const silvan_params_t &p, uint64_t used,
+                      bool alpha_kept) {
+    const uint64_t kind = job_kind(G, p);
     // only a job whose second pass kept the first pass's alpha can use
     // samples drawn ahead in its first launch
     if (!alpha_kept) {
-        job_total_.erase(G->tune_class());
+        job_total_.erase(kind);
         return;
     }
-    std::deque<uint64_t> &h = job_total_[G->tune_class()];
+    if (job_total_.size() >= kHintKinds && !job_total_.count(kind)) job_total_.clear();
+    std::deque<uint64_t> &h = job_total_[kind];
     h.push_back(used);
     while (h.size() > kHintJobs) h.pop_front();
 }
@@ -1020,7 +1050,24 @@ Engine *engine_acquire(uint64_t n, uint32_t slots, int *rc) {
             }
         }
     }
+    // Idle engines for smaller graphs make room for the new one, which serves
+    // their requests too and takes over what they have measured.
+    std::vector<Engine *> old;
+    {
+        std::lock_guard<std::mutex> lk(g_pool_mu);
+        for (size_t i = 0; i < g_pool_free.size();)
+            if (g_pool_free[i].device == dev && g_pool_free[i].requested_slots == slots) {
+                old.push_back(g_pool_free[i].eng);
+                g_pool_free.erase(g_pool_free.begin() + i);
+            } else {
+                i++;
+            }
+    }
     Engine *e = new Engine();
+    for (Engine *o : old) {
+        e->adopt(*o);
+        delete o;
+    }
     *rc = e->init(n, slots, 0);
     if (*rc != SILVAN_OK) {
         // release idle engines of this device and try once more
@@ -1789,7 +1836,7 @@ bool Job::next_request(JobRequest &r) {
         uint64_t ahead = phase_ == kPass2 ? lookahead_
                                           : std::min<uint64_t>(lookahead_tail_, 4 * target_);
         if (phase_ == kPass1 && hint_total_ > target_ && hint_total_ > pass_samples_) {
-            // the earlier jobs of this class of graphs suggest drawing
+            // the earlier jobs of this kind suggest drawing
             // hint_total_ samples (Engine::job_hint) with pass 2 on the same
             // stream: draw that far at once, so that one launch usually
             // covers the whole estimation (a second launch costs more than
@@ -2218,7 +2265,7 @@ int Job::run(silvan_result_t *res, FILE *sink) {
     std::vector<JobRequest> reqs(1);
     std::vector<uint64_t> nrec;
     set_lookahead(own_engine_->free_samples(g_, true), own_engine_->free_samples(g_, false));
-    hint_total_ = own_engine_->job_hint(g_);
+    hint_total_ = own_engine_->job_hint(g_, p_);
     while (!done()) {
         if (!next_request(reqs[0])) {
             set_error("sample index space exhausted");
@@ -2233,9 +2280,9 @@ int Job::run(silvan_result_t *res, FILE *sink) {
         set_lookahead(own_engine_->free_samples(g_, true), own_engine_->free_samples(g_, false));
     }
     RK(finish(res));
-    // the next job of this class of graphs draws about as far in its first
-    // launch (when the second pass kept alpha, so those draws are used)
-    own_engine_->note_job(g_, result_.first_pass_samples + result_.num_samples,
+    // the next job of this kind draws about as far in its first launch (when
+    // the second pass kept alpha, so those draws are used)
+    own_engine_->note_job(g_, p_, result_.first_pass_samples + result_.num_samples,
                           alpha_ == p_.alpha);
     return SILVAN_OK;
 }
@@ -2302,15 +2349,27 @@ int run_batched(const std::vector<Job *> &jobs, uint64_t mem_budget, silvan_resu
     }
     uint32_t slots = 0;
     for (Job *j : jobs) slots = std::max(slots, j->params().slots);
-    Engine eng;
-    RK(eng.init(n_max, slots, mem_budget));
-    // the jobs use the engine's stream only while it exists
-    struct Detach {
+    // A pooled engine, as single jobs use it, unless the caller bounds its
+    // memory.
+    struct Hold {
         const std::vector<Job *> &js;
-        ~Detach() {
+        std::unique_ptr<Engine> own;
+        Engine *pooled = nullptr;
+        ~Hold() {  // the jobs use the engine's stream only while they hold it
             for (Job *j : js) j->detach();
+            engine_release(pooled);
         }
-    } detach{jobs};
+    } hold{jobs, nullptr};
+    if (mem_budget == 0) {
+        int rc = SILVAN_OK;
+        hold.pooled = engine_acquire(n_max, slots, &rc);
+        RK(rc);
+        hold.pooled->reset_timers();
+    } else {
+        hold.own.reset(new Engine());
+        RK(hold.own->init(n_max, slots, mem_budget));
+    }
+    Engine &eng = hold.pooled ? *hold.pooled : *hold.own;
     for (Job *j : jobs) RK(j->begin(sink, eng.stream()));
     std::vector<Job *> act;
     std::vector<JobRequest> reqs;

@@ -156,8 +156,16 @@ class Engine {
     uint32_t free_samples(const DeviceGraph *G, bool tail_only) const;
     // Samples (both passes) the last single-job run on G's class of graphs
     // used, when its second pass kept alpha (0: none recorded)
-    uint64_t job_hint(const DeviceGraph *G) const;
-    void note_job(const DeviceGraph *G, uint64_t used, bool alpha_kept);
+    uint64_t job_hint(const DeviceGraph *G, const silvan_params_t &p) const;
+    void note_job(const DeviceGraph *G, const silvan_params_t &p, uint64_t used, bool alpha_kept);
+    // takes over another engine's measurements of graph classes and job kinds
+    void adopt(Engine &o) {
+        stats_.merge(o.stats_);
+        last_.merge(o.last_);
+        warp_stats_.merge(o.warp_stats_);
+        job_total_.merge(o.job_total_);
+    }
+    static uint64_t job_kind(const DeviceGraph *G, const silvan_params_t &p);
     uint64_t launches() const { return launches_; }
     float sample_ms() const { return sample_ms_; }
     void reset_timers() {
@@ -238,9 +246,10 @@ class Engine {
     };
     std::unordered_map<uint64_t, LastLaunch> last_;  // by tune_class()
     std::unordered_map<uint64_t, WarpStats> warp_stats_;  // by tune_class()
-    // by tune_class(): the samples of the last kHintJobs jobs (see job_hint)
+    // by job_kind(), at most kHintKinds of them: the samples of the last
+    // kHintJobs jobs (see job_hint)
     std::unordered_map<uint64_t, std::deque<uint64_t>> job_total_;
-    static constexpr size_t kHintJobs = 8, kHintMin = 4;
+    static constexpr size_t kHintJobs = 8, kHintMin = 4, kHintKinds = 256;
 };
 
 class Job {
