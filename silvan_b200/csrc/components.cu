@@ -11,11 +11,13 @@
 //     to max over components of ecc_f(pivot) + ecc_b(pivot) = 2 ecc(pivot),
 //     the eccentricity being the distance of the last node of the BFS from
 //     the pivot (compute_ecc_in_scc, :238-270).
-// Components: lock-free union-find over the edges that always links the
-// larger root under the smaller one (so every root is its component's
-// smallest id), then every node's root and a prefix count of the roots.
+// Components: every node starts under its smallest neighbour and the trees are
+// flattened; a lock-free union-find over the edges then links what is left,
+// always the larger root under the smaller one (so every root is its
+// component's smallest id); then every node's root and a prefix count of the
+// roots.
 // Eccentricities: one breadth-first search from all pivots at once (the
-// components are disjoint), level by level.
+// components are disjoint), all levels in one launch.
 //
 // Directed graphs: their component numbers are the completion order of the
 // reference's sequential DFS (the void test of the sampler compares them, so
@@ -28,6 +30,7 @@
 #include <vector>
 
 #include "components.h"
+#include "grid_barrier.cuh"
 
 namespace silvan {
 
@@ -55,33 +58,96 @@ __device__ __forceinline__ uint32_t find_root(uint32_t *parent, uint32_t x) {
     return x;
 }
 
-__global__ void cc_init_kernel(uint32_t *parent, uint32_t n) {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
-        parent[v] = v;
+// A node's smallest neighbour, if that is smaller, is its parent: a forest that
+// needs no links.
+__global__ void cc_init_kernel(const uint32_t *off, const uint32_t *adj, uint32_t *parent,
+                               uint32_t n) {
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n;
+         v += gridDim.x * blockDim.x) {
+        const uint32_t b = off[v], e = off[v + 1];
+        parent[v] = b < e ? min(v, adj[b]) : v;
+    }
 }
 
-// One warp per row: every edge (u, w) unites the two sets.
-__global__ void cc_union_kernel(const uint32_t *off, const uint32_t *adj, uint32_t n,
+// Pointer jumping: every thread moves its node's parent to the grandparent until
+// that is a root, and as the others do the same each step doubles the way.  No
+// links are made meanwhile, so every root found is the tree's.
+__global__ void cc_flatten_kernel(uint32_t *parent, uint32_t n) {
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n;
+         v += gridDim.x * blockDim.x) {
+        uint32_t p = __ldcg(&parent[v]);
+        for (uint32_t gp; (gp = __ldcg(&parent[p])) != p; p = gp) parent[v] = gp;
+    }
+}
+
+// The last row that starts at or before entry k (it holds the entry): a 32-way
+// search by the whole warp.
+__device__ __forceinline__ uint32_t row_of_entry(const uint32_t *off, uint32_t n, uint32_t k) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t l = 0, h = n;  // off[l] <= k, and off[h] > k or h == n
+    while (h - l > 1) {
+        const uint32_t step = (h - l + 31u) / 32u;
+        const uint32_t i = l + lane * step;
+        const uint32_t c = (uint32_t)__popc(
+            __ballot_sync(0xffffffffu, i < h && off[i] <= k));  // lane 0 always counts
+        h = min(h, l + c * step);
+        l = l + (c - 1u) * step;
+    }
+    return l;
+}
+
+// Every edge (u, w) unites the two sets.  A warp takes a chunk of entries wherever
+// they lie, so that rows of 2 and of 100,000 entries keep all lanes busy (with a
+// warp per row the 490,000 rows of a lattice took 356 us; now 58, after 43 for
+// the sample), and knows their rows from the ends of 32 rows, one in each lane.
+__global__ void cc_union_kernel(const uint32_t *off, const uint32_t *adj, uint32_t n, uint32_t m,
                                 uint32_t *parent) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < n; u += warps) {
-        for (uint32_t k = off[u] + lane; k < off[u + 1]; k += 32) {
-            const uint32_t w = adj[k];
-            if (w <= u) continue;  // each undirected edge once
-            uint32_t a = find_root(parent, u), b = find_root(parent, w);
-            while (a != b) {
-                if (a > b) {
-                    const uint32_t t = a;
-                    a = b;
-                    b = t;
+    const uint32_t chunk = min(32u, m / (32u * warps) + 1u) * 32u;  // 32 to 1,024 entries
+    const uint32_t chunks = m / chunk + (m % chunk ? 1u : 0u);
+    for (uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < chunks; c += warps) {
+        uint32_t pos = c * chunk;
+        const uint32_t k1 = min(m - pos, chunk) + pos;
+        uint32_t r = row_of_entry(off, n, pos);
+        uint32_t end = off[min(r + 1u + lane, n)];  // where row r + lane ends
+        while (pos < k1) {
+            uint32_t wend = __shfl_sync(0xffffffffu, end, 31);
+            if (wend <= pos) {
+                r += 32u;
+                end = off[min(r + 1u + lane, n)];
+                wend = __shfl_sync(0xffffffffu, end, 31);
+                if (wend <= pos) {  // many empty rows
+                    r = row_of_entry(off, n, pos);
+                    end = off[min(r + 1u + lane, n)];
+                    wend = __shfl_sync(0xffffffffu, end, 31);
                 }
-                // link the larger root b under the smaller a, if b is still a root
-                const uint32_t old = atomicCAS(&parent[b], b, a);
-                if (old == b) break;
-                a = find_root(parent, a);
-                b = find_root(parent, old);
             }
+            const uint32_t lim = min(k1, wend), k = pos + lane;
+            uint32_t row = 0;  // rows of the window that end at or before k
+#pragma unroll
+            for (uint32_t s = 16; s > 0; s >>= 1)
+                if (__shfl_sync(0xffffffffu, end, row + s - 1u) <= k) row += s;
+            if (lane < lim - pos) {
+                const uint32_t u = r + row, w = adj[k];
+                if (w < u) {  // each undirected edge once
+                    uint32_t a = find_root(parent, u), b = find_root(parent, w);
+                    while (a != b) {
+                        if (a > b) {
+                            const uint32_t t = a;
+                            a = b;
+                            b = t;
+                        }
+                        // link the larger root b under the smaller a, if b is still a root
+                        const uint32_t old = atomicCAS(&parent[b], b, a);
+                        if (old == b) break;
+                        a = find_root(parent, a);
+                        b = find_root(parent, old);
+                    }
+                }
+            }
+            __syncwarp();
+            pos = lim - pos > 32u ? pos + 32u : lim;
         }
     }
 }
@@ -101,6 +167,24 @@ __global__ void cc_compress_kernel(const uint32_t *parent, uint32_t n, uint32_t 
     }
 }
 
+// The largest key of each component, from one (component, key) a lane (of the
+// warp's active lanes, all 32 or the first few): one atomic for a warp whose
+// lanes lie in one component, and only where the key exceeds what is there.
+// 490,000 atomics on the one address of a giant component took 320 us.
+__device__ __forceinline__ void component_max(unsigned long long *best, uint32_t c,
+                                              unsigned long long key) {
+    const uint32_t act = __activemask();
+    bool first = true;
+    if (act == 0xffffffffu && __match_any_sync(0xffffffffu, c) == 0xffffffffu) {
+        const uint32_t hi = __reduce_max_sync(0xffffffffu, (uint32_t)(key >> 32));
+        const uint32_t lo = __reduce_max_sync(
+            0xffffffffu, (uint32_t)(key >> 32) == hi ? (uint32_t)key : 0u);
+        key = (unsigned long long)hi << 32 | lo;
+        first = (threadIdx.x & 31) == 0;
+    }
+    if (first && key > __ldcg(&best[c])) atomicMax(&best[c], key);
+}
+
 // cc[v] = number of roots below v's root; the pivot key of each component:
 // degree sum (2 x degree) in the high word, the inverted id in the low word.
 __global__ void cc_number_kernel(const uint32_t *root, const uint32_t *rank, const uint32_t *off,
@@ -109,48 +193,152 @@ __global__ void cc_number_kernel(const uint32_t *root, const uint32_t *rank, con
         const uint32_t c = rank[root[v]];
         cc[v] = c;
         const unsigned long long deg2 = 2ull * (off[v + 1] - off[v]);
-        atomicMax(&pivot_key[c], (deg2 << 32) | (0xffffffffull - v));
+        component_max(pivot_key, c, (deg2 << 32) | (0xffffffffull - v));
     }
 }
 
-__global__ void bfs_seed_kernel(const unsigned long long *pivot_key, uint32_t ncomp, int32_t *dist,
-                                uint32_t *frontier) {
+__global__ void bfs_seed_kernel(const unsigned long long *pivot_key, uint32_t ncomp,
+                                uint32_t *seen, uint32_t *queue) {
     for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < ncomp;
          c += gridDim.x * blockDim.x) {
         const uint32_t p = 0xffffffffu - (uint32_t)(pivot_key[c] & 0xffffffffull);
-        dist[p] = 0;
-        frontier[c] = p;
+        seen[p] = 1;
+        queue[c] = p;
     }
 }
 
-// One warp per frontier node: unvisited neighbours join the next level.
-__global__ void bfs_level_kernel(const uint32_t *off, const uint32_t *adj, const uint32_t *frontier,
-                                 uint32_t count, int32_t level, int32_t *dist, uint32_t *next,
-                                 uint32_t *next_count) {
+// The breadth-first searches from all pivots at once, each inside its component
+// (the components are disjoint; where edges lead out of a component, cc keeps
+// the search inside), in one cooperative launch: a lattice has a hundred levels
+// of a few hundred nodes, and a launch, a copy of the count and a wait for it
+// took 25 us for each where a level in here takes 5 (one CTA of 512 threads an
+// SM: 492 us for all of 490,000 nodes; of 1,024: 620, of 128: 581).
+//
+// queue holds the pivots and gets every node once; a level is the part that the
+// level before appended.  A warp takes a few nodes of the level, as many as
+// leave no warp without work (at most 32), and goes through their entries 32 at
+// a time; rows of more than kLongRow entries are left to all warps together
+// after the others.  Counts are kept three levels apart, so that the one being
+// zeroed is not read any more and not yet appended to.
+//
+// ctl: [0..2] nodes appended, [3..5] long rows, [6] the barrier, [8] the
+// deepest level, [9] set when a wait gave up.  ecc (where given) gets each
+// component's eccentricity.
+constexpr int kBfsThreads = 512;
+constexpr uint32_t kLongRow = 2048;
+constexpr uint32_t kBfsCtl = 10;
+constexpr uint32_t kBfsPolls = 1u << 26;  // a minute: a level may hold all of a large graph
+
+struct BfsArgs {
+    const uint32_t *off, *adj;
+    const uint32_t *cc;  // null: no edge leaves a component
+    uint32_t *queue, *seen, *long_rows, *ctl;
+    int32_t *ecc;  // null: not wanted
+    uint32_t ncomp;
+};
+
+// One entry a lane: nodes not seen yet join the next level.
+// `look` spares the atomic where a look shows the node was seen; on a narrow
+// level the look is one more wait in a chain of waits.
+__device__ __forceinline__ void bfs_visit(const BfsArgs &a, bool act, uint32_t k, uint32_t cu,
+                                          int32_t level, bool look, uint32_t *next,
+                                          uint32_t *next_count) {
+    bool join = false;
+    uint32_t w = 0;
+    if (act) {
+        w = a.adj[k];
+        join = (!a.cc || a.cc[w] == cu) && (!look || __ldcg(&a.seen[w]) == 0u) &&
+               atomicExch(&a.seen[w], 1u) == 0u;
+    }
+    const uint32_t mask = __ballot_sync(0xffffffffu, join);
+    if (!mask) return;
     const uint32_t lane = threadIdx.x & 31;
+    uint32_t at = 0;
+    if (lane == 0) at = atomicAdd(next_count, (uint32_t)__popc(mask));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (join) {
+        next[at + (uint32_t)__popc(mask & ((1u << lane) - 1u))] = w;
+        if (a.ecc) a.ecc[cu] = level + 1;  // levels rise: the last one written stays
+    }
+}
+
+__global__ void __launch_bounds__(kBfsThreads, 1) bfs_kernel(const BfsArgs a) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < count; i += warps) {
-        const uint32_t u = frontier[i];
-        for (uint32_t k = off[u] + lane; k < off[u + 1]; k += 32) {
-            const uint32_t w = adj[k];
-            if (__ldcg(&dist[w]) >= 0) continue;
-            if (atomicCAS(&dist[w], -1, level + 1) == -1) next[atomicAdd(next_count, 1u)] = w;
+    uint32_t count = a.ncomp, lo = 0, passed = 0;
+    int32_t level = 0;
+    for (;; level++) {
+        const uint32_t now = (uint32_t)level % 3u, nxt = (now + 1u) % 3u, old = (now + 2u) % 3u;
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            a.ctl[old] = 0u;
+            a.ctl[3u + nxt] = 0u;
+        }
+        uint32_t *next = a.queue + lo + count, *next_count = &a.ctl[nxt];
+        const uint32_t group = min(32u, count / warps + (count % warps ? 1u : 0u));
+        for (uint32_t i0 = warp * group; i0 < count; i0 += warps * group) {
+            uint32_t b = 0, len = 0, cu = 0;
+            if (lane < group && i0 + lane < count) {
+                const uint32_t u = __ldcg(&a.queue[lo + i0 + lane]);
+                b = a.off[u];
+                len = a.off[u + 1] - b;
+                if (a.cc) cu = a.cc[u];
+                if (len > kLongRow) {
+                    a.long_rows[atomicAdd(&a.ctl[3u + now], 1u)] = u;
+                    len = 0;
+                }
+            }
+            uint32_t ends = len;  // inclusive prefix
+#pragma unroll
+            for (uint32_t o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, ends, o);
+                if (lane >= o) ends += y;
+            }
+            const uint32_t total = __shfl_sync(0xffffffffu, ends, 31);
+            for (uint32_t it = 0; it < total; it += 32u) {
+                const uint32_t item = it + lane;
+                uint32_t row = 0;
+#pragma unroll
+                for (uint32_t s = 16; s > 0; s >>= 1)
+                    if (__shfl_sync(0xffffffffu, ends, row + s - 1u) <= item) row += s;
+                const uint32_t k = __shfl_sync(0xffffffffu, b + len - ends, row) + item;
+                const uint32_t c = __shfl_sync(0xffffffffu, cu, row);
+                bfs_visit(a, item < total, k, c, level, group > 8u, next, next_count);
+            }
+        }
+        if (!grid_barrier_to(a.ctl + 6, passed += gridDim.x, kBfsPolls)) break;
+        const uint32_t nl = __ldcg(&a.ctl[3u + now]);
+        if (nl) {
+            for (uint32_t j = 0; j < nl; j++) {
+                const uint32_t u = __ldcg(&a.long_rows[j]);
+                const uint32_t b = a.off[u], len = a.off[u + 1] - b;
+                const uint32_t c = a.cc ? a.cc[u] : 0u;
+                for (uint32_t i = warp * 32u; i < len; i += warps * 32u)
+                    bfs_visit(a, i + lane < len, b + i + lane, c, level, true, next, next_count);
+            }
+            if (!grid_barrier_to(a.ctl + 6, passed += gridDim.x, kBfsPolls)) break;
+        }
+        lo += count;
+        count = __ldcg(next_count);
+        if (count == 0u) {
+            if (blockIdx.x == 0 && threadIdx.x == 0) a.ctl[8] = (uint32_t)level;
+            return;
         }
     }
+    if (threadIdx.x == 0) atomicExch(&a.ctl[9], 1u);
 }
 
-__global__ void ecc_kernel(const int32_t *dist, const uint32_t *cc, uint32_t n, int32_t *ecc) {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
-        atomicMax(&ecc[cc[v]], dist[v]);
-}
-
-__global__ void diam_kernel(const int32_t *ecc, uint32_t ncomp, unsigned int *diam) {
-    uint32_t mx = 0;
-    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < ncomp;
-         c += gridDim.x * blockDim.x)
-        mx = max(mx, 2u * (uint32_t)ecc[c]);
-    for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(diam, mx);
+// Queues the search from the ncomp seeded pivots.
+cudaError_t launch_bfs(const BfsArgs &a, cudaStream_t st) {
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaMemsetAsync(a.ctl, 0, 4 * kBfsCtl, st);
+    if (e != cudaSuccess) return e;
+    BfsArgs args = a;
+    void *params[] = {&args};
+    return cudaLaunchCooperativeKernel((const void *)bfs_kernel, dim3((unsigned)sms),
+                                       dim3(kBfsThreads), params, 0, st);
 }
 
 // ---- directed graphs: the diameter bound over given component ids --------
@@ -161,37 +349,7 @@ __global__ void dir_pivot_kernel(const uint32_t *oo, const uint32_t *io, const u
                                  uint32_t n, unsigned long long *pivot_key) {
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
         const unsigned long long d = (unsigned long long)(oo[v + 1] - oo[v]) + (io[v + 1] - io[v]);
-        atomicMax(&pivot_key[cc[v]], (d << 32) | (0xffffffffull - v));
-    }
-}
-
-__global__ void dir_seed_kernel(const unsigned long long *pivot_key, uint32_t ncomp,
-                                int32_t *dist_f, int32_t *dist_b, uint32_t *frontier) {
-    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < ncomp;
-         c += gridDim.x * blockDim.x) {
-        const uint32_t p = 0xffffffffu - (uint32_t)(pivot_key[c] & 0xffffffffull);
-        dist_f[p] = 0;
-        dist_b[p] = 0;
-        frontier[c] = p;
-    }
-}
-
-// One level of the breadth-first searches from every pivot at once, each
-// staying inside its pivot's component (the components are disjoint, so the
-// searches never meet).
-__global__ void dir_bfs_level_kernel(const uint32_t *off, const uint32_t *adj, const uint32_t *cc,
-                                     const uint32_t *frontier, uint32_t count, int32_t level,
-                                     int32_t *dist, uint32_t *next, uint32_t *next_count) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < count; i += warps) {
-        const uint32_t u = frontier[i];
-        const uint32_t cu = cc[u];
-        for (uint32_t k = off[u] + lane; k < off[u + 1]; k += 32) {
-            const uint32_t w = adj[k];
-            if (cc[w] != cu || __ldcg(&dist[w]) >= 0) continue;
-            if (atomicCAS(&dist[w], -1, level + 1) == -1) next[atomicAdd(next_count, 1u)] = w;
-        }
+        component_max(pivot_key, cc[v], (d << 32) | (0xffffffffull - v));
     }
 }
 
@@ -255,15 +413,15 @@ int device_directed_bound(DeviceGraph &G, cudaStream_t st) {
         if (rc == SILVAN_OK) bufs.push_back(*p);
         return rc;
     };
-    uint32_t *frontier = nullptr, *next = nullptr, *cnt = nullptr, *flag = nullptr;
-    int32_t *dist_f = nullptr, *dist_b = nullptr, *ecc_f = nullptr, *ecc_b = nullptr, *fp = nullptr;
+    uint32_t *queue = nullptr, *seen = nullptr, *long_rows = nullptr, *ctl = nullptr,
+             *flag = nullptr;
+    int32_t *ecc_f = nullptr, *ecc_b = nullptr, *fp = nullptr;
     unsigned long long *pivot_key = nullptr, *n_inter = nullptr;
     unsigned int *d_diam = nullptr;
-    CC_RK(get((void **)&dist_f, 4ull * n));
-    CC_RK(get((void **)&dist_b, 4ull * n));
-    CC_RK(get((void **)&frontier, 4ull * n));
-    CC_RK(get((void **)&next, 4ull * n));
-    CC_RK(get((void **)&cnt, 16));
+    CC_RK(get((void **)&queue, 4ull * n));
+    CC_RK(get((void **)&seen, 4ull * n));
+    CC_RK(get((void **)&long_rows, 4ull * (std::max(G.m, G.m_in) / kLongRow + 1)));
+    CC_RK(get((void **)&ctl, 4ull * 2 * kBfsCtl));
     CC_RK(get((void **)&flag, 16));
     CC_RK(get((void **)&n_inter, 8));
     CC_RK(get((void **)&d_diam, 4));
@@ -274,33 +432,21 @@ int device_directed_bound(DeviceGraph &G, cudaStream_t st) {
     CC_CK(cudaMemsetAsync(pivot_key, 0, 8ull * ncomp, st));
     CC_CK(cudaMemsetAsync(ecc_f, 0, 4ull * ncomp, st));
     CC_CK(cudaMemsetAsync(ecc_b, 0, 4ull * ncomp, st));
-    CC_CK(cudaMemsetAsync(dist_f, 0xff, 4ull * n, st));
-    CC_CK(cudaMemsetAsync(dist_b, 0xff, 4ull * n, st));
     CC_CK(cudaMemsetAsync(d_diam, 0, 4, st));
     CC_CK(cudaMemsetAsync(n_inter, 0, 8, st));
     CC_CK(cudaMemsetAsync(flag, 0, 16, st));
     dir_pivot_kernel<<<592, 256, 0, st>>>(G.d_out_off, G.d_in_off, G.d_cc, n, pivot_key);
-    dir_seed_kernel<<<64, 256, 0, st>>>(pivot_key, ncomp, dist_f, dist_b, frontier);
     CC_CK(cudaGetLastError());
     // eccentricity of every pivot inside its component, forward then backward
     // (compute_ecc_in_scc, silvan/src/Graph.cpp:238-270)
     for (int dir = 0; dir < 2; dir++) {
-        const uint32_t *off = dir == 0 ? G.d_out_off : G.d_in_off;
-        const uint32_t *adj = dir == 0 ? G.d_out_adj : G.d_in_adj;
-        int32_t *dist = dir == 0 ? dist_f : dist_b;
-        if (dir == 1) dir_seed_kernel<<<64, 256, 0, st>>>(pivot_key, ncomp, dist_f, dist_b, frontier);
-        uint32_t count = ncomp;
-        for (int32_t level = 0; count > 0; level++) {
-            CC_CK(cudaMemsetAsync(cnt, 0, 4, st));
-            dir_bfs_level_kernel<<<1184, 256, 0, st>>>(off, adj, G.d_cc, frontier, count, level,
-                                                       dist, next, cnt);
-            CC_CK(cudaGetLastError());
-            CC_CK(cudaMemcpyAsync(&count, cnt, 4, cudaMemcpyDeviceToHost, st));
-            CC_CK(cudaStreamSynchronize(st));
-            std::swap(frontier, next);
-        }
-        ecc_kernel<<<592, 256, 0, st>>>(dist, G.d_cc, n, dir == 0 ? ecc_f : ecc_b);
+        CC_CK(cudaMemsetAsync(seen, 0, 4ull * n, st));
+        bfs_seed_kernel<<<64, 256, 0, st>>>(pivot_key, ncomp, seen, queue);
         CC_CK(cudaGetLastError());
+        CC_CK(launch_bfs(BfsArgs{dir == 0 ? G.d_out_off : G.d_in_off,
+                                 dir == 0 ? G.d_out_adj : G.d_in_adj, G.d_cc, queue, seen,
+                                 long_rows, ctl + dir * kBfsCtl, dir == 0 ? ecc_f : ecc_b, ncomp},
+                         st));
     }
     // the recursion over the condensation
     const uint64_t m = G.m;
@@ -310,10 +456,15 @@ int device_directed_bound(DeviceGraph &G, cudaStream_t st) {
                                            flag + 1);
     CC_CK(cudaMemcpyAsync(fp, ecc_f, 4ull * ncomp, cudaMemcpyDeviceToDevice, st));
     unsigned long long mi = 0;
-    uint32_t badf = 0;
+    uint32_t badf = 0, bfs[2 * kBfsCtl];
+    CC_CK(cudaMemcpyAsync(bfs, ctl, sizeof(bfs), cudaMemcpyDeviceToHost, st));
     CC_CK(cudaMemcpyAsync(&mi, n_inter, 8, cudaMemcpyDeviceToHost, st));
     CC_CK(cudaMemcpyAsync(&badf, flag + 1, 4, cudaMemcpyDeviceToHost, st));
     CC_CK(cudaStreamSynchronize(st));
+    if (bfs[9] || bfs[kBfsCtl + 9]) {
+        set_error("the breadth-first searches of the diameter bound did not end");
+        return SILVAN_E_TIMEOUT;
+    }
     if (badf || mi > m) {
         set_error("component ids are not in the reference's completion order");
         return SILVAN_E_STATE;
@@ -369,25 +520,31 @@ int device_undirected_components(DeviceGraph &G, cudaStream_t st) {
         return rc;
     };
     uint32_t *parent = nullptr, *root = nullptr, *is_root = nullptr, *rank = nullptr,
-             *frontier = nullptr, *next = nullptr, *cnt = nullptr;
-    int32_t *dist = nullptr, *ecc = nullptr;
+             *queue = nullptr, *seen = nullptr, *long_rows = nullptr, *ctl = nullptr;
     unsigned long long *pivot_key = nullptr;
-    unsigned int *d_diam = nullptr;
     CC_RK(get((void **)&parent, 4ull * n));
     CC_RK(get((void **)&root, 4ull * n));
     CC_RK(get((void **)&is_root, 4ull * n));
     CC_RK(get((void **)&rank, 4ull * (n + 1)));
-    CC_RK(get((void **)&dist, 4ull * n));
-    CC_RK(get((void **)&frontier, 4ull * n));
-    CC_RK(get((void **)&next, 4ull * n));
-    CC_RK(get((void **)&cnt, 4));
-    CC_RK(get((void **)&d_diam, 4));
+    CC_RK(get((void **)&queue, 4ull * n));
+    CC_RK(get((void **)&seen, 4ull * n));
+    CC_RK(get((void **)&long_rows, 4ull * (G.m / kLongRow + 1)));
+    CC_RK(get((void **)&ctl, 4ull * kBfsCtl));
     uint32_t *d_cc = nullptr;
     CC_RK(device_alloc((void **)&d_cc, 4ull * n));  // owned by the graph
     G.d_cc = d_cc;
 
-    cc_init_kernel<<<592, 256, 0, st>>>(parent, n);
-    cc_union_kernel<<<1184, 256, 0, st>>>(G.d_out_off, G.d_out_adj, n, parent);
+    cc_init_kernel<<<1184, 256, 0, st>>>(G.d_out_off, G.d_out_adj, parent, n);
+    cc_flatten_kernel<<<1184, 256, 0, st>>>(parent, n);
+    // A 32nd of the entries first: with all of them at once, hundreds of thousands
+    // of lanes would find the same few roots apart and fight over the links
+    // (the lattice of 490,000 nodes: 338 us in one go, 43 + 9 + 58 this way).
+    const uint32_t m = (uint32_t)G.m;
+    if (m / 32) {
+        cc_union_kernel<<<1184, 256, 0, st>>>(G.d_out_off, G.d_out_adj, n, m / 32, parent);
+        cc_flatten_kernel<<<1184, 256, 0, st>>>(parent, n);
+    }
+    if (m) cc_union_kernel<<<1184, 256, 0, st>>>(G.d_out_off, G.d_out_adj, n, m, parent);
     cc_compress_kernel<<<592, 256, 0, st>>>(parent, n, root, is_root);
     CC_CK(cudaGetLastError());
     size_t tb = 0;
@@ -401,30 +558,24 @@ int device_undirected_components(DeviceGraph &G, cudaStream_t st) {
     CC_CK(cudaStreamSynchronize(st));
     const uint32_t ncomp = last_rank + last_root;
     CC_RK(get((void **)&pivot_key, 8ull * ncomp));
-    CC_RK(get((void **)&ecc, 4ull * ncomp));
     CC_CK(cudaMemsetAsync(pivot_key, 0, 8ull * ncomp, st));
-    CC_CK(cudaMemsetAsync(ecc, 0, 4ull * ncomp, st));
-    CC_CK(cudaMemsetAsync(dist, 0xff, 4ull * n, st));
-    CC_CK(cudaMemsetAsync(d_diam, 0, 4, st));
+    CC_CK(cudaMemsetAsync(seen, 0, 4ull * n, st));
     cc_number_kernel<<<592, 256, 0, st>>>(root, rank, G.d_out_off, n, d_cc, pivot_key);
-    bfs_seed_kernel<<<64, 256, 0, st>>>(pivot_key, ncomp, dist, frontier);
+    bfs_seed_kernel<<<64, 256, 0, st>>>(pivot_key, ncomp, seen, queue);
     CC_CK(cudaGetLastError());
-    uint32_t count = ncomp;
-    for (int32_t level = 0; count > 0; level++) {
-        CC_CK(cudaMemsetAsync(cnt, 0, 4, st));
-        bfs_level_kernel<<<1184, 256, 0, st>>>(G.d_out_off, G.d_out_adj, frontier, count, level,
-                                               dist, next, cnt);
-        CC_CK(cudaGetLastError());
-        CC_CK(cudaMemcpyAsync(&count, cnt, 4, cudaMemcpyDeviceToHost, st));
-        CC_CK(cudaStreamSynchronize(st));
-        std::swap(frontier, next);
-    }
-    ecc_kernel<<<592, 256, 0, st>>>(dist, d_cc, n, ecc);
-    diam_kernel<<<64, 256, 0, st>>>(ecc, ncomp, d_diam);
-    CC_CK(cudaGetLastError());
-    unsigned int diam = 0;
-    CC_CK(cudaMemcpyAsync(&diam, d_diam, 4, cudaMemcpyDeviceToHost, st));
+    CC_CK(launch_bfs(BfsArgs{G.d_out_off, G.d_out_adj, nullptr, queue, seen, long_rows, ctl,
+                             nullptr, ncomp},
+                     st));
+    uint32_t bfs[kBfsCtl];
+    CC_CK(cudaMemcpyAsync(bfs, ctl, sizeof(bfs), cudaMemcpyDeviceToHost, st));
     CC_CK(cudaStreamSynchronize(st));
+    if (bfs[9]) {
+        set_error("the breadth-first searches of the diameter bound did not end");
+        return SILVAN_E_TIMEOUT;
+    }
+    // max over components of 2 ecc(pivot): the searches run side by side, so the
+    // deepest level is the largest eccentricity
+    const unsigned int diam = 2u * bfs[8];
     G.ncomp = ncomp;
     G.diameter = diam;
     return SILVAN_OK;

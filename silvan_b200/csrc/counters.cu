@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "counters.cuh"
+#include "grid_barrier.cuh"
 
 namespace silvan {
 
@@ -50,42 +51,6 @@ constexpr uint32_t kBarrierPolls = 1u << 22;  // far above any real wait (micros
 
 __device__ __forceinline__ uint32_t round_records(const RoundBuffers &rb, const ApplyArgs &a) {
     return (uint32_t)min((uint64_t)a.n_records, rb.rec_cap);
-}
-
-__device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p) {
-    uint32_t v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ void st_release(uint32_t *p, uint32_t v) {
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// Grid-wide barrier over bar[0] (arrivals) and bar[1] (generation); false
-// when this CTA gave up waiting.
-__device__ bool grid_barrier(uint32_t *bar) {
-    __syncthreads();
-    int ok = 1;
-    if (threadIdx.x == 0) {
-        const uint32_t gen = ld_acquire(&bar[1]);
-        __threadfence();
-        if (atomicAdd(&bar[0], 1u) == gridDim.x - 1) {
-            bar[0] = 0u;
-            __threadfence();
-            st_release(&bar[1], gen + 1u);
-        } else {
-            uint32_t i = 0;
-            while (ld_acquire(&bar[1]) == gen) {
-                if (++i > kBarrierPolls) {
-                    ok = 0;
-                    break;
-                }
-                __nanosleep(32);
-            }
-        }
-    }
-    return __syncthreads_and(ok) != 0;
 }
 
 __device__ void bucket_count(const RoundBuffers &rb, const ApplyArgs &a) {
@@ -353,13 +318,13 @@ __global__ void __launch_bounds__(kCommitThreads, 1) prepare_draw_kernel(const A
     const ApplyArgs &a = st.a;
     uint32_t *bar = rb.n_touched + 2;
     bucket_count(rb, a);
-    if (!grid_barrier(bar)) goto timeout;
+    if (!grid_barrier(bar, kBarrierPolls)) goto timeout;
     {
         const uint32_t T = __ldcg(rb.n_touched);
         bucket_alloc(rb, T);
-        if (!grid_barrier(bar)) goto timeout;
+        if (!grid_barrier(bar, kBarrierPolls)) goto timeout;
         bucket_scatter(rb, a);
-        if (!grid_barrier(bar)) goto timeout;
+        if (!grid_barrier(bar, kBarrierPolls)) goto timeout;
         order_huge(rb, jc, a.count, sm);
         order_others(rb, T, sm);
         // the scatter cursors back to zero for the next draw
