@@ -612,11 +612,12 @@ void Engine::drop_execs() {
 }
 
 // The round's kernels (round_begin, the warp sampler when it is used, the CTA
-// sampler) captured once per (CTA size, grid, warp sampler) and replayed with
+// sampler) captured once per (CTA size, grid, warp sampler, near states) and replayed with
 // new segments.
-int Engine::sampler_exec(int block, uint32_t grid, bool warp, cudaGraphExec_t *out) {
+int Engine::sampler_exec(int block, uint32_t grid, bool warp, uint32_t near_cap,
+                         cudaGraphExec_t *out) {
     for (const Exec &x : execs_)
-        if (x.block == block && x.grid == grid && x.warp == warp) {
+        if (x.block == block && x.grid == grid && x.warp == warp && x.near_cap == near_cap) {
             *out = x.exec;
             return SILVAN_OK;
         }
@@ -626,6 +627,7 @@ int Engine::sampler_exec(int block, uint32_t grid, bool warp, cudaGraphExec_t *o
     L.hdr = d_hdr_;
     L.segs = d_segs_;
     L.assist = board_;
+    L.near_cap = near_cap;
     WarpLaunch WL{};
     if (warp) {
         L.list = warps_.list;
@@ -650,8 +652,8 @@ int Engine::sampler_exec(int block, uint32_t grid, bool warp, cudaGraphExec_t *o
     cudaError_t e4 = cudaGraphInstantiate(&x, g, 0);
     cudaGraphDestroy(g);
     CK(e4);
-    if (execs_.size() >= 16) drop_execs();
-    execs_.push_back(Exec{block, grid, warp, x});
+    if (execs_.size() >= 32) drop_execs();
+    execs_.push_back(Exec{block, grid, warp, near_cap, x});
     *out = x;
     return SILVAN_OK;
 }
@@ -852,7 +854,11 @@ int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> 
         drop_execs();
     }
     cudaGraphExec_t exec = nullptr;
-    RK(sampler_exec(block, grid, warp, &exec));
+    uint64_t n_near = 0;  // the largest graph whose nodes' states fit in shared memory
+    for (uint32_t i : idx)
+        if (jobs[i]->graph()->n <= sampler_near_max(block))
+            n_near = std::max<uint64_t>(n_near, jobs[i]->graph()->n);
+    RK(sampler_exec(block, grid, warp, n_near ? sampler_near_cap(n_near, block) : 0u, &exec));
     for (;;) {
         CK(cudaMemcpyAsync(d_segs_, h_segs_, sizeof(SegDesc) * idx.size(),
                            cudaMemcpyHostToDevice, stream_));

@@ -209,12 +209,14 @@ class Engine {
         int block;
         uint32_t grid;
         bool warp;  // the warp sampler first
+        uint32_t near_cap;
         cudaGraphExec_t exec;
     };
     int ensure_segs(uint32_t nsegs);
     int choose_block(const std::vector<Job *> &jobs, const std::vector<JobRequest> &reqs,
                      const std::vector<uint32_t> &idx, uint32_t total) const;
-    int sampler_exec(int block, uint32_t grid, bool warp, cudaGraphExec_t *out);
+    int sampler_exec(int block, uint32_t grid, bool warp, uint32_t near_cap,
+                     cudaGraphExec_t *out);
     void drop_execs();
     SlotPool slots_;
     WarpPool warps_;

@@ -38,7 +38,11 @@ namespace silvan {
 
 namespace {
 
-constexpr int kItems = 4;        // scan items per lane per tile
+// Scan items per lane per tile.  A tile costs a warp about as many instructions
+// for an empty slot as for a full one, and most levels hold a few hundred
+// entries; with 4, R-MAT 16 samples took 4.0 ms instead of 3.5 and a 384 x 384
+// lattice 222 instead of 187.
+constexpr int kItems = 2;
 // Samples a CTA takes from the round at once while many are left; one
 // thread each draws the endpoints and runs the void test, so the void
 // samples (most of them on sparse directed graphs) cost a fraction of a
@@ -102,6 +106,7 @@ struct SamplerSmem {
     uint32_t a_ok;     // the tile's waits ended
     uint32_t a_drained, a_polls, a_nap;  // no sample left; board polls since; next nap (ns)
     uint32_t a_spin;    // polls of a bounded wait (RoundHeader::wait_polls)
+    uint32_t light;     // nodes joined by last_tile
     uint32_t a_leave;   // a shared level of this CTA's sample failed: take no more samples
     // samples taken from the round in a chunk and screened in parallel: the
     // void ones are finished at once, the others wait here
@@ -109,6 +114,30 @@ struct SamplerSmem {
     uint32_t pend_w[kScreen], pend_u[kScreen], pend_v[kScreen], pend_d[kScreen];
     uint32_t pend_n, pend_i, scr_w0, scr_v;
 };
+
+// States of the nodes, two bits each, behind SamplerSmem, for graphs of at most
+// SamplerLaunch::near_cap nodes: 0 not visited, kSideU or kSideV, 3 joined in
+// the level that is being expanded.  A copy of what the slot's records say: a
+// probe is a shared-memory read instead of a 32-byte sector of its own, most of
+// them missed in L2 (592 slots of 65,536 records: 1.2 GB).
+template <int BLOCK>
+struct Near {
+    static constexpr size_t kOffset = (sizeof(SamplerSmem<BLOCK>) + 15) & ~(size_t)15;
+};
+template <int BLOCK>
+__device__ __forceinline__ uint32_t *near_states() {
+    extern __shared__ __align__(16) unsigned char sampler_smem[];
+    return reinterpret_cast<uint32_t *>(sampler_smem + Near<BLOCK>::kOffset);
+}
+template <int BLOCK>
+__device__ __forceinline__ uint32_t near_get(uint32_t y) {
+    return near_states<BLOCK>()[y >> 4] >> (2u * (y & 15u)) & 3u;
+}
+// From 0 to c, or (c = a ^ b) from a to b.
+template <int BLOCK>
+__device__ __forceinline__ void near_xor(uint32_t y, uint32_t c) {
+    atomicXor(&near_states<BLOCK>()[y >> 4], c << (2u * (y & 15u)));
+}
 
 // Exclusive block scan of one value per thread; returns the block total.
 // tmp needs kWarps + 1 entries.
@@ -176,7 +205,7 @@ constexpr uint32_t kNoNode = 0xffffffffu;
 // most half as many nodes as the table has entries.
 template <int BLOCK>
 __device__ __forceinline__ uint32_t tile_slot(uint32_t *keys, uint32_t y) {
-    constexpr int kLog = BLOCK == 128 ? 10 : BLOCK == 256 ? 11 : BLOCK == 512 ? 12 : 13;
+    constexpr int kLog = BLOCK == 128 ? 9 : BLOCK == 256 ? 10 : BLOCK == 512 ? 11 : 12;
     static_assert((1 << kLog) == Shape<BLOCK>::kHash, "table size");
     uint32_t h = (y * 2654435769u) >> (32 - kLog);
     for (int i = 0; i < Shape<BLOCK>::kHash; i++) {
@@ -333,6 +362,71 @@ __device__ __forceinline__ void record_hit(NodeRec *r, uint32_t g, uint32_t x,
     atomicAdd(reinterpret_cast<unsigned long long *>(&r->sigma), sg);
 }
 
+// A tile of a level that has a meeting edge already, so the search's last: its
+// joined nodes are never expanded, and no path goes through them (a path's edge
+// between the sides starts on the frontier), so they need no record, no queue
+// position and no degree.  What is left is to mark and count them, to count
+// the hits and to append the meeting edges in item order.  On power-law graphs
+// the last level holds most of a search's edges: 86,700 samples of R-MAT 16 took
+// 7.0 ms, 6.6 with the states in shared memory (and two items a lane), and take
+// 3.5 with these tiles; without the states 7.1, as every mark is then an atomic
+// on a record that comes from memory.
+template <int BLOCK>
+__device__ __forceinline__ void last_tile(SamplerSmem<BLOCK> &s, NodeRec *rec, uint32_t *queue,
+                                          uint2 *meet, uint32_t new_st, bool near,
+                                          const uint32_t (&ys)[kItems], uint32_t (&code)[kItems],
+                                          const uint32_t (&li)[kItems], uint32_t &qend,
+                                          uint32_t &mend, uint32_t &hits, uint32_t t0) {
+    constexpr int kWarps = Shape<BLOCK>::kWarps;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // the two tiles at a barrier write different counts
+    uint32_t *counts = (t0 / (uint32_t)Shape<BLOCK>::kTile) & 1u ? s.warp_a : s.warp_b;
+    uint32_t rm[kItems];
+    bool any = false;
+#pragma unroll
+    for (int k = 0; k < kItems; k++) {
+        bool join = false;
+        if (code[k] == 1 || code[k] == 4) hits++;
+        if (code[k] == 1) {
+            if (near) {
+                const uint32_t sh = 2u * (ys[k] & 15u);
+                join = (atomicOr(&near_states<BLOCK>()[ys[k] >> 4], 3u << sh) >> sh & 3u) == 0u;
+            } else {
+                join = atomicCAS(&rec[ys[k]].st, 0u, new_st) == 0u;
+            }
+        }
+        const uint32_t bn = __ballot_sync(0xffffffffu, join);
+        const uint32_t bm = __ballot_sync(0xffffffffu, code[k] == 2);
+        if (bn) {
+            uint32_t at = 0;
+            if (lane == 0) at = atomicAdd(&s.light, (uint32_t)__popc(bn));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            // the records of these are put back from the queue, in any order
+            if (!near && join) queue[qend + at + __popc(bn & lanemask_lt())] = ys[k];
+        }
+        rm[k] = __popc(bm & lanemask_lt());
+        any = any || bm != 0u;
+        if (lane == 0) counts[k * kWarps + warp] = __popc(bm);
+    }
+    __syncwarp();
+    if (__syncthreads_or(any) == 0) return;
+    uint32_t at = mend, all = 0;
+    for (int e = lane; e < kItems * kWarps; e += 32) all += counts[e];
+    all = __reduce_add_sync(0xffffffffu, all);
+#pragma unroll
+    for (int k = 0; k < kItems; k++) {
+        uint32_t before = 0;
+        for (int e = lane; e < k * kWarps + warp; e += 32) before += counts[e];
+        before = __reduce_add_sync(0xffffffffu, before);
+        if (code[k] == 2) {
+            const uint32_t pos = at + before + rm[k];
+            if (pos < kMeetCap) meet[pos] = make_uint2(s.f_node[li[k]], ys[k]);
+        }
+    }
+    if (threadIdx.x == 0 && mend + all > kMeetCap && s.status == 0) s.status = SILVAN_E_CAPACITY;
+    mend = min(mend + all, kMeetCap);
+}
+
 // Expands one BFS level of `side` (silvan/src/Sp_sampler.cpp:89-143).
 //
 // The level is latency-bound on deep, narrow searches (a grid's ~200 levels
@@ -344,7 +438,7 @@ __device__ __forceinline__ void record_hit(NodeRec *r, uint32_t g, uint32_t x,
 template <int BLOCK>
 __device__ void expand_level(const SegDesc &A, SamplerSmem<BLOCK> &s, NodeRec *rec,
                              uint32_t *queue, uint2 *meet, uint32_t side, uint32_t lo,
-                             uint32_t hi, uint32_t depth) {
+                             uint32_t hi, uint32_t depth, bool near) {
     constexpr int kWarps = Shape<BLOCK>::kWarps;
     constexpr int kTile = Shape<BLOCK>::kTile;
     constexpr int kChunk = Shape<BLOCK>::kChunk;
@@ -359,6 +453,10 @@ __device__ void expand_level(const SegDesc &A, SamplerSmem<BLOCK> &s, NodeRec *r
     // ends of the queue and of the meeting list, advanced tile by tile in
     // every thread alike (thread 0 stores them when the level is done)
     uint32_t qend = s.end_q, mend = s.nmeet;
+    // the nodes [q0, marked) of the queue have state 3 for now
+    const uint32_t q0 = qend;
+    uint32_t marked = qend;
+    const uint32_t mend0 = mend;
     for (uint32_t c0 = lo; c0 < hi; c0 += kChunk) {
         const uint32_t nc = min((uint32_t)kChunk, hi - c0);
         // stage the chunk: row starts, degrees (prefix), sigma; nodes without
@@ -432,8 +530,16 @@ __device__ void expand_level(const SegDesc &A, SamplerSmem<BLOCK> &s, NodeRec *r
                 ys[k] = it < G ? __ldg(&adj[s.f_off[li[k]] + it]) : 0u;
             }
             uint32_t sty[kItems], dg[kItems];
+            if (near) {
 #pragma unroll
-            for (int k = 0; k < kItems; k++) sty[k] = code[k] ? __ldcg(&rec[ys[k]].st) : 0u;
+                for (int k = 0; k < kItems; k++) {
+                    const uint32_t b = near_get<BLOCK>(ys[k]);
+                    sty[k] = b == 3u ? new_st : st_make(b, 0);
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < kItems; k++) sty[k] = code[k] ? __ldcg(&rec[ys[k]].st) : 0u;
+            }
 #pragma unroll
             for (int k = 0; k < kItems; k++) {
                 if (!code[k]) continue;
@@ -442,6 +548,11 @@ __device__ void expand_level(const SegDesc &A, SamplerSmem<BLOCK> &s, NodeRec *r
                 else if (sty[k] == new_st) code[k] = 4;
                 else if (st_side(sty[k]) != side) code[k] = 2;
                 else code[k] = 0;
+            }
+            if (mend > mend0) {
+                last_tile<BLOCK>(s, rec, queue, meet, new_st, near, ys, code, li, qend, mend,
+                                 hits_local, t0);
+                continue;
             }
             // the rows of the unvisited ones (needed by the hits that join)
 #pragma unroll
@@ -564,10 +675,14 @@ __device__ void expand_level(const SegDesc &A, SamplerSmem<BLOCK> &s, NodeRec *r
                 qend += an;
                 mend = min(mend + am, kMeetCap);
             }
+            // no later tile looks for the last one's joins
+            const bool last = c0 + (uint32_t)kChunk >= hi && t0 + (uint32_t)kTile >= G;
+            if (!last) marked = qend;
 #pragma unroll
             for (int k = 0; k < kItems; k++) {
                 if (code[k] == 1) {
                     const uint32_t y = ys[k];
+                    if (near) near_xor<BLOCK>(y, last ? side : 3u);
                     queue[oa[k] + rn[k]] = y;
                     // the joining hit: st, cnt = 1, sigma, first = last = key
                     const uint32_t it = t0 + (uint32_t)(k * BLOCK) + threadIdx.x;
@@ -603,6 +718,10 @@ __device__ void expand_level(const SegDesc &A, SamplerSmem<BLOCK> &s, NodeRec *r
         gbase += G;
         __syncthreads();
     }
+    if (near && mend == mend0)
+        for (uint32_t i = q0 + threadIdx.x; i < marked; i += BLOCK)
+            near_xor<BLOCK>(__ldcg(&queue[i]), 3u ^ side);
+    __syncwarp();
     // degree sum of the new level (u32, wrapping like the reference's counter)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -622,7 +741,7 @@ __device__ void expand_level(const SegDesc &A, SamplerSmem<BLOCK> &s, NodeRec *r
         }
         s.sum_new = sn;
         s.pred_hits += ph;
-        s.end_q = qend;
+        s.end_q = qend + (near ? 0u : s.light);
         s.nmeet = mend;
     }
     // the caller's thread 0 consumes sum_new and the ends before its next barrier
@@ -823,20 +942,20 @@ __device__ __forceinline__ int32_t post_level(const SamplerLaunch &L, SamplerSme
     const uint2 r0 = drows[x0];
     const uint32_t items = depth == 0 ? r0.y - r0.x : (side_u ? s.sum_u : s.sum_v);
     const uint32_t F = hi - lo;
-    // Default threshold: 32 tiles while the round still has samples to hand
-    // out, 16 tiles once every sample is taken (on R-MAT scale 20, over 60
-    // seeds: 16 and 24 tiles alike, 8 tiles 5 % longer, 4 tiles 7 %, 2 tiles
-    // 10 %; eight tiles while samples remain 5 % longer).  While samples remain, every
-    // CTA is busy with its own and helps only between samples, and a shared
-    // tile costs more than one expanded alone (the look-backs and the tile
-    // table), so only levels long enough to become the launch's tail are
-    // shared; once the round is drained, the CTAs without samples are idle
-    // and the last samples' levels are what the launch waits for.
+    // Default threshold: 128 items per thread of the CTA while the round still
+    // has samples to hand out, 64 once every sample is taken (on R-MAT scale
+    // 20, over 60 seeds: 64 and 96 alike, 32 5 % longer, 16 7 %, 8 10 %; 32
+    // while samples remain 5 % longer).  While samples remain, every CTA is
+    // busy with its own and helps only between samples, and a shared tile
+    // costs more than one expanded alone (the look-backs and the tile table),
+    // so only levels long enough to become the launch's tail are shared; once
+    // the round is drained, the CTAs without samples are idle and the last
+    // samples' levels are what the launch waits for.
     uint32_t thr = A.assist_items;
     if (thr == kAssistItemsAuto) {
-        if (items < 16u * (uint32_t)Shape<BLOCK>::kTile) return -1;
+        if (items < 64u * BLOCK) return -1;
         const bool draining = ld_acquire_u32(&L.hdr->work) >= list_total(L.hdr->todo);
-        thr = (draining ? 16u : 32u) * (uint32_t)Shape<BLOCK>::kTile;
+        thr = (draining ? 64u : 128u) * BLOCK;
     }
     if (items < thr || F > L.assist.node_cap ||
         (uint64_t)items / Shape<BLOCK>::kTile + F / Shape<BLOCK>::kChunk + 2u > L.assist.tile_cap)
@@ -1345,6 +1464,8 @@ __global__ void __launch_bounds__(BLOCK, Shape<BLOCK>::kMinBlocks) sampler_kerne
         s.t_key[i] = kNoNode;
         s.t_item[i] = 0xffffffffu;
     }
+    for (uint32_t i = threadIdx.x; i < L.near_cap / 64u; i += BLOCK)
+        reinterpret_cast<uint4 *>(near_states<BLOCK>())[i] = make_uint4(0, 0, 0, 0);
     uint32_t seg = 0xffffffffu;
     for (;;) {
         if (threadIdx.x == 0) {
@@ -1431,7 +1552,13 @@ __global__ void __launch_bounds__(BLOCK, Shape<BLOCK>::kMinBlocks) sampler_kerne
         const long long t_sample0 = clock64();
         // endpoints drawn and screened (screen_chunk)
         const uint32_t u = s.u, v = s.v;
+        const bool near = A.n <= L.near_cap;
         if (threadIdx.x == 0) {
+            s.light = 0;
+            if (near) {
+                near_xor<BLOCK>(u, kSideU);
+                near_xor<BLOCK>(v, kSideV);
+            }
             rec[u].st = st_make(kSideU, 0);
             rec[u].sigma = 1;
             rec[v].st = st_make(kSideV, 0);
@@ -1468,10 +1595,10 @@ __global__ void __launch_bounds__(BLOCK, Shape<BLOCK>::kMinBlocks) sampler_kerne
                                 ? post_level<BLOCK>(L, s, side_u, lo, hi, depth)
                                 : -1;
             __syncthreads();
-            if (s.a_entry < 0 ||
-                !expand_level_assisted<BLOCK>(L, A, s, rec, queue, meet, exp_side, lo, hi, depth,
-                                              (uint32_t)s.a_entry))
-                expand_level(A, s, rec, queue, meet, exp_side, lo, hi, depth);
+            const bool alone =
+                s.a_entry < 0 || !expand_level_assisted<BLOCK>(L, A, s, rec, queue, meet, exp_side,
+                                                               lo, hi, depth, (uint32_t)s.a_entry);
+            if (alone) expand_level(A, s, rec, queue, meet, exp_side, lo, hi, depth, near);
             if (threadIdx.x == 0) {
                 if (depth + 1 < (uint32_t)kMaxLevels) {
                     s.lvl_lo[side_u ? 0 : 1][depth + 1] = q0;
@@ -1491,6 +1618,12 @@ __global__ void __launch_bounds__(BLOCK, Shape<BLOCK>::kMinBlocks) sampler_kerne
             }
             __syncthreads();
             if (s.nmeet > 0 || s.sum_new == 0 || s.status != 0) break;
+            if (near && !alone) {  // the level's joins, made by several CTAs
+                for (uint32_t i = q0 + threadIdx.x; i < s.end_q; i += BLOCK)
+                    near_xor<BLOCK>(__ldcg(&queue[i]), exp_side);
+                __syncwarp();
+                __syncthreads();
+            }
         }
 
         // ---- meeting-edge weights and the number of paths (:159-170) ----------
@@ -1689,6 +1822,9 @@ __global__ void __launch_bounds__(BLOCK, Shape<BLOCK>::kMinBlocks) sampler_kerne
                 hits[a4[j]] = 0;
             }
         }
+        if (near)
+            for (uint32_t i = threadIdx.x; i < (A.n + 63u) / 64u; i += BLOCK)
+                reinterpret_cast<uint4 *>(near_states<BLOCK>())[i] = make_uint4(0, 0, 0, 0);
         const uint32_t eq = s.end_q;
         for (uint32_t i0 = threadIdx.x; i0 < eq; i0 += 4 * BLOCK) {
             uint32_t q4[4];
@@ -1706,7 +1842,7 @@ __global__ void __launch_bounds__(BLOCK, Shape<BLOCK>::kMinBlocks) sampler_kerne
             A.out_np[sl] = s.status == 0 ? np : 0;
             A.out_vis[sl] = s.vis;
             A.out_status[sl] = s.status;
-            A.out_ball[sl] = s.end_q;
+            A.out_ball[sl] = s.end_q + (near ? s.light : 0u);
             A.out_pred[sl] = s.pred_hits;
             const unsigned long long dc = (unsigned long long)(clock64() - t_sample0);
             atomicAdd(&L.hdr->cycles, dc);
@@ -1768,7 +1904,7 @@ cudaError_t sampler_init_slots(NodeRec *rec, uint32_t *hits, uint64_t total_node
 }
 
 namespace {
-constexpr uint32_t kAssistTileCap = 1u << 16;
+constexpr uint32_t kAssistTileCap = 1u << 17;
 uint64_t align256(uint64_t b) { return (b + 255u) & ~255ull; }
 }  // namespace
 
@@ -1809,14 +1945,14 @@ namespace {
 // device (the attribute is per device; setting it again is harmless).
 struct SizedKernel {
     const void *fn;
-    size_t smem;
+    size_t smem;  // without near states
 };
 
 template <int BLOCK>
 cudaError_t sized_kernel(SizedKernel *k) {
-    *k = {reinterpret_cast<const void *>(sampler_kernel<BLOCK>), sizeof(SamplerSmem<BLOCK>)};
+    *k = {reinterpret_cast<const void *>(sampler_kernel<BLOCK>), Near<BLOCK>::kOffset};
     return cudaFuncSetAttribute(sampler_kernel<BLOCK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)k->smem);
+                                (int)(k->smem + sampler_near_max(BLOCK) / 4));
 }
 
 cudaError_t sized_kernel(int block, SizedKernel *k) {
@@ -1830,20 +1966,30 @@ cudaError_t sized_kernel(int block, SizedKernel *k) {
 }
 }  // namespace
 
+uint32_t sampler_near_cap(uint64_t n, int block) {
+    if (n > sampler_near_max(block)) return 0;
+    uint32_t cap = 4096;
+    while (cap < n) cap *= 2;
+    return cap;
+}
+
 cudaError_t sampler_launch(const SamplerLaunch &L, uint32_t grid, cudaStream_t stream, int block) {
     if (grid == 0) return cudaSuccess;
+    if (L.near_cap > sampler_near_max(block) || L.near_cap % 64) return cudaErrorInvalidValue;
     SizedKernel k{};
     const cudaError_t e = sized_kernel(block, &k);
     if (e != cudaSuccess) return e;
     void *args[] = {const_cast<SamplerLaunch *>(&L)};
-    return cudaLaunchKernel(k.fn, dim3(grid), dim3((unsigned)block), args, k.smem, stream);
+    return cudaLaunchKernel(k.fn, dim3(grid), dim3((unsigned)block), args,
+                            k.smem + L.near_cap / 4, stream);
 }
 
 int sampler_max_ctas_per_sm(int block) {
     int n = 0;
     SizedKernel k{};
     if (sized_kernel(block, &k) != cudaSuccess) return 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k.fn, block, k.smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k.fn, block,
+                                                  k.smem + sampler_near_max(block) / 4);
     return n;
 }
 

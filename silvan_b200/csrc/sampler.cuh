@@ -12,9 +12,9 @@ namespace silvan {
 constexpr int kSamplerBlock = 512;   // default threads per slot
 constexpr int kSamplerBlocks[4] = {128, 256, 512, 1024};  // compiled CTA sizes
 constexpr uint32_t kMeetCap = 1u << 16;  // meeting edges per sample
-// SegDesc::assist_items value for the default threshold: levels of at least
-// 32 tiles of the launch's CTA size while the round has samples left, 16
-// tiles once it is drained
+// SegDesc::assist_items value for the default threshold: levels of at least 128
+// entries per thread of the launch's CTAs while the round has samples left, 64
+// once it is drained
 constexpr uint32_t kAssistItemsAuto = 0xffffffffu;
 
 // One job's share of a sampler launch: samples [first_sample, first_sample +
@@ -159,6 +159,9 @@ struct SamplerLaunch {
     // work indices left by the warp sampler, list_cap per class (nullptr: all)
     const uint32_t *list;
     uint32_t list_cap;
+    // the samples of graphs of at most this many nodes keep the nodes' states
+    // in shared memory (sampler_near_cap(); 0: none)
+    uint32_t near_cap;
 };
 
 // Neutral records for `slots` slots of n nodes.
@@ -177,6 +180,13 @@ cudaError_t sampler_round_begin(const SamplerLaunch &L, uint32_t max_segs, cudaS
 // kSamplerBlocks; persistent, work-stealing).
 cudaError_t sampler_launch(const SamplerLaunch &L, uint32_t grid, cudaStream_t stream,
                            int block = kSamplerBlock);
+
+// Nodes whose states fit beside a `block`-thread sampler CTA, all CTAs that are
+// resident without them staying so: two bits a node, 64 KB an SM.
+constexpr uint32_t sampler_near_max(int block) { return 256u * (uint32_t)block; }
+// SamplerLaunch::near_cap for graphs of up to n nodes: the next power of two
+// (4,096 or more), 0 beyond sampler_near_max().
+uint32_t sampler_near_cap(uint64_t n, int block);
 
 // Resident CTAs per SM of the `block`-thread sampler (0 for other sizes).
 int sampler_max_ctas_per_sm(int block = kSamplerBlock);
