@@ -439,7 +439,7 @@ DeviceGraph::~DeviceGraph() {
 // SlotPool
 // ---------------------------------------------------------------------------
 uint64_t SlotPool::bytes_per_slot(uint64_t n) {
-    return n * (sizeof(NodeRec) + 12) + (uint64_t)kMeetCap * 16;
+    return n * (sizeof(NodeRec) + 12) + (uint64_t)kMeetCap * 16 + 4 * state_words(n);
 }
 
 int SlotPool::alloc(uint32_t s, uint64_t nn, cudaStream_t st) {
@@ -453,9 +453,17 @@ int SlotPool::alloc(uint32_t s, uint64_t nn, cudaStream_t st) {
     RK(dmalloc(&touched, tot));
     RK(dmalloc(&meet, (uint64_t)s * kMeetCap));
     RK(dmalloc(&meet_pre, (uint64_t)s * kMeetCap));
-    CK(sampler_init_slots(rec, hits, tot, st));
+    RK(dmalloc(&states, s * state_words(nn)));
+    CK(init(st));
     CK(cudaStreamSynchronize(st));
     return SILVAN_OK;
+}
+
+cudaError_t SlotPool::init(cudaStream_t st) {
+    cudaError_t e = sampler_init_slots(rec, hits, (uint64_t)slots * n, st);
+    if (e == cudaSuccess)
+        e = cudaMemsetAsync(states, 0, 4 * (uint64_t)slots * state_words(n), st);
+    return e;
 }
 
 void SlotPool::free_all() {
@@ -465,6 +473,7 @@ void SlotPool::free_all() {
     dfree(touched);
     dfree(meet);
     dfree(meet_pre);
+    dfree(states);
     slots = 0;
 }
 
@@ -615,15 +624,18 @@ void Engine::drop_execs() {
 // sampler) captured once per (CTA size, grid, warp sampler, near states) and replayed with
 // new segments.
 int Engine::sampler_exec(int block, uint32_t grid, bool warp, uint32_t near_cap,
-                         cudaGraphExec_t *out) {
+                         bool in_slot, cudaGraphExec_t *out) {
     for (const Exec &x : execs_)
-        if (x.block == block && x.grid == grid && x.warp == warp && x.near_cap == near_cap) {
+        if (x.block == block && x.grid == grid && x.warp == warp && x.near_cap == near_cap &&
+            x.in_slot == in_slot) {
             *out = x.exec;
             return SILVAN_OK;
         }
     SamplerLaunch L{};
-    L.slots = SlotArrays{slots_.rec,  slots_.queue,    slots_.hits, slots_.touched,
-                         slots_.meet, slots_.meet_pre, slots_.n};
+    L.slots = SlotArrays{slots_.rec,     slots_.queue,     slots_.hits,
+                         slots_.touched, slots_.meet,      slots_.meet_pre,
+                         slots_.n,       in_slot ? slots_.states : nullptr,
+                         SlotPool::state_words(slots_.n)};
     L.hdr = d_hdr_;
     L.segs = d_segs_;
     L.assist = board_;
@@ -653,7 +665,7 @@ int Engine::sampler_exec(int block, uint32_t grid, bool warp, uint32_t near_cap,
     cudaGraphDestroy(g);
     CK(e4);
     if (execs_.size() >= 32) drop_execs();
-    execs_.push_back(Exec{block, grid, warp, near_cap, x});
+    execs_.push_back(Exec{block, grid, warp, near_cap, in_slot, x});
     *out = x;
     return SILVAN_OK;
 }
@@ -761,6 +773,10 @@ uint64_t DeviceGraph::tune_class() const {
     return (directed ? 1ull : 0ull) | lg(n) << 1 | lg(n ? m / n : 0) << 8;
 }
 
+namespace {
+constexpr uint32_t kWideDiameter = 64;
+}
+
 int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> &reqs,
                   std::vector<uint64_t> &records) {
     std::vector<uint32_t> idx;
@@ -854,11 +870,23 @@ int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> 
         drop_execs();
     }
     cudaGraphExec_t exec = nullptr;
-    uint64_t n_near = 0;  // the largest graph whose nodes' states fit in shared memory
-    for (uint32_t i : idx)
-        if (jobs[i]->graph()->n <= sampler_near_max(block))
-            n_near = std::max<uint64_t>(n_near, jobs[i]->graph()->n);
-    RK(sampler_exec(block, grid, warp, n_near ? sampler_near_cap(n_near, block) : 0u, &exec));
+    // The nodes' states: in shared memory where every graph of the round fits
+    // (R-MAT 16: 7.1 ms of sampling with the records, 3.4 so; lattices of up to
+    // 180 x 180 the same either way), else in the slots, unless all the graphs
+    // are long ones: their levels are narrow and their balls compact, so that the
+    // records' sectors are near one another and the bits cost an extra pass per
+    // level (diameter bounds of 8 to 16: R-MAT 20 2.0 ms -> 1.35, R-MAT 18 3.0 ->
+    // 1.95, 200,000 nodes of Barabasi-Albert 2.3 -> 2.0; bounds of 176 and 182,
+    // lattices: 5.15 -> 5.6 and 3.9 -> 4.1).
+    uint64_t n_round = 0;
+    bool wide = false;
+    for (uint32_t i : idx) {
+        const DeviceGraph &G = *jobs[i]->graph();
+        n_round = std::max<uint64_t>(n_round, G.n);
+        wide = wide || G.diameter < kWideDiameter;
+    }
+    const uint32_t near_cap = sampler_near_cap(n_round, block);
+    RK(sampler_exec(block, grid, warp, near_cap, near_cap == 0 && wide, &exec));
     for (;;) {
         CK(cudaMemcpyAsync(d_segs_, h_segs_, sizeof(SegDesc) * idx.size(),
                            cudaMemcpyHostToDevice, stream_));
@@ -883,8 +911,7 @@ int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> 
             // to them any more) before any later round uses it.  The samples
             // concerned carry SILVAN_E_TIMEOUT into their jobs' commits; if
             // samples were left undrawn, the whole round fails.
-            CK(sampler_init_slots(slots_.rec, slots_.hits, (uint64_t)slots_.slots * slots_.n,
-                                  stream_));
+            CK(slots_.init(stream_));
             CK(cudaStreamSynchronize(stream_));
             slot_resets_++;
             if (h_hdr_->finished < list_total(h_hdr_->todo)) {

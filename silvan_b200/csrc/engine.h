@@ -97,8 +97,11 @@ struct SlotPool {
     uint32_t *queue = nullptr, *hits = nullptr, *touched = nullptr;
     uint2 *meet = nullptr;
     uint64_t *meet_pre = nullptr;
+    uint32_t *states = nullptr;
     int alloc(uint32_t slots, uint64_t n, cudaStream_t s);
+    cudaError_t init(cudaStream_t s);  // neutral slots, on the stream
     void free_all();
+    static uint64_t state_words(uint64_t n) { return (n + 15) / 16; }
     static uint64_t bytes_per_slot(uint64_t n);
     ~SlotPool() { free_all(); }
 };
@@ -210,12 +213,13 @@ class Engine {
         uint32_t grid;
         bool warp;  // the warp sampler first
         uint32_t near_cap;
+        bool in_slot;
         cudaGraphExec_t exec;
     };
     int ensure_segs(uint32_t nsegs);
     int choose_block(const std::vector<Job *> &jobs, const std::vector<JobRequest> &reqs,
                      const std::vector<uint32_t> &idx, uint32_t total) const;
-    int sampler_exec(int block, uint32_t grid, bool warp, uint32_t near_cap,
+    int sampler_exec(int block, uint32_t grid, bool warp, uint32_t near_cap, bool in_slot,
                      cudaGraphExec_t *out);
     void drop_execs();
     SlotPool slots_;

@@ -115,11 +115,18 @@ struct SamplerSmem {
     uint32_t pend_n, pend_i, scr_w0, scr_v;
 };
 
-// States of the nodes, two bits each, behind SamplerSmem, for graphs of at most
-// SamplerLaunch::near_cap nodes: 0 not visited, kSideU or kSideV, 3 joined in
-// the level that is being expanded.  A copy of what the slot's records say: a
-// probe is a shared-memory read instead of a 32-byte sector of its own, most of
-// them missed in L2 (592 slots of 65,536 records: 1.2 GB).
+// Where a search looks up whether a node was visited.
+//   kInRecord  the node's record: a 32-byte sector of its own, most of them missed
+//              in L2 (592 slots of 65,536 records: 1.2 GB)
+//   kInShared  two bits a node behind SamplerSmem, for graphs of up to
+//              sampler_near_max() nodes
+//   kInSlot    two bits a node in the slot: 128 nodes a sector, and the words of
+//              all slots together fit in L2 where the records do not (296 slots
+//              of a million nodes: 78 MB)
+// The bits are 0 for not visited, kSideU or kSideV, 3 for joined in the level that
+// is being expanded: a copy of what the records say.
+constexpr int kInRecord = 0, kInShared = 1, kInSlot = 2;
+
 template <int BLOCK>
 struct Near {
     static constexpr size_t kOffset = (sizeof(SamplerSmem<BLOCK>) + 15) & ~(size_t)15;
@@ -129,14 +136,25 @@ __device__ __forceinline__ uint32_t *near_states() {
     extern __shared__ __align__(16) unsigned char sampler_smem[];
     return reinterpret_cast<uint32_t *>(sampler_smem + Near<BLOCK>::kOffset);
 }
-template <int BLOCK>
-__device__ __forceinline__ uint32_t near_get(uint32_t y) {
-    return near_states<BLOCK>()[y >> 4] >> (2u * (y & 15u)) & 3u;
+template <int BLOCK, int MODE>
+__device__ __forceinline__ uint32_t state_get(const uint32_t *slot, uint32_t y) {
+    const uint32_t w = MODE == kInSlot ? __ldcg(&slot[y >> 4]) : near_states<BLOCK>()[y >> 4];
+    return w >> (2u * (y & 15u)) & 3u;
 }
 // From 0 to c, or (c = a ^ b) from a to b.
-template <int BLOCK>
-__device__ __forceinline__ void near_xor(uint32_t y, uint32_t c) {
-    atomicXor(&near_states<BLOCK>()[y >> 4], c << (2u * (y & 15u)));
+template <int BLOCK, int MODE>
+__device__ __forceinline__ void state_xor(uint32_t *slot, uint32_t y, uint32_t c) {
+    c <<= 2u * (y & 15u);
+    if (MODE == kInSlot) atomicXor(&slot[y >> 4], c);
+    else atomicXor(&near_states<BLOCK>()[y >> 4], c);
+}
+// Marks y joined; whether it was not visited before.
+template <int BLOCK, int MODE>
+__device__ __forceinline__ bool state_join(uint32_t *slot, uint32_t y) {
+    const uint32_t sh = 2u * (y & 15u);
+    const uint32_t old = MODE == kInSlot ? atomicOr(&slot[y >> 4], 3u << sh)
+                                         : atomicOr(&near_states<BLOCK>()[y >> 4], 3u << sh);
+    return (old >> sh & 3u) == 0u;
 }
 
 // Exclusive block scan of one value per thread; returns the block total.
@@ -369,11 +387,11 @@ __device__ __forceinline__ void record_hit(NodeRec *r, uint32_t g, uint32_t x,
 // the hits and to append the meeting edges in item order.  On power-law graphs
 // the last level holds most of a search's edges: 86,700 samples of R-MAT 16 took
 // 7.0 ms, 6.6 with the states in shared memory (and two items a lane), and take
-// 3.5 with these tiles; without the states 7.1, as every mark is then an atomic
-// on a record that comes from memory.
-template <int BLOCK>
+// 3.4 with these tiles; with kInRecord 7.1, as every mark is then an atomic on a
+// record that comes from memory.
+template <int BLOCK, int MODE>
 __device__ __forceinline__ void last_tile(SamplerSmem<BLOCK> &s, NodeRec *rec, uint32_t *queue,
-                                          uint2 *meet, uint32_t new_st, bool near,
+                                          uint2 *meet, uint32_t new_st, uint32_t *states,
                                           const uint32_t (&ys)[kItems], uint32_t (&code)[kItems],
                                           const uint32_t (&li)[kItems], uint32_t &qend,
                                           uint32_t &mend, uint32_t &hits, uint32_t t0) {
@@ -388,12 +406,8 @@ __device__ __forceinline__ void last_tile(SamplerSmem<BLOCK> &s, NodeRec *rec, u
         bool join = false;
         if (code[k] == 1 || code[k] == 4) hits++;
         if (code[k] == 1) {
-            if (near) {
-                const uint32_t sh = 2u * (ys[k] & 15u);
-                join = (atomicOr(&near_states<BLOCK>()[ys[k] >> 4], 3u << sh) >> sh & 3u) == 0u;
-            } else {
-                join = atomicCAS(&rec[ys[k]].st, 0u, new_st) == 0u;
-            }
+            if (MODE == kInRecord) join = atomicCAS(&rec[ys[k]].st, 0u, new_st) == 0u;
+            else join = state_join<BLOCK, MODE>(states, ys[k]);
         }
         const uint32_t bn = __ballot_sync(0xffffffffu, join);
         const uint32_t bm = __ballot_sync(0xffffffffu, code[k] == 2);
@@ -401,8 +415,8 @@ __device__ __forceinline__ void last_tile(SamplerSmem<BLOCK> &s, NodeRec *rec, u
             uint32_t at = 0;
             if (lane == 0) at = atomicAdd(&s.light, (uint32_t)__popc(bn));
             at = __shfl_sync(0xffffffffu, at, 0);
-            // the records of these are put back from the queue, in any order
-            if (!near && join) queue[qend + at + __popc(bn & lanemask_lt())] = ys[k];
+            // records or states in memory are put back from the queue, in any order
+            if (MODE != kInShared && join) queue[qend + at + __popc(bn & lanemask_lt())] = ys[k];
         }
         rm[k] = __popc(bm & lanemask_lt());
         any = any || bm != 0u;
@@ -435,10 +449,10 @@ __device__ __forceinline__ void last_tile(SamplerSmem<BLOCK> &s, NodeRec *rec, u
 // state through L2) and only then stores or issues atomics: a store between
 // two loads would serialise them, because the compiler cannot prove that they
 // do not alias.
-template <int BLOCK>
+template <int BLOCK, int MODE>
 __device__ void expand_level(const SegDesc &A, SamplerSmem<BLOCK> &s, NodeRec *rec,
                              uint32_t *queue, uint2 *meet, uint32_t side, uint32_t lo,
-                             uint32_t hi, uint32_t depth, bool near) {
+                             uint32_t hi, uint32_t depth, uint32_t *states) {
     constexpr int kWarps = Shape<BLOCK>::kWarps;
     constexpr int kTile = Shape<BLOCK>::kTile;
     constexpr int kChunk = Shape<BLOCK>::kChunk;
@@ -530,10 +544,10 @@ __device__ void expand_level(const SegDesc &A, SamplerSmem<BLOCK> &s, NodeRec *r
                 ys[k] = it < G ? __ldg(&adj[s.f_off[li[k]] + it]) : 0u;
             }
             uint32_t sty[kItems], dg[kItems];
-            if (near) {
+            if (MODE != kInRecord) {
 #pragma unroll
                 for (int k = 0; k < kItems; k++) {
-                    const uint32_t b = near_get<BLOCK>(ys[k]);
+                    const uint32_t b = state_get<BLOCK, MODE>(states, ys[k]);
                     sty[k] = b == 3u ? new_st : st_make(b, 0);
                 }
             } else {
@@ -550,7 +564,7 @@ __device__ void expand_level(const SegDesc &A, SamplerSmem<BLOCK> &s, NodeRec *r
                 else code[k] = 0;
             }
             if (mend > mend0) {
-                last_tile<BLOCK>(s, rec, queue, meet, new_st, near, ys, code, li, qend, mend,
+                last_tile<BLOCK, MODE>(s, rec, queue, meet, new_st, states, ys, code, li, qend, mend,
                                  hits_local, t0);
                 continue;
             }
@@ -682,7 +696,8 @@ __device__ void expand_level(const SegDesc &A, SamplerSmem<BLOCK> &s, NodeRec *r
             for (int k = 0; k < kItems; k++) {
                 if (code[k] == 1) {
                     const uint32_t y = ys[k];
-                    if (near) near_xor<BLOCK>(y, last ? side : 3u);
+                    if (MODE != kInRecord)
+                        state_xor<BLOCK, MODE>(states, y, last ? side : 3u);
                     queue[oa[k] + rn[k]] = y;
                     // the joining hit: st, cnt = 1, sigma, first = last = key
                     const uint32_t it = t0 + (uint32_t)(k * BLOCK) + threadIdx.x;
@@ -718,9 +733,9 @@ __device__ void expand_level(const SegDesc &A, SamplerSmem<BLOCK> &s, NodeRec *r
         gbase += G;
         __syncthreads();
     }
-    if (near && mend == mend0)
+    if (MODE != kInRecord && mend == mend0)
         for (uint32_t i = q0 + threadIdx.x; i < marked; i += BLOCK)
-            near_xor<BLOCK>(__ldcg(&queue[i]), 3u ^ side);
+            state_xor<BLOCK, MODE>(states, __ldcg(&queue[i]), 3u ^ side);
     __syncwarp();
     // degree sum of the new level (u32, wrapping like the reference's counter)
 #pragma unroll
@@ -741,7 +756,7 @@ __device__ void expand_level(const SegDesc &A, SamplerSmem<BLOCK> &s, NodeRec *r
         }
         s.sum_new = sn;
         s.pred_hits += ph;
-        s.end_q = qend + (near ? 0u : s.light);
+        s.end_q = qend + (MODE == kInRecord ? s.light : 0u);
         s.nmeet = mend;
     }
     // the caller's thread 0 consumes sum_new and the ends before its next barrier
@@ -1430,7 +1445,7 @@ __device__ __noinline__ void screen_chunk(const SamplerLaunch &L, SamplerSmem<BL
     __syncthreads();
 }
 
-template <int BLOCK>
+template <int BLOCK, int MODE>
 __global__ void __launch_bounds__(BLOCK, Shape<BLOCK>::kMinBlocks) sampler_kernel(SamplerLaunch L) {
     constexpr int kWarps = Shape<BLOCK>::kWarps;
     extern __shared__ __align__(16) unsigned char sampler_smem[];
@@ -1443,6 +1458,7 @@ __global__ void __launch_bounds__(BLOCK, Shape<BLOCK>::kMinBlocks) sampler_kerne
     uint32_t *touched = L.slots.touched + base;
     uint2 *meet = L.slots.meet + (uint64_t)slot * kMeetCap;
     uint64_t *mpre = L.slots.meet_pre + (uint64_t)slot * kMeetCap;
+    uint32_t *states = MODE == kInSlot ? L.slots.states + slot * L.slots.state_words : nullptr;
     const uint32_t total = list_total(L.hdr->todo);
     const uint32_t nsegs = L.hdr->nsegs;
     const SegDesc &A = s.seg;
@@ -1464,7 +1480,7 @@ __global__ void __launch_bounds__(BLOCK, Shape<BLOCK>::kMinBlocks) sampler_kerne
         s.t_key[i] = kNoNode;
         s.t_item[i] = 0xffffffffu;
     }
-    for (uint32_t i = threadIdx.x; i < L.near_cap / 64u; i += BLOCK)
+    for (uint32_t i = threadIdx.x; MODE == kInShared && i < L.near_cap / 64u; i += BLOCK)
         reinterpret_cast<uint4 *>(near_states<BLOCK>())[i] = make_uint4(0, 0, 0, 0);
     uint32_t seg = 0xffffffffu;
     for (;;) {
@@ -1552,12 +1568,11 @@ __global__ void __launch_bounds__(BLOCK, Shape<BLOCK>::kMinBlocks) sampler_kerne
         const long long t_sample0 = clock64();
         // endpoints drawn and screened (screen_chunk)
         const uint32_t u = s.u, v = s.v;
-        const bool near = A.n <= L.near_cap;
         if (threadIdx.x == 0) {
             s.light = 0;
-            if (near) {
-                near_xor<BLOCK>(u, kSideU);
-                near_xor<BLOCK>(v, kSideV);
+            if (MODE != kInRecord) {
+                state_xor<BLOCK, MODE>(states, u, kSideU);
+                state_xor<BLOCK, MODE>(states, v, kSideV);
             }
             rec[u].st = st_make(kSideU, 0);
             rec[u].sigma = 1;
@@ -1598,7 +1613,8 @@ __global__ void __launch_bounds__(BLOCK, Shape<BLOCK>::kMinBlocks) sampler_kerne
             const bool alone =
                 s.a_entry < 0 || !expand_level_assisted<BLOCK>(L, A, s, rec, queue, meet, exp_side,
                                                                lo, hi, depth, (uint32_t)s.a_entry);
-            if (alone) expand_level(A, s, rec, queue, meet, exp_side, lo, hi, depth, near);
+            if (alone)
+                expand_level<BLOCK, MODE>(A, s, rec, queue, meet, exp_side, lo, hi, depth, states);
             if (threadIdx.x == 0) {
                 if (depth + 1 < (uint32_t)kMaxLevels) {
                     s.lvl_lo[side_u ? 0 : 1][depth + 1] = q0;
@@ -1618,9 +1634,9 @@ __global__ void __launch_bounds__(BLOCK, Shape<BLOCK>::kMinBlocks) sampler_kerne
             }
             __syncthreads();
             if (s.nmeet > 0 || s.sum_new == 0 || s.status != 0) break;
-            if (near && !alone) {  // the level's joins, made by several CTAs
+            if (MODE != kInRecord && !alone) {  // the level's joins, made by several CTAs
                 for (uint32_t i = q0 + threadIdx.x; i < s.end_q; i += BLOCK)
-                    near_xor<BLOCK>(__ldcg(&queue[i]), exp_side);
+                    state_xor<BLOCK, MODE>(states, __ldcg(&queue[i]), exp_side);
                 __syncwarp();
                 __syncthreads();
             }
@@ -1822,7 +1838,7 @@ __global__ void __launch_bounds__(BLOCK, Shape<BLOCK>::kMinBlocks) sampler_kerne
                 hits[a4[j]] = 0;
             }
         }
-        if (near)
+        if (MODE == kInShared)
             for (uint32_t i = threadIdx.x; i < (A.n + 63u) / 64u; i += BLOCK)
                 reinterpret_cast<uint4 *>(near_states<BLOCK>())[i] = make_uint4(0, 0, 0, 0);
         const uint32_t eq = s.end_q;
@@ -1835,14 +1851,20 @@ __global__ void __launch_bounds__(BLOCK, Shape<BLOCK>::kMinBlocks) sampler_kerne
             }
 #pragma unroll
             for (int j = 0; j < 4; j++)
-                if (q4[j] != 0xffffffffu) rec_reset(&rec[q4[j]]);
+                if (q4[j] != 0xffffffffu) {
+                    rec_reset(&rec[q4[j]]);
+                    if (MODE == kInSlot) states[q4[j] >> 4] = 0u;
+                }
         }
+        if (MODE == kInSlot)  // last_tile's nodes have no record
+            for (uint32_t i = threadIdx.x; i < s.light; i += BLOCK)
+                states[__ldcg(&queue[eq + i]) >> 4] = 0u;
         if (threadIdx.x == 0) {
             A.out_pl[sl] = s.status == 0 ? pl : 0;
             A.out_np[sl] = s.status == 0 ? np : 0;
             A.out_vis[sl] = s.vis;
             A.out_status[sl] = s.status;
-            A.out_ball[sl] = s.end_q + (near ? s.light : 0u);
+            A.out_ball[sl] = s.end_q + (MODE == kInRecord ? 0u : s.light);
             A.out_pred[sl] = s.pred_hits;
             const unsigned long long dc = (unsigned long long)(clock64() - t_sample0);
             atomicAdd(&L.hdr->cycles, dc);
@@ -1941,28 +1963,37 @@ cudaError_t sampler_round_begin(const SamplerLaunch &L, uint32_t max_segs, cudaS
 }
 
 namespace {
-// The kernel of a CTA size, its shared memory opted into on the current
-// device (the attribute is per device; setting it again is harmless).
+// The kernel of a CTA size and a place of the states, its shared memory opted
+// into on the current device (the attribute is per device; setting it again is
+// harmless).
 struct SizedKernel {
     const void *fn;
-    size_t smem;  // without near states
+    size_t smem;  // without states
 };
 
-template <int BLOCK>
+template <int BLOCK, int MODE>
 cudaError_t sized_kernel(SizedKernel *k) {
-    *k = {reinterpret_cast<const void *>(sampler_kernel<BLOCK>), Near<BLOCK>::kOffset};
-    return cudaFuncSetAttribute(sampler_kernel<BLOCK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(k->smem + sampler_near_max(BLOCK) / 4));
+    *k = {reinterpret_cast<const void *>(sampler_kernel<BLOCK, MODE>), Near<BLOCK>::kOffset};
+    const size_t most = k->smem + (MODE == kInShared ? sampler_near_max(BLOCK) / 4 : 0);
+    return cudaFuncSetAttribute(sampler_kernel<BLOCK, MODE>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
 }
 
+template <int MODE>
 cudaError_t sized_kernel(int block, SizedKernel *k) {
     switch (block) {
-    case 128: return sized_kernel<128>(k);
-    case 256: return sized_kernel<256>(k);
-    case 512: return sized_kernel<512>(k);
-    case 1024: return sized_kernel<1024>(k);
+    case 128: return sized_kernel<128, MODE>(k);
+    case 256: return sized_kernel<256, MODE>(k);
+    case 512: return sized_kernel<512, MODE>(k);
+    case 1024: return sized_kernel<1024, MODE>(k);
     default: return cudaErrorInvalidValue;
     }
+}
+
+cudaError_t sized_kernel(int block, int mode, SizedKernel *k) {
+    return mode == kInShared ? sized_kernel<kInShared>(block, k)
+           : mode == kInSlot ? sized_kernel<kInSlot>(block, k)
+                             : sized_kernel<kInRecord>(block, k);
 }
 }  // namespace
 
@@ -1977,7 +2008,8 @@ cudaError_t sampler_launch(const SamplerLaunch &L, uint32_t grid, cudaStream_t s
     if (grid == 0) return cudaSuccess;
     if (L.near_cap > sampler_near_max(block) || L.near_cap % 64) return cudaErrorInvalidValue;
     SizedKernel k{};
-    const cudaError_t e = sized_kernel(block, &k);
+    const int mode = L.near_cap ? kInShared : L.slots.states ? kInSlot : kInRecord;
+    const cudaError_t e = sized_kernel(block, mode, &k);
     if (e != cudaSuccess) return e;
     void *args[] = {const_cast<SamplerLaunch *>(&L)};
     return cudaLaunchKernel(k.fn, dim3(grid), dim3((unsigned)block), args,
@@ -1985,12 +2017,16 @@ cudaError_t sampler_launch(const SamplerLaunch &L, uint32_t grid, cudaStream_t s
 }
 
 int sampler_max_ctas_per_sm(int block) {
-    int n = 0;
-    SizedKernel k{};
-    if (sized_kernel(block, &k) != cudaSuccess) return 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k.fn, block,
-                                                  k.smem + sampler_near_max(block) / 4);
-    return n;
+    int least = 1 << 20;
+    for (int mode : {kInRecord, kInShared, kInSlot}) {
+        int n = 0;
+        SizedKernel k{};
+        if (sized_kernel(block, mode, &k) != cudaSuccess) return 0;
+        if (mode == kInShared) k.smem += sampler_near_max(block) / 4;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k.fn, block, k.smem);
+        least = n < least ? n : least;
+    }
+    return least;
 }
 
 }  // namespace silvan

@@ -149,6 +149,10 @@ struct SlotArrays {
     uint2 *meet;        // slot s owns [s*kMeetCap, (s+1)*kMeetCap)
     uint64_t *meet_pre;
     uint64_t stride;    // nodes per slot (largest graph served)
+    // slot s owns [s*state_words, (s+1)*state_words): two bits a node, all zero
+    // between samples (nullptr: the records tell)
+    uint32_t *states;
+    uint64_t state_words;
 };
 
 struct SamplerLaunch {
@@ -159,8 +163,8 @@ struct SamplerLaunch {
     // work indices left by the warp sampler, list_cap per class (nullptr: all)
     const uint32_t *list;
     uint32_t list_cap;
-    // the samples of graphs of at most this many nodes keep the nodes' states
-    // in shared memory (sampler_near_cap(); 0: none)
+    // at least every graph's nodes: the states of the nodes are kept in shared
+    // memory (sampler_near_cap(); 0: in slots.states)
     uint32_t near_cap;
 };
 
