@@ -207,7 +207,7 @@ class Engine {
     struct WarpStats {
         uint64_t drawn = 0, left = 0;
     };
-    bool try_warps(const DeviceGraph *G) const;
+    bool try_warps(const DeviceGraph *G, uint32_t total) const;
     struct Exec {
         int block;
         uint32_t grid;
