@@ -676,7 +676,7 @@ int Engine::sampler_exec(int block, uint32_t grid, bool warp, uint32_t near_cap,
 // round, or the CTA time of all its samples spread over the resident CTAs,
 // whichever is longer.
 int Engine::choose_block(const std::vector<Job *> &jobs, const std::vector<JobRequest> &reqs,
-                         const std::vector<uint32_t> &idx, uint32_t total) const {
+                         const std::vector<uint32_t> &idx, uint32_t total, bool warp) const {
     const silvan_params_t &p0 = jobs[idx[0]]->params();
     if (p0.block) return (int)p0.block;
     if (p0.form == SILVAN_FORM_PLAIN) return kSamplerBlock;
@@ -685,7 +685,7 @@ int Engine::choose_block(const std::vector<Job *> &jobs, const std::vector<JobRe
         const int b = order[oi];
         if (!max_grid_[b]) continue;
         for (uint32_t i : idx) {
-            auto it = stats_.find(jobs[i]->graph()->tune_class());
+            auto it = stats_.find(stats_key(jobs[i]->graph(), warp));
             if (it == stats_.end() || it->second[b].rounds == 0) return kSamplerBlocks[b];
         }
     }
@@ -695,7 +695,7 @@ int Engine::choose_block(const std::vector<Job *> &jobs, const std::vector<JobRe
         if (!max_grid_[b]) continue;
         double tail = 0, work = 0;
         for (uint32_t i : idx) {
-            const BlockStats &st = stats_.at(jobs[i]->graph()->tune_class())[b];
+            const BlockStats &st = stats_.at(stats_key(jobs[i]->graph(), warp))[b];
             tail = std::max(tail, st.tail_ms);
             work += reqs[i].count * st.cta_ms;
         }
@@ -730,7 +730,8 @@ void Engine::fair_share(const std::vector<Job *> &jobs, std::vector<JobRequest> 
     uint32_t grid = 0;
     for (int b = 0; b < kNB; b++) grid = std::max(grid, max_grid_[b]);
     for (size_t i = 0; i < n; i++) {
-        auto it = stats_.find(jobs[i]->graph()->tune_class());
+        auto it = stats_.find(stats_key(jobs[i]->graph(), true));
+        if (it == stats_.end()) it = stats_.find(stats_key(jobs[i]->graph(), false));
         if (it == stats_.end()) return;
         double best = 0;
         for (int b = 0; b < kNB; b++) {
@@ -852,15 +853,6 @@ int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> 
     h_hdr_->cycles = 0;
     h_hdr_->max_cycles = 0;
     h_hdr_->wait_polls = polls;
-    const int block = choose_block(jobs, reqs, idx, total);
-    int bi = -1;
-    for (int b = 0; b < kNB; b++)
-        if (kSamplerBlocks[b] == block && max_grid_[b]) bi = b;
-    if (bi < 0) {
-        set_error("sampler CTA size must be 128, 256, 512 or 1024 threads");
-        return SILVAN_E_BADARG;
-    }
-    const uint32_t grid = std::min<uint32_t>(max_grid_[bi], total);
     // Samples are first tried one warp each.  Not in the plain form (11 samples
     // a launch), and not when a job sets its own help-board threshold, which
     // asks for levels of the CTA sampler.
@@ -872,6 +864,15 @@ int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> 
             if (ai != 0u && ai != 0xffffffffu) warp = false;
         }
     }
+    const int block = choose_block(jobs, reqs, idx, total, warp);
+    int bi = -1;
+    for (int b = 0; b < kNB; b++)
+        if (kSamplerBlocks[b] == block && max_grid_[b]) bi = b;
+    if (bi < 0) {
+        set_error("sampler CTA size must be 128, 256, 512 or 1024 threads");
+        return SILVAN_E_BADARG;
+    }
+    const uint32_t grid = std::min<uint32_t>(max_grid_[bi], total);
     if (warp && total > warps_.list_cap) {
         RK(warps_.ensure_list(total));
         drop_execs();
@@ -953,7 +954,7 @@ int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> 
                 // the slowest sample of a launch grows with the launch's size
                 // and is rare: the estimate follows a longer tail at once and
                 // a shorter one slowly
-                BlockStats &st = stats_[jobs[i]->graph()->tune_class()][bi];
+                BlockStats &st = stats_[stats_key(jobs[i]->graph(), warp)][bi];
                 st.cta_ms = st.rounds ? 0.5 * (st.cta_ms + cta_ms) : cta_ms;
                 st.tail_ms = (!st.rounds || tail_ms > st.tail_ms) ? tail_ms
                                                                   : 0.75 * st.tail_ms + 0.25 * tail_ms;

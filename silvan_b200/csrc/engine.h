@@ -218,7 +218,11 @@ class Engine {
     };
     int ensure_segs(uint32_t nsegs);
     int choose_block(const std::vector<Job *> &jobs, const std::vector<JobRequest> &reqs,
-                     const std::vector<uint32_t> &idx, uint32_t total) const;
+                     const std::vector<uint32_t> &idx, uint32_t total, bool warp) const;
+    // a launch that warps draw first leaves the CTAs other samples: measured apart
+    static uint64_t stats_key(const DeviceGraph *G, bool warp) {
+        return G->tune_class() << 1 | (warp ? 1u : 0u);
+    }
     int sampler_exec(int block, uint32_t grid, bool warp, uint32_t near_cap, bool in_slot,
                      cudaGraphExec_t *out);
     void drop_execs();
@@ -233,7 +237,7 @@ class Engine {
     uint32_t max_segs_ = 0;
     std::vector<Exec> execs_;          // captured round_begin + sampler per (block, grid)
     uint32_t max_grid_[kNB] = {};      // resident CTAs per CTA size (0 = unusable)
-    std::unordered_map<uint64_t, std::array<BlockStats, kNB>> stats_;  // by tune_class()
+    std::unordered_map<uint64_t, std::array<BlockStats, kNB>> stats_;  // by stats_key()
     std::array<uint64_t, kNB> block_samples_{};
     uint32_t sampler_launches_ = 0;
     uint32_t assisted_levels_ = 0;  // BFS levels expanded with the help board
