@@ -217,6 +217,12 @@ int silvan_read_topk(silvan_job_t j, uint32_t *nodes, double *values, uint32_t c
 int silvan_read_counters(silvan_job_t j, double *approx, double *wimpy, int64_t *mcrade,
                          int32_t *partition_index);
 
+/* Polls after which a wait between the CTAs that group a draw's records by node
+ * gives up, from the next draw on: the job then fails with SILVAN_E_TIMEOUT and
+ * later jobs are unaffected.  The default (2^22) is far above any real wait; 0
+ * polls make every such wait fail (a hook for tests of that failure path). */
+int silvan_job_commit_polls(silvan_job_t j, uint32_t polls);
+
 int silvan_job_destroy(silvan_job_t j);
 
 /* ---- step-wise interface ------------------------------------------------- */

@@ -393,6 +393,15 @@ int silvan_job_run(silvan_job_t j, silvan_result_t *res, void *log) {
     return j->job->run(res, (FILE *)log);
 }
 
+int silvan_job_commit_polls(silvan_job_t j, uint32_t polls) {
+    if (!j) {
+        set_error("null argument");
+        return SILVAN_E_BADARG;
+    }
+    j->job->set_commit_polls(polls);
+    return SILVAN_OK;
+}
+
 int silvan_run_rounds(silvan_job_t j, uint32_t rounds, silvan_status_t *st, void *log) {
     if (!j) {
         set_error("null argument");

@@ -39,15 +39,18 @@ namespace {
 //   D  each bucket put in sample order, its entries with their factor and
 //      signs: the huge buckets by whole CTAs (claimed from a cursor), then the
 //      others one warp each (fixed assignment); cursors zeroed
-// Each barrier is bounded: a CTA that waits longer than kBarrierPolls polls
-// records SILVAN_E_TIMEOUT in the job's error word and leaves the kernel.
+// Each barrier is bounded: a CTA that waits longer than ApplyArgs::polls polls
+// records SILVAN_E_TIMEOUT in the job's error word and leaves the kernel.  Such a
+// draw is published with no touched node, so that the commit rounds queued behind
+// it read none of the buckets, and a later draw of the job (its error is only
+// seen at the next check) ends at once: the counts it would start from are not
+// zero.
 //
 // Once per draw, not per commit round: an estimation commits a draw in about
 // ten rounds, and the three barriers and their phases were more than half of
 // each (R-MAT 20, a million nodes: 14 of 31-35 us; a round is now 27 and the draw 55 once).
 // ---------------------------------------------------------------------------
 constexpr int kCommitThreads = 1024;
-constexpr uint32_t kBarrierPolls = 1u << 22;  // far above any real wait (microseconds)
 
 __device__ __forceinline__ uint32_t round_records(const RoundBuffers &rb, const ApplyArgs &a) {
     return (uint32_t)min((uint64_t)a.n_records, rb.rec_cap);
@@ -292,16 +295,21 @@ __device__ void order_others(const RoundBuffers &rb, uint32_t T, OrderSmem &sm) 
     }
 }
 
-// The last CTA out keeps the draw's counts and zeroes the control words.
-__device__ void prepare_exit(const RoundBuffers &rb) {
+// The last CTA out keeps the draw's counts (zeros when a CTA did not reach the
+// end) and zeroes the control words.
+__device__ void prepare_exit(const RoundBuffers &rb, bool complete) {
     __syncthreads();
     if (threadIdx.x == 0) {
+        if (!complete) atomicExch(rb.n_touched + 10, 1u);
         __threadfence();
         if (atomicAdd(rb.n_touched + 6, 1u) == gridDim.x - 1) {
-            rb.n_touched[8] = __ldcg(&rb.n_touched[0]);
-            rb.n_touched[9] = __ldcg(&rb.n_touched[1]);
+            const bool all = __ldcg(&rb.n_touched[10]) == 0u;
+            rb.n_touched[8] = all ? __ldcg(&rb.n_touched[0]) : 0u;
+            rb.n_touched[9] = all ? __ldcg(&rb.n_touched[1]) : 0u;
+            rb.n_touched[10] = 0u;
             rb.n_touched[0] = 0u;
             rb.n_touched[1] = 0u;
+            rb.n_touched[2] = 0u;  // arrivals at a barrier that was given up
             rb.n_touched[4] = 0u;
             rb.n_touched[5] = 0u;
             rb.n_touched[6] = 0u;
@@ -317,14 +325,18 @@ __global__ void __launch_bounds__(kCommitThreads, 1) prepare_draw_kernel(const A
     const JobCounters &jc = st.jc;
     const ApplyArgs &a = st.a;
     uint32_t *bar = rb.n_touched + 2;
+    if (__ldcg(&jc.sc->error) == SILVAN_E_TIMEOUT) {  // the job has failed
+        prepare_exit(rb, false);
+        return;
+    }
     bucket_count(rb, a);
-    if (!grid_barrier(bar, kBarrierPolls)) goto timeout;
+    if (!grid_barrier(bar, a.polls)) goto timeout;
     {
         const uint32_t T = __ldcg(rb.n_touched);
         bucket_alloc(rb, T);
-        if (!grid_barrier(bar, kBarrierPolls)) goto timeout;
+        if (!grid_barrier(bar, a.polls)) goto timeout;
         bucket_scatter(rb, a);
-        if (!grid_barrier(bar, kBarrierPolls)) goto timeout;
+        if (!grid_barrier(bar, a.polls)) goto timeout;
         order_huge(rb, jc, a.count, sm);
         order_others(rb, T, sm);
         // the scatter cursors back to zero for the next draw
@@ -332,11 +344,11 @@ __global__ void __launch_bounds__(kCommitThreads, 1) prepare_draw_kernel(const A
              t += gridDim.x * blockDim.x)
             rb.node_cnt[rb.touched[t]] = 0;
     }
-    prepare_exit(rb);
+    prepare_exit(rb, true);
     return;
 timeout:
     if (threadIdx.x == 0) atomicCAS(&jc.sc->error, 0, SILVAN_E_TIMEOUT);
-    prepare_exit(rb);
+    prepare_exit(rb, false);
 }
 
 // ---------------------------------------------------------------------------

@@ -12,6 +12,8 @@ namespace silvan {
 
 constexpr uint32_t kDrawSamples = 65536;  // samples of a draw at most
 constexpr uint32_t kHugeBucket = 256;     // larger buckets are ordered by a whole CTA
+// Polls of a grid barrier of prepare_draw: far above any real wait (microseconds).
+constexpr uint32_t kCommitPolls = 1u << 22;
 constexpr int kMaxPartitions = 128;
 
 // Job-level scalars kept on the device.
@@ -57,10 +59,11 @@ struct RoundBuffers {
     // bucketing by node
     uint32_t *node_cnt;      // n, zero between rounds
     uint32_t *touched;       // distinct nodes of the round
-    // control words (zero when allocated; prepare_draw leaves [0..7] zero):
-    // [0] touched nodes, [1] large buckets, [2..3] grid barrier, [4]
+    // control words (zero when allocated; prepare_draw leaves [0..2], [4..7] and
+    // [10] zero): [0] touched nodes, [1] large buckets, [2..3] grid barrier, [4]
     // bucket-space cursor, [5] claims of the huge ones, [6] CTAs done, [7] huge
-    // buckets; of the prepared draw: [8] touched nodes, [9] large buckets
+    // buckets, [10] set when a CTA left early; of the prepared draw: [8] touched
+    // nodes, [9] large buckets (both zero when a barrier was given up)
     uint32_t *n_touched;
     uint32_t *bucket_off;    // start of each touched node's bucket
     uint32_t *bucket_len;    // its number of entries
@@ -99,6 +102,7 @@ struct ApplyArgs {
     uint32_t D;
     int32_t journal;         // save what the round changes (RoundJournal) so it can be undone
     uint32_t stamp;          // of a journaled round: distinct from every earlier one's
+    uint32_t polls;          // of each grid barrier of prepare_draw
 };
 
 // What a journaled commit round overwrites: the old counters of each node it

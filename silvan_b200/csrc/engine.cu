@@ -1375,6 +1375,7 @@ ApplyState Job::apply_state(const JobRequest &r) {
     a.pass = r.pass;
     a.track_cross = r.track_cross ? 1 : 0;
     a.D = g_->diameter;
+    a.polls = commit_polls_;
     return st;
 }
 

@@ -307,6 +307,8 @@ class Job {
     int read_counters(double *approx, double *wimpy, int64_t *mcrade, int32_t *part);
     int read_topk(uint32_t *nodes, double *values, uint32_t cap, uint32_t *count);
 
+    void set_commit_polls(uint32_t polls) { commit_polls_ = polls; }
+
     // ---- used by Engine -------------------------------------------------------
     DeviceGraph *graph() const { return g_; }
     const silvan_params_t &params() const { return p_; }
@@ -365,6 +367,7 @@ class Job {
     // run or moves the next schedule point
     RoundJournal jr_{};
     uint32_t stamp_ = 0;  // of the last journaled round
+    uint32_t commit_polls_ = kCommitPolls;  // of the commit's grid barriers
     cudaEvent_t ev_chk_ = nullptr;  // the check's reads have landed
     struct Overlap {
         bool on = false;      // on_drawn is committing a drawn range
