@@ -12,10 +12,12 @@
 // while its own row is scanned for the next level (undirected graphs; directed
 // ones pull it from the reverse row).  Backward: with
 // g(w) = (1 + delta(w)) / sigma(w), delta(v) = sigma(v) x the sum of g over v's
-// successors on the next level; g(v) then takes sigma(v)'s place.  Path counts
-// are integers below 2^53, so their sums are exact in any order, and every
-// other sum runs in the row's order over fixed lanes: the value does not
-// depend on scheduling.
+// successors on the next level; g(v) then takes sigma(v)'s place.  Every sum
+// runs in the row's order over fixed lanes, so the value does not depend on
+// scheduling, except that rows which do not match (kForward) add their path
+// counts in the order of arrival: exact up to 2^53, rounded beyond.  A count
+// beyond the doubles' range is infinite: the pairs that end in such a node add
+// nothing, and a node with one whose successors have one too gets NaN.
 //
 // What bounds it: two scans of all rows per source, each entry a probe of the
 // neighbour's level.  Up to 19,164 nodes, the levels, the queue, the path
@@ -28,6 +30,7 @@
 #include "brandes.h"
 
 #include <algorithm>
+#include <cfloat>
 #include <vector>
 
 namespace silvan {
@@ -239,7 +242,14 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) brandes_kernel(BrandesArg
                           return ok && (uint32_t)dist[x] == (uint32_t)l + 1u ? val[x] : 0.0;
                       },
                       [&](uint32_t v, double a) {
-                          const double sg = val[v], delta = sg * a;
+                          const double sg = val[v];
+                          double delta = sg * a;
+                          if (sg > DBL_MAX) {  // infinity times nothing is nothing
+                              const uint32_t e = A.out_off[v + 1];
+                              uint32_t k = A.out_off[v];
+                              while (k < e && (uint32_t)dist[A.out_adj[k]] != (uint32_t)l + 1u) k++;
+                              if (k == e) delta = 0.0;
+                          }
                           if (v != s) sum[v] += delta;
                           val[v] = (1.0 + delta) / sg;
                       });
