@@ -153,6 +153,15 @@ __device__ __forceinline__ DrawEntry draw_entry(const RoundBuffers &rb, unsigned
     return d;
 }
 
+// In sample order at `pos`: x where the records were (read for the last time
+// before the barrier), sample and signs in the place of an entry (of the same
+// bucket, whose entries the caller has read).  20 bytes a record in all.
+__device__ __forceinline__ void entry_store(const RoundBuffers &rb, uint32_t pos,
+                                            const DrawEntry &d) {
+    rb.x[pos] = d.x;
+    rb.entries[pos] = (unsigned long long)d.sample << 32 | d.signs;
+}
+
 // Shared memory of phase D: the samples of the CTA's huge bucket and the set
 // bits before each word; then each warp's bucket.
 struct OrderSmem {
@@ -189,7 +198,7 @@ __device__ void order_huge(const RoundBuffers &rb, const JobCounters &jc, uint32
         if (b > S) {  // more entries than samples: not a bucket of distinct samples
             if (threadIdx.x == 0) {
                 atomicCAS(&jc.sc->error, 0, SILVAN_E_STATE);
-                rb.bucket_span[t] = make_uint2(0u, 0u);
+                rb.bucket_span[t] = make_ushort2(0, 0);
             }
             __syncthreads();
             continue;
@@ -232,13 +241,20 @@ __device__ void order_huge(const RoundBuffers &rb, const JobCounters &jc, uint32
             if (sidx >= S) continue;
             const uint32_t w = sidx >> 5;
             const uint32_t r = sm.h.wpre[w] + __popc(sm.h.bits[w] & ((1u << (sidx & 31)) - 1u));
-            rb.sorted[b0 + r] = draw_entry(rb, e);
-            uint32_t *span = reinterpret_cast<uint32_t *>(&rb.bucket_span[t]);
-            if (r == 0u) span[0] = sidx;
-            if (r == b - 1u) span[1] = sidx;
+            rb.x[b0 + r] = draw_entry(rb, e).x;
+            rb.order[b0 + r] = sidx;
+            uint16_t *span = reinterpret_cast<uint16_t *>(&rb.bucket_span[t]);
+            if (r == 0u) span[0] = (uint16_t)sidx;
+            if (r == b - 1u) span[1] = (uint16_t)sidx;
         }
         __syncwarp();
         __syncthreads();
+        // all entries are read: samples and signs take their places
+        for (uint32_t i = threadIdx.x; i < b; i += kCommitThreads) {
+            const uint32_t sidx = __ldcg(&rb.order[b0 + i]);
+            if (sidx < S)
+                rb.entries[b0 + i] = (unsigned long long)sidx << 32 | __ldcg(&rb.signs[sidx]);
+        }
     }
     __syncthreads();
 }
@@ -256,16 +272,16 @@ __device__ void order_others(const RoundBuffers &rb, uint32_t T, OrderSmem &sm) 
         const uint32_t b = __ldcg(&rb.bucket_len[t]);
         if (b > kHugeBucket) continue;
         const uint32_t off = __ldcg(&rb.bucket_off[t]);
-        uint32_t *span = reinterpret_cast<uint32_t *>(&rb.bucket_span[t]);
+        uint16_t *span = reinterpret_cast<uint16_t *>(&rb.bucket_span[t]);
         if (b <= 32u) {
             const unsigned long long key = lane < b ? __ldcg(&rb.entries[off + lane]) : ~0ull;
             uint32_t rank = 0;
             for (uint32_t j = 0; j < b; j++)
                 rank += __shfl_sync(0xffffffffu, key, (int)j) < key;
             if (lane < b) {
-                rb.sorted[off + rank] = draw_entry(rb, key);
-                if (rank == 0u) span[0] = (uint32_t)(key >> 32);
-                if (rank == b - 1u) span[1] = (uint32_t)(key >> 32);
+                entry_store(rb, off + rank, draw_entry(rb, key));
+                if (rank == 0u) span[0] = (uint16_t)(key >> 32);
+                if (rank == b - 1u) span[1] = (uint16_t)(key >> 32);
             }
         } else {
             unsigned long long key[kKeys];
@@ -286,9 +302,9 @@ __device__ void order_others(const RoundBuffers &rb, uint32_t T, OrderSmem &sm) 
 #pragma unroll
             for (uint32_t r = 0; r < kKeys; r++) {
                 if (r * 32u + lane >= b) continue;
-                rb.sorted[off + rank[r]] = draw_entry(rb, key[r]);
-                if (rank[r] == 0u) span[0] = (uint32_t)(key[r] >> 32);
-                if (rank[r] == b - 1u) span[1] = (uint32_t)(key[r] >> 32);
+                entry_store(rb, off + rank[r], draw_entry(rb, key[r]));
+                if (rank[r] == 0u) span[0] = (uint16_t)(key[r] >> 32);
+                if (rank[r] == b - 1u) span[1] = (uint16_t)(key[r] >> 32);
             }
         }
         __syncwarp();
@@ -450,8 +466,6 @@ __device__ __forceinline__ void fold_journal(const RoundJournal &jr, const Apply
         jr.last_upd[t] = s.lu0;
     } else if (lane == 26) {
         jr.wimpy[t] = s.v;
-    } else if (lane == 27) {
-        jr.stamp[t] = a.stamp;
     }
 }
 
@@ -599,12 +613,12 @@ __device__ __forceinline__ void fold_stage(FoldScratch &fs, uint32_t i, const Dr
     fs.sample[i] = e.sample;
 }
 
-__device__ __forceinline__ DrawEntry entry_load(const DrawEntry *p) {
-    const uint4 w = __ldcg(reinterpret_cast<const uint4 *>(p));
+__device__ __forceinline__ DrawEntry entry_load(const RoundBuffers &rb, uint32_t pos) {
+    const unsigned long long m = __ldcg(&rb.entries[pos]);
     DrawEntry e;
-    e.x = __hiloint2double((int)w.y, (int)w.x);
-    e.signs = w.z;
-    e.sample = w.w;
+    e.x = __ldcg(&rb.x[pos]);
+    e.signs = (uint32_t)m;
+    e.sample = (uint32_t)(m >> 32);
     return e;
 }
 
@@ -623,16 +637,17 @@ __device__ void fold_large(const RoundBuffers &rb, const JobCounters &jc, const 
     for (uint32_t li = w; li < NL; li += nw) {
         const uint32_t t = __ldcg(&rb.large[li]);
         const uint32_t off = __ldcg(&rb.bucket_off[t]), b = __ldcg(&rb.bucket_len[t]);
-        const uint2 span = __ldcg(&rb.bucket_span[t]);
+        const ushort2 span = __ldcg(&rb.bucket_span[t]);
         const uint32_t node = __ldcg(&rb.touched[t]);
         if (span.x >= a.hi || span.y < a.lo) continue;
         NodeState st = fold_load(jc, a, node);
-        const DrawEntry *E = rb.sorted + off;
+        // the samples are the entries' high words
+        const uint32_t *sample = reinterpret_cast<const uint32_t *>(rb.entries + off) + 1;
         uint32_t l = 0, h = span.x >= a.lo ? 0u : b;  // first entry at or beyond lo in [l, h]
         while (h > l) {
             const uint32_t step = (h - l + 31u) / 32u;
             const uint32_t i = l + lane * step;
-            const bool below = i < h && __ldcg(&E[i].sample) < a.lo;
+            const bool below = i < h && __ldcg(&sample[2u * i]) < a.lo;
             const uint32_t k = (uint32_t)__popc(__ballot_sync(0xffffffffu, below));
             if (k == 0u) break;
             h = min(h, l + k * step);
@@ -641,7 +656,7 @@ __device__ void fold_large(const RoundBuffers &rb, const JobCounters &jc, const 
         DrawEntry e{0.0, 0u, 0xffffffffu}, next[kAhead];
 #pragma unroll
         for (uint32_t p = 0; p < kAhead; p++)
-            if (l + p * 32u + lane < b) next[p] = entry_load(&E[l + p * 32u + lane]);
+            if (l + p * 32u + lane < b) next[p] = entry_load(rb, off + l + p * 32u + lane);
         const bool few = (uint64_t)a.first_sample + a.hi < (1ull << 26);
         bool first = true;
         for (uint32_t i = l;; i += 32u) {
@@ -655,7 +670,7 @@ __device__ void fold_large(const RoundBuffers &rb, const JobCounters &jc, const 
             first = false;
             if (lane < k) fold_stage(fs, lane, e);
             const uint32_t far = i + kAhead * 32u + lane;
-            if (far < b) next[kAhead - 1] = entry_load(&E[far]);
+            if (far < b) next[kAhead - 1] = entry_load(rb, off + far);
             __syncwarp();
             const bool one = e.x == 1.0;
             const bool plain = one || (e.x >= 0x1p-25 && e.x <= 1.0 - 0x1p-25);
@@ -679,7 +694,7 @@ __device__ void fold_small(const RoundBuffers &rb, const JobCounters &jc, const 
     for (uint32_t t0 = w * kBatch; t0 < T; t0 += nw * kBatch) {
         const uint32_t t = t0 + lane;
         uint32_t off = 0, len = 33, node = 0;
-        uint2 span = make_uint2(0u, 0u);
+        ushort2 span = make_ushort2(0, 0);
         if (lane < kBatch && t < T) {
             off = __ldcg(&rb.bucket_off[t]);
             len = __ldcg(&rb.bucket_len[t]);
@@ -693,7 +708,7 @@ __device__ void fold_small(const RoundBuffers &rb, const JobCounters &jc, const 
         DrawEntry e_n{0.0, 0u, 0xffffffffu};
         NodeState s_n{0.0, 0u, 0u, true};
         if (m) {
-            if (lane < l_n) e_n = entry_load(&rb.sorted[o_n + lane]);
+            if (lane < l_n) e_n = entry_load(rb, o_n + lane);
             s_n = fold_load(jc, a, v_n);
         }
         while (m) {
@@ -707,7 +722,7 @@ __device__ void fold_small(const RoundBuffers &rb, const JobCounters &jc, const 
                 l_n = __shfl_sync(0xffffffffu, len, i);
                 v_n = __shfl_sync(0xffffffffu, node, i);
                 e_n.sample = 0xffffffffu;
-                if (lane < l_n) e_n = entry_load(&rb.sorted[o_n + lane]);
+                if (lane < l_n) e_n = entry_load(rb, o_n + lane);
                 s_n = fold_load(jc, a, v_n);
             }
             const bool in = lane < l && e.sample >= a.lo && e.sample < a.hi;
@@ -809,16 +824,19 @@ cudaError_t apply_init() {
     return cudaSuccess;
 }
 
-// One warp per node of the draw's touched list that the round saved, lanes as
-// in the fold.
+// One warp per node of the draw's touched list, lanes as in the fold.  The nodes
+// that the round folded (and saved) have a last update at or beyond `from`, the
+// round's first sample + 1: every contribution is positive.
 __global__ void undo_round_kernel(RoundBuffers rb, JobCounters jc, RoundJournal jr, int pass,
-                                  uint32_t D, uint32_t stamp) {
+                                  uint32_t D, uint32_t from) {
     const uint32_t T = __ldcg(rb.n_touched + 8);
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < T; t += nw) {
-        if (jr.stamp[t] != stamp) continue;
         const uint32_t node = rb.touched[t];
+        const bool folded = jc.last_upd[node] >= from;
+        __syncwarp();  // every lane has looked before lane 25 writes
+        if (!folded) continue;
         if (lane < kTrials) {
             if (pass == 2)
                 jc.mcrade[(uint64_t)node * kTrials + lane] = jr.mcrade[(uint64_t)t * kTrials + lane];
@@ -1117,8 +1135,8 @@ __global__ void divide_kernel(const double *approx, double m, double *out, uint3
 }
 
 cudaError_t undo_round(const RoundBuffers &rb, const JobCounters &jc, const RoundJournal &jr,
-                       int pass, uint32_t D, uint32_t stamp, cudaStream_t stream) {
-    undo_round_kernel<<<296, 512, 0, stream>>>(rb, jc, jr, pass, D, stamp);
+                       int pass, uint32_t D, uint32_t from, cudaStream_t stream) {
+    undo_round_kernel<<<296, 512, 0, stream>>>(rb, jc, jr, pass, D, from);
     return cudaGetLastError();
 }
 

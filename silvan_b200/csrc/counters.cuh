@@ -35,7 +35,7 @@ struct JobScalars {
 static_assert(sizeof(JobScalars) % 8 == 0, "JobScalars is copied in 8-byte words");
 
 // One contribution to a node, as a commit round reads it.
-struct __align__(16) DrawEntry {
+struct DrawEntry {
     double x;         // count * (1 / num_paths)
     uint32_t signs;   // the sample's Rademacher signs
     uint32_t sample;  // round-local index
@@ -67,12 +67,19 @@ struct RoundBuffers {
     uint32_t *n_touched;
     uint32_t *bucket_off;    // start of each touched node's bucket
     uint32_t *bucket_len;    // its number of entries
-    uint2 *bucket_span;      // its first and last sample
-    uint32_t *large;         // buckets of more than 32 entries (listed by bucket_alloc)
+    ushort2 *bucket_span;    // its first and last sample
+    // buckets of more than 32 entries (listed by bucket_alloc): fewer than a
+    // 32nd of the records
+    uint32_t *large;
     uint32_t *n_large;       // = n_touched + 1 (both zeroed together)
     uint32_t *huge;          // buckets of more than kHugeBucket entries
-    unsigned long long *entries;  // sample << 32 | count, grouped by node
-    DrawEntry *sorted;            // the same, each bucket in sample order
+    // grouped by node: sample << 32 | count, and from prepare_draw on, each
+    // bucket in sample order, sample << 32 | signs
+    unsigned long long *entries;
+    // in the records' place once those are grouped: a bucket's contributions in
+    // sample order, and behind them the order of the huge ones while it is found
+    double *x;
+    uint32_t *order;
     uint32_t *work_counter;  // sampler work counter
 };
 
@@ -101,7 +108,6 @@ struct ApplyArgs {
     int32_t track_cross;     // pass 1 of top-k mode
     uint32_t D;
     int32_t journal;         // save what the round changes (RoundJournal) so it can be undone
-    uint32_t stamp;          // of a journaled round: distinct from every earlier one's
     uint32_t polls;          // of each grid barrier of prepare_draw
 };
 
@@ -116,7 +122,6 @@ struct RoundJournal {
     double *approx;        // n
     double *wimpy;         // n
     uint32_t *last_upd;    // n
-    uint32_t *stamp;       // n: the journaled round that saved the entry
     JobScalars *sc;        // 1
     uint64_t *sp_lengths;  // D + 1
 };
@@ -139,11 +144,12 @@ cudaError_t apply_round(const ApplyState &st, cudaStream_t stream);
 // Resident grid of the prepare kernel on the current device (call before
 // capturing).
 cudaError_t apply_init();
-// Restores what the last commit round (journaled with `stamp`) changed: the
-// nodes it folded, and the scalars and path-length counts as the check before
-// it saved them.
+// Restores what the last commit round (journaled) changed: the nodes it folded,
+// whose last_upd is at or beyond `from` (1 + the global index of the round's first
+// sample), and the scalars and path-length counts as the check before it saved
+// them.
 cudaError_t undo_round(const RoundBuffers &rb, const JobCounters &jc, const RoundJournal &jr,
-                       int pass, uint32_t D, uint32_t stamp, cudaStream_t stream);
+                       int pass, uint32_t D, uint32_t from, cudaStream_t stream);
 
 // Reduction for one stopping-rule evaluation: per partition and trial the
 // maximum of mcrade (LLONG_MIN when no node of the partition was updated;

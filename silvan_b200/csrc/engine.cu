@@ -1190,7 +1190,6 @@ Job::~Job() {
     dfree(r.bucket_off);
     dfree(r.bucket_len);
     dfree(r.entries);
-    dfree(r.sorted);
     dfree(r.bucket_span);
     dfree(r.huge);
     dfree(jc_.approx);
@@ -1217,7 +1216,6 @@ Job::~Job() {
     dfree(jr_.approx);
     dfree(jr_.wimpy);
     dfree(jr_.last_upd);
-    dfree(jr_.stamp);
     dfree(jr_.sc);
     dfree(jr_.sp_lengths);
     if (ev_chk_) cudaEventDestroy(ev_chk_);
@@ -1265,18 +1263,19 @@ int Job::grow_records(uint64_t cap) {
     dfree(r.bucket_off);
     dfree(r.bucket_len);
     dfree(r.entries);
-    dfree(r.sorted);
     dfree(r.bucket_span);
     dfree(r.huge);
     r.rec_cap = cap;
     const uint64_t tcap = std::min<uint64_t>(cap, n_) + 1;
     RK(dmalloc(&r.recs, cap));
+    static_assert(sizeof(PathRec) >= sizeof(double) + sizeof(uint32_t), "x and order fit");
+    r.x = reinterpret_cast<double *>(r.recs);
+    r.order = reinterpret_cast<uint32_t *>(r.x + cap);
     RK(dmalloc(&r.touched, tcap));
-    RK(dmalloc(&r.large, tcap));
+    RK(dmalloc(&r.large, std::min<uint64_t>(tcap, cap / 33 + 1)));
     RK(dmalloc(&r.bucket_off, tcap + 1));
     RK(dmalloc(&r.bucket_len, tcap));
     RK(dmalloc(&r.entries, cap));
-    RK(dmalloc(&r.sorted, cap));
     RK(dmalloc(&r.bucket_span, tcap));
     RK(dmalloc(&r.huge, cap / kHugeBucket + 1));
     return SILVAN_OK;
@@ -1285,8 +1284,8 @@ int Job::grow_records(uint64_t cap) {
 uint64_t Job::device_bytes() const {
     const uint64_t n = n_;
     uint64_t b = n * (8 + 8 + 8 * kTrials + 4 + 1 + 4 + 4 + 4 + 4);
-    if (p_.k == 0) b += n * (8 * kTrials + 8 + 8 + 4 + 4);  // the round journal
-    b += (uint64_t)kRoundSamples * 36 + rb_.rec_cap * (12 + 8 + sizeof(DrawEntry)) +
+    if (p_.k == 0) b += n * (8 * kTrials + 8 + 8 + 4);  // the round journal
+    b += (uint64_t)kRoundSamples * 36 + rb_.rec_cap * (12 + 8) +
          std::min<uint64_t>(rb_.rec_cap, n) * 16;
     return b;
 }
@@ -1328,8 +1327,6 @@ int Job::init() {
         RK(dmalloc(&jr_.approx, n));
         RK(dmalloc(&jr_.wimpy, n));
         RK(dmalloc(&jr_.last_upd, n));
-        RK(dmalloc(&jr_.stamp, n));
-        CK(cudaMemset(jr_.stamp, 0, sizeof(uint32_t) * n));
         RK(dmalloc(&jr_.sc, 1));
         RK(dmalloc(&jr_.sp_lengths, (uint64_t)g_->diameter + 1));
         CK(cudaEventCreateWithFlags(&ev_chk_, cudaEventDisableTiming));
@@ -1399,7 +1396,6 @@ int Job::apply_range(const JobRequest &r, uint32_t lo, uint32_t hi, bool journal
     if (lo >= hi) return SILVAN_OK;
     ApplyState st = apply_state(r);
     st.a.journal = journal ? 1 : 0;
-    st.a.stamp = journal ? ++stamp_ : 0u;
     st.a.lo = lo;
     st.a.hi = hi;
     CK(apply_round(st, stream_));
@@ -2114,7 +2110,8 @@ int Job::speculate() {
 }
 
 int Job::undo_speculation() {
-    CK(undo_round(rb_, jc_, jr_, 2, g_->diameter, stamp_, stream_));
+    CK(undo_round(rb_, jc_, jr_, 2, g_->diameter,
+                  (uint32_t)(base_global_ + ov_.spec_lo + 1), stream_));
     launches += 1;
     ov_.spec_lo = ov_.spec_hi = 0;
     return SILVAN_OK;

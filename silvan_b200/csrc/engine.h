@@ -366,7 +366,6 @@ class Job {
     // while the host evaluates the check, and undone if the check stops the
     // run or moves the next schedule point
     RoundJournal jr_{};
-    uint32_t stamp_ = 0;  // of the last journaled round
     uint32_t commit_polls_ = kCommitPolls;  // of the commit's grid barriers
     cudaEvent_t ev_chk_ = nullptr;  // the check's reads have landed
     struct Overlap {

@@ -83,8 +83,8 @@ struct Server {
 
     static uint64_t job_bytes(uint64_t n, uint64_t D) {
         // counters + node buckets + round buffers at their initial capacity
-        return n * (8 + 8 + 8ull * kTrials + 4 + 1 + 4 + 4 + 4 + 4 + 8 + 8 + 4) + (D + 1) * 8 +
-               65536ull * 36 + (1ull << 20) * (20 + sizeof(DrawEntry)) + (64ull << 20);
+        return n * (8 + 8 + 8ull * kTrials + 4 + 1 + 4 + 4 + 4 + 4 + 8) + (D + 1) * 8 +
+               65536ull * 36 + (1ull << 20) * 20 + (64ull << 20);
     }
 
     void loop(int device) {
