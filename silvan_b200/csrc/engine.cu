@@ -438,6 +438,18 @@ DeviceGraph::~DeviceGraph() {
 // ---------------------------------------------------------------------------
 // SlotPool
 // ---------------------------------------------------------------------------
+namespace {
+constexpr uint64_t align256(uint64_t b) { return (b + 255) & ~255ull; }
+
+// The next `count` elements of a block, 256-byte aligned like the block.
+template <typename T>
+T *take(uint8_t *&p, uint64_t count) {
+    T *at = reinterpret_cast<T *>(p);
+    p += align256(sizeof(T) * count);
+    return at;
+}
+}  // namespace
+
 uint64_t SlotPool::bytes_per_slot(uint64_t n) {
     return n * (sizeof(NodeRec) + 12) + (uint64_t)kMeetCap * 16 + 4 * state_words(n);
 }
@@ -448,12 +460,16 @@ int SlotPool::alloc(uint32_t s, uint64_t nn, cudaStream_t st) {
     n = nn;
     const uint64_t tot = (uint64_t)s * nn;
     RK(dmalloc(&rec, tot));
-    RK(dmalloc(&queue, tot));
     RK(dmalloc(&hits, tot));
-    RK(dmalloc(&touched, tot));
-    RK(dmalloc(&meet, (uint64_t)s * kMeetCap));
-    RK(dmalloc(&meet_pre, (uint64_t)s * kMeetCap));
     RK(dmalloc(&states, s * state_words(nn)));
+    const uint64_t meets = (uint64_t)s * kMeetCap;
+    scratch_bytes = 2 * align256(4 * tot) + 16 * meets;
+    RK(dmalloc(&scratch, scratch_bytes));
+    uint8_t *p = scratch;
+    queue = take<uint32_t>(p, tot);
+    touched = take<uint32_t>(p, tot);
+    meet = take<uint2>(p, meets);
+    meet_pre = take<uint64_t>(p, meets);
     CK(init(st));
     CK(cudaStreamSynchronize(st));
     return SILVAN_OK;
@@ -468,12 +484,9 @@ cudaError_t SlotPool::init(cudaStream_t st) {
 
 void SlotPool::free_all() {
     dfree(rec);
-    dfree(queue);
     dfree(hits);
-    dfree(touched);
-    dfree(meet);
-    dfree(meet_pre);
     dfree(states);
+    dfree(scratch);
     slots = 0;
 }
 
@@ -483,21 +496,54 @@ void SlotPool::free_all() {
 uint32_t WarpPool::cap_for(uint64_t n) { return (uint32_t)std::min<uint64_t>(n, 65536u); }
 
 uint64_t WarpPool::bytes_per_warp(uint64_t cap) {
-    return cap * (sizeof(BallRec) + sizeof(uint2) + 4) + (uint64_t)kWarpMeets * 16 +
+    return cap * kBallBytes + (uint64_t)kWarpMeets * 16 +
            2ull * kWarpLevels * sizeof(uint2);
 }
 
-int WarpPool::alloc(uint32_t w, uint32_t cap) {
-    free_all();
+uint64_t WarpPool::bytes(uint64_t warps, uint64_t cap) {
+    return warps * bytes_per_warp(cap) + 6 * 256;  // the arrays' alignment
+}
+
+void WarpPool::place(uint8_t *p, uint32_t w, uint32_t cap) {
     warps = w;
     s.cap = cap;
     const uint64_t tot = (uint64_t)w * cap;
-    RK(dmalloc(&s.ball, tot));
-    RK(dmalloc(&s.rows, tot));
-    RK(dmalloc(&s.touched, tot));
-    RK(dmalloc(&s.meet, (uint64_t)w * kWarpMeets));
-    RK(dmalloc(&s.mpre, (uint64_t)w * kWarpMeets));
-    RK(dmalloc(&s.lvl, (uint64_t)w * 2 * kWarpLevels));
+    s.ball = take<BallRec>(p, tot);
+    s.rows = take<uint2>(p, tot);
+    s.touched = take<uint32_t>(p, tot);
+    s.meet = take<uint2>(p, (uint64_t)w * kWarpMeets);
+    s.mpre = take<uint64_t>(p, (uint64_t)w * kWarpMeets);
+    s.lvl = take<uint2>(p, (uint64_t)w * 2 * kWarpLevels);
+}
+
+// The warps' state in `left` bytes beside the slots where that is enough for all
+// of the `most` warps, else in the slots' scratch, which the CTA sampler uses only
+// after the warp sampler has ended and does not expect to be in any state: an
+// engine whose slots take all of its memory keeps them all.  (With an eighth set
+// aside for the warps it had 95 slots instead of 109 for 200,000 nodes in 1 GiB.)
+int WarpPool::alloc(uint32_t most, uint64_t n, uint64_t left, const SlotPool &slots) {
+    free_all();
+    if (most == 0) return SILVAN_OK;
+    const uint32_t cap = cap_for(n);
+    const auto fits = [](uint64_t have) { return have > bytes(0, 0) ? have - bytes(0, 0) : 0; };
+    const uint32_t beside = (uint32_t)std::min<uint64_t>(most, fits(left) / bytes_per_warp(cap));
+    // in the scratch: balls of 4,096 nodes at least, larger ones where all warps
+    // can have them
+    const uint64_t room = fits(slots.scratch_bytes);
+    const uint32_t least = std::min<uint32_t>(cap, 4096u);
+    const uint64_t share = room / most;
+    const uint32_t c =
+        share > bytes_per_warp(least)
+            ? (uint32_t)std::min<uint64_t>(cap, (share - bytes_per_warp(0)) / kBallBytes)
+            : least;
+    const uint32_t inside = (uint32_t)std::min<uint64_t>(most, room / bytes_per_warp(c));
+    if (beside == most || beside > inside) {
+        if (dmalloc(&own, bytes(beside, cap)) == SILVAN_OK) {
+            place(own, beside, cap);
+            return SILVAN_OK;
+        }
+    }
+    if (inside > 0) place(slots.scratch, inside, c);
     return SILVAN_OK;
 }
 
@@ -513,12 +559,7 @@ int WarpPool::ensure_list(uint32_t total) {
 }
 
 void WarpPool::free_all() {
-    dfree(s.ball);
-    dfree(s.rows);
-    dfree(s.touched);
-    dfree(s.meet);
-    dfree(s.mpre);
-    dfree(s.lvl);
+    dfree(own);
     dfree(list);
     warps = list_cap = 0;
 }
@@ -575,21 +616,16 @@ int Engine::init(uint64_t n_max, uint32_t slots, uint64_t mem_budget) {
         CK(cudaMemGetInfo(&fr, &tot));
         mem_budget = (fr + block_cache().idle_bytes(dev)) / 2;
     }
-    // the warp sampler's state: as many warps as stay resident, within an
-    // eighth of the budget
-    {
-        const uint32_t cap = WarpPool::cap_for(n_max);
-        const uint64_t per = WarpPool::bytes_per_warp(cap);
-        const uint64_t most = (uint64_t)sms * std::max(0, warp_sampler_per_sm());
-        const uint64_t w = std::min<uint64_t>(most, mem_budget / 8 / per);
-        if (w > 0) {
-            RK(warps_.alloc((uint32_t)w, cap));
-            mem_budget -= w * per;
-        }
-    }
-    const uint64_t fit = mem_budget / std::max<uint64_t>(SlotPool::bytes_per_slot(n_max), 1);
+    // the slots first, then the warp sampler's state in what they leave, at most
+    // an eighth of the budget
+    const uint64_t per_slot = std::max<uint64_t>(SlotPool::bytes_per_slot(n_max), 1);
+    const uint64_t fit = mem_budget / per_slot;
     if (fit < slots) slots = (uint32_t)std::max<uint64_t>(fit, 1);
     RK(slots_.alloc(slots, n_max, stream_));
+    const uint64_t taken = slots * per_slot;
+    RK(warps_.alloc((uint32_t)sms * (uint32_t)std::max(0, warp_sampler_per_sm()), n_max,
+                    std::min(mem_budget / 8, mem_budget > taken ? mem_budget - taken : 0),
+                    slots_));
     RK(device_alloc(&board_mem_, assist_board_bytes(n_max)));
     CK(assist_board_init(&board_, board_mem_, n_max, stream_));
     for (int b = 0; b < kNB; b++) max_grid_[b] = std::min(resident[b], slots);
@@ -864,6 +900,11 @@ int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> 
             if (ai != 0u && ai != 0xffffffffu) warp = false;
         }
     }
+    if (warp && total > warps_.list_cap) {
+        // no room for the list of what they leave: the CTAs draw it all
+        if (warps_.ensure_list(total) != SILVAN_OK) warp = false;
+        drop_execs();
+    }
     const int block = choose_block(jobs, reqs, idx, total, warp);
     int bi = -1;
     for (int b = 0; b < kNB; b++)
@@ -873,10 +914,6 @@ int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> 
         return SILVAN_E_BADARG;
     }
     const uint32_t grid = std::min<uint32_t>(max_grid_[bi], total);
-    if (warp && total > warps_.list_cap) {
-        RK(warps_.ensure_list(total));
-        drop_execs();
-    }
     cudaGraphExec_t exec = nullptr;
     // The nodes' states: in shared memory where every graph of the round fits
     // (R-MAT 16: 7.1 ms of sampling with the records, 3.4 so; lattices of up to

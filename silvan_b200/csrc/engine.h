@@ -98,6 +98,9 @@ struct SlotPool {
     uint2 *meet = nullptr;
     uint64_t *meet_pre = nullptr;
     uint32_t *states = nullptr;
+    // queue, touched, meet and meet_pre lie in it: nothing in them outlives a sample
+    uint8_t *scratch = nullptr;
+    uint64_t scratch_bytes = 0;
     int alloc(uint32_t slots, uint64_t n, cudaStream_t s);
     cudaError_t init(cudaStream_t s);  // neutral slots, on the stream
     void free_all();
@@ -110,12 +113,16 @@ struct SlotPool {
 struct WarpPool {
     WarpSlots s{};
     uint32_t warps = 0;
+    uint8_t *own = nullptr;    // the state, unless it lies in the slots' scratch
     uint32_t *list = nullptr;  // samples left to the CTA sampler
     uint32_t list_cap = 0;
-    int alloc(uint32_t warps, uint32_t cap);
+    int alloc(uint32_t most, uint64_t n, uint64_t left, const SlotPool &slots);
     int ensure_list(uint32_t total);
     void free_all();
+    void place(uint8_t *p, uint32_t warps, uint32_t cap);
+    static constexpr uint64_t kBallBytes = sizeof(BallRec) + sizeof(uint2) + 4;  // a node
     static uint64_t bytes_per_warp(uint64_t cap);
+    static uint64_t bytes(uint64_t warps, uint64_t cap);
     static uint32_t cap_for(uint64_t n);
     ~WarpPool() { free_all(); }
 };
