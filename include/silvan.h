@@ -223,6 +223,13 @@ int silvan_read_counters(silvan_job_t j, double *approx, double *wimpy, int64_t 
  * polls make every such wait fail (a hook for tests of that failure path). */
 int silvan_job_commit_polls(silvan_job_t j, uint32_t polls);
 
+/* How the job's samples have been drawn so far (any pointer may be NULL): the
+ * slots and the warps of the engine that drew last, the samples that were tried
+ * one warp each, and those of them that were left to the general search.  The
+ * samples are the same either way. */
+int silvan_job_sampler_info(silvan_job_t j, uint32_t *slots, uint32_t *warps,
+                            uint64_t *warp_tried, uint64_t *warp_left);
+
 int silvan_job_destroy(silvan_job_t j);
 
 /* ---- step-wise interface ------------------------------------------------- */

@@ -38,7 +38,7 @@ EXPORTS = [
     "silvan_jobs_run_batched", "silvan_server_create", "silvan_server_submit",
     "silvan_server_poll", "silvan_server_wait", "silvan_server_estimates", "silvan_server_stats",
     "silvan_server_destroy", "silvan_replay_samples_noalloc", "silvan_exact_betweenness",
-    "silvan_job_commit_polls",
+    "silvan_job_commit_polls", "silvan_job_sampler_info",
 ]
 
 REQ_QUEUED, REQ_RUNNING, REQ_DONE = 1, 2, 3
@@ -130,6 +130,7 @@ def load(path: str = LIB_PATH):
         "silvan_read_topk": (C.c_int, [P, P, P, C.c_uint32, P]),
         "silvan_read_counters": (C.c_int, [P, P, P, P, P]),
         "silvan_job_commit_polls": (C.c_int, [P, C.c_uint32]),
+        "silvan_job_sampler_info": (C.c_int, [P, P, P, P, P]),
         "silvan_job_destroy": (C.c_int, [P]),
         "silvan_replay_samples": (C.c_int, [P, C.c_uint64, C.c_uint32, C.c_uint32, C.c_double,
                                             C.c_uint32, P, P, P, P, P, P, P, C.c_uint64, P]),
@@ -438,6 +439,12 @@ class Probabilistic:
     def commit_polls(self, polls):
         """Limit of the waits that group a draw's records (silvan_job_commit_polls)."""
         _check(load().silvan_job_commit_polls(self.h, polls))
+
+    def sampler_info(self):
+        """How the samples were drawn (silvan_job_sampler_info)."""
+        v = [C.c_uint32(), C.c_uint32(), C.c_uint64(), C.c_uint64()]
+        _check(load().silvan_job_sampler_info(self.h, *[C.byref(x) for x in v]))
+        return dict(zip(("slots", "warps", "warp_tried", "warp_left"), (x.value for x in v)))
 
     def step(self, rounds=1):
         """Runs at most `rounds` rounds of the job's own schedule (silvan_run_rounds)."""

@@ -402,6 +402,20 @@ int silvan_job_commit_polls(silvan_job_t j, uint32_t polls) {
     return SILVAN_OK;
 }
 
+int silvan_job_sampler_info(silvan_job_t j, uint32_t *slots, uint32_t *warps,
+                            uint64_t *warp_tried, uint64_t *warp_left) {
+    if (!j) {
+        set_error("null argument");
+        return SILVAN_E_BADARG;
+    }
+    const SamplerInfo &i = j->job->sampler_info;
+    if (slots) *slots = i.slots;
+    if (warps) *warps = i.warps;
+    if (warp_tried) *warp_tried = i.warp_tried;
+    if (warp_left) *warp_left = i.warp_left;
+    return SILVAN_OK;
+}
+
 int silvan_run_rounds(silvan_job_t j, uint32_t rounds, silvan_status_t *st, void *log) {
     if (!j) {
         set_error("null argument");

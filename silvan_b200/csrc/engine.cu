@@ -1007,6 +1007,13 @@ int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> 
         uint32_t base = 0;
         for (uint32_t s = 0; s < idx.size(); s++) {
             Job *job = jobs[idx[s]];
+            SamplerInfo &si = job->sampler_info;
+            si.slots = slots_.slots;
+            si.warps = warps_.warps;
+            if (warp && h_segs_[s].compact) {
+                si.warp_tried += reqs[idx[s]].count;
+                si.warp_left += h_cursors_[max_segs_ + s];
+            }
             if (h_cursors_[s] > job->round_buffers().rec_cap) {
                 uint64_t cap = job->round_buffers().rec_cap;
                 while (cap < h_cursors_[s]) cap *= 2;

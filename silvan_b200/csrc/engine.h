@@ -127,6 +127,13 @@ struct WarpPool {
     ~WarpPool() { free_all(); }
 };
 
+// How a job's samples were drawn: the engine that drew last, and the samples
+// tried one warp each and left by the warps, in all.
+struct SamplerInfo {
+    uint32_t slots = 0, warps = 0;
+    uint64_t warp_tried = 0, warp_left = 0;
+};
+
 struct JobRequest {
     uint32_t first_global = 0;  // global sample index of the range's first sample
     uint32_t count = 0;
@@ -323,6 +330,7 @@ class Job {
     RoundBuffers &round_buffers() { return rb_; }
     int grow_records(uint64_t cap);
     uint64_t launches = 0;
+    SamplerInfo sampler_info;
 
   private:
     enum Phase { kInit, kPass1, kPass2, kDone };
