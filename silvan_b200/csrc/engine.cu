@@ -451,7 +451,8 @@ T *take(uint8_t *&p, uint64_t count) {
 }  // namespace
 
 uint64_t SlotPool::bytes_per_slot(uint64_t n) {
-    return n * (sizeof(NodeRec) + 12) + (uint64_t)kMeetCap * 16 + 4 * state_words(n);
+    return n * (sizeof(NodeRec) + 12) + (uint64_t)kMeetCap * 16 + 16 * kSlotLevels +
+           4 * state_words(n);
 }
 
 int SlotPool::alloc(uint32_t s, uint64_t nn, cudaStream_t st) {
@@ -463,13 +464,14 @@ int SlotPool::alloc(uint32_t s, uint64_t nn, cudaStream_t st) {
     RK(dmalloc(&hits, tot));
     RK(dmalloc(&states, s * state_words(nn)));
     const uint64_t meets = (uint64_t)s * kMeetCap;
-    scratch_bytes = 2 * align256(4 * tot) + 16 * meets;
+    scratch_bytes = 2 * align256(4 * tot) + 16 * meets + 16ull * s * kSlotLevels;
     RK(dmalloc(&scratch, scratch_bytes));
     uint8_t *p = scratch;
     queue = take<uint32_t>(p, tot);
     touched = take<uint32_t>(p, tot);
     meet = take<uint2>(p, meets);
     meet_pre = take<uint64_t>(p, meets);
+    levels = take<uint2>(p, 2ull * s * kSlotLevels);
     CK(init(st));
     CK(cudaStreamSynchronize(st));
     return SILVAN_OK;
@@ -671,7 +673,7 @@ int Engine::sampler_exec(int block, uint32_t grid, bool warp, uint32_t near_cap,
     L.slots = SlotArrays{slots_.rec,     slots_.queue,     slots_.hits,
                          slots_.touched, slots_.meet,      slots_.meet_pre,
                          slots_.n,       in_slot ? slots_.states : nullptr,
-                         SlotPool::state_words(slots_.n)};
+                         SlotPool::state_words(slots_.n), slots_.levels};
     L.hdr = d_hdr_;
     L.segs = d_segs_;
     L.assist = board_;

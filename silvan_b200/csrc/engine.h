@@ -98,7 +98,8 @@ struct SlotPool {
     uint2 *meet = nullptr;
     uint64_t *meet_pre = nullptr;
     uint32_t *states = nullptr;
-    // queue, touched, meet and meet_pre lie in it: nothing in them outlives a sample
+    uint2 *levels = nullptr;
+    // queue, touched, meet, meet_pre and levels lie in it: nothing in them outlives a sample
     uint8_t *scratch = nullptr;
     uint64_t scratch_bytes = 0;
     int alloc(uint32_t slots, uint64_t n, cudaStream_t s);

@@ -156,6 +156,13 @@ int replay_samples_noalloc(const DeviceGraph &G, uint64_t seed, uint32_t first, 
     off += align256(sizeof(uint2) * kMeetCap * slots);
     S.meet_pre = (uint64_t *)(base + off);
     off += align256(sizeof(uint64_t) * kMeetCap * slots);
+    // the bounds of far levels where there is room: without them a rank far from
+    // the ends takes longer, no graph is refused for them
+    const size_t levels = align256(sizeof(uint2) * 2 * kSlotLevels * slots);
+    if (off + levels <= kScratchBytes) {
+        S.levels = (uint2 *)(base + off);
+        off += levels;
+    }
     if (off > kScratchBytes) {
         set_error("internal scratch layout overflow");
         return SILVAN_E_STATE;

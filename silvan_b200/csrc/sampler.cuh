@@ -12,6 +12,7 @@ namespace silvan {
 constexpr int kSamplerBlock = 512;   // default threads per slot
 constexpr int kSamplerBlocks[4] = {128, 256, 512, 1024};  // compiled CTA sizes
 constexpr uint32_t kMeetCap = 1u << 16;  // meeting edges per sample
+constexpr uint32_t kSlotLevels = 256;    // levels per side whose queue bounds a slot keeps
 // SegDesc::assist_items value for the default threshold: levels of at least 128
 // entries per thread of the launch's CTAs while the round has samples left, 64
 // once it is drained
@@ -153,6 +154,9 @@ struct SlotArrays {
     // between samples (nullptr: the records tell)
     uint32_t *states;
     uint64_t state_words;
+    // slot s owns [2*s*kSlotLevels, 2*(s+1)*kSlotLevels): queue bounds of levels
+    // (nullptr: only the first ones are kept)
+    uint2 *levels;
 };
 
 struct SamplerLaunch {
