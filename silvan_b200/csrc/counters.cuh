@@ -11,6 +11,7 @@
 namespace silvan {
 
 constexpr uint32_t kDrawSamples = 65536;  // samples of a draw at most
+constexpr uint32_t kSmallDraw = 64;       // the first part is committed as it is grouped
 constexpr uint32_t kHugeBucket = 256;     // larger buckets are ordered by a whole CTA
 // Polls of a grid barrier of prepare_draw: far above any real wait (microseconds).
 constexpr uint32_t kCommitPolls = 1u << 22;
@@ -136,7 +137,8 @@ struct ApplyState {
 
 // Groups the records of a draw (samples [0, a.count), a.n_records records) by
 // node, each node's in sample order, for the commit rounds that follow: one
-// cooperative kernel whose phases are separated by grid-wide barriers.
+// cooperative kernel whose phases are separated by grid-wide barriers.  It also
+// commits the samples [a.lo, a.hi), if any (for draws of up to kSmallDraw samples).
 cudaError_t prepare_draw(const ApplyState &st, cudaStream_t stream);
 // Commits round-local samples [a.lo, a.hi) of the prepared draw to the job
 // counters.

@@ -1423,11 +1423,13 @@ ApplyState Job::apply_state(const JobRequest &r) {
 }
 
 // Groups the raw outputs that the engine left in rb_ for the drawn range r, for
-// the commits of its parts.
-int Job::prepare_range(const JobRequest &r, uint64_t n_records) {
+// the commits of its parts, and commits samples [lo, hi) of a small one.
+int Job::prepare_range(const JobRequest &r, uint64_t n_records, uint32_t lo, uint32_t hi) {
     static_assert(kRoundSamples <= kDrawSamples, "a draw fits the bitmap of its samples");
     ApplyState st = apply_state(r);
     st.a.n_records = (uint32_t)n_records;
+    st.a.lo = lo;
+    st.a.hi = hi;
     CK(prepare_draw(st, stream_));
     launches += 1;
     return SILVAN_OK;
@@ -2091,17 +2093,17 @@ int Job::on_drawn(const JobRequest &r, uint64_t n_records) {
     }
     const uint64_t save_apply = launches;
     CK(cudaEventRecord(ev_commit_[0], stream_));
-    RK(prepare_range(r, n_records));
-    for (;;) {
+    for (bool grouped = false;; grouped = true) {
         JobRequest rc = r;
         rc.pass = phase_ == kPass1 ? 1 : 2;
         rc.track_cross = phase_ == kPass1 && !absolute_;
         const uint64_t cur = base_global_ + pass_samples_;
         const uint64_t c_hi = std::min(base_global_ + target_, g1);
-        if (c_hi > cur) {
-            RK(apply_range(rc, (uint32_t)(cur - g0), (uint32_t)(c_hi - g0)));
-            pass_samples_ += c_hi - cur;
-        }
+        const uint32_t lo = (uint32_t)(cur - g0), hi = (uint32_t)(std::max(c_hi, cur) - g0);
+        const bool small = !grouped && r.count <= kSmallDraw;
+        if (!grouped) RK(prepare_range(rc, n_records, lo, small ? hi : lo));
+        if (!small) RK(apply_range(rc, lo, hi));
+        pass_samples_ += hi - lo;
         if (pass_samples_ < target_) break;  // the next point lies beyond the drawn range
         const Phase ph = phase_;
         ov_.on = true;

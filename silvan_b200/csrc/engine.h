@@ -336,7 +336,7 @@ class Job {
   private:
     enum Phase { kInit, kPass1, kPass2, kDone };
     int alloc_round(uint32_t max_samples, uint64_t rec_cap);
-    int prepare_range(const JobRequest &r, uint64_t n_records);
+    int prepare_range(const JobRequest &r, uint64_t n_records, uint32_t lo, uint32_t hi);
     int apply_range(const JobRequest &r, uint32_t lo, uint32_t hi, bool journal = false);
     ApplyState apply_state(const JobRequest &r);
     int evaluate();

@@ -51,8 +51,7 @@ constexpr uint32_t kScreen = 8;
 // Levels per side with recorded bounds: the first ones in shared memory, the
 // others in the slot.  Without them the rank of a predecessor is found on the
 // node's reverse row: for a hub of 3,000 entries between two chains of 150 nodes
-// 116 ms a run instead of 5, with 12 of
-// 11,000 samples through it.
+// 116 ms a run instead of 5, with 12 of 11,000 samples through it.
 constexpr int kMaxLevels = (int)kSlotLevels, kNearLevels = 64;
 
 // Per-CTA-size constants: BLOCK threads serve one sample.  Smaller CTAs put
