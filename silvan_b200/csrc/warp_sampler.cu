@@ -707,7 +707,8 @@ __global__ void __launch_bounds__(32, 22528 / T) warp_sampler_kernel(WarpLaunch 
             const uint2 rv = make_uint2(__shfl_sync(kFull, row_v.x, i),
                                         __shfl_sync(kFull, row_v.y, i));
             const uint32_t si = __shfl_sync(kFull, sl, i);
-            uint32_t wide = 0;
+            // a graph that is not tried is one whose samples are long: listed first
+            uint32_t wide = 0xffffffffu;
             const bool done =
                 (A.compact & kCompactOn) != 0u &&
                 draw_sample(A, s, W, si, __shfl_sync(kFull, u, i), __shfl_sync(kFull, v, i),
