@@ -69,7 +69,8 @@ struct DeviceGraph {
     int device = 0;
     // Class of the graph for the sampler's schedule statistics: graphs with
     // the same direction, node count and mean degree (both to a power of 2)
-    // share them, so a stream of fresh graphs of a few shapes is tuned once.
+    // share them, long ones (lattices) apart from short ones, so a stream of
+    // fresh graphs of a few shapes is tuned once.
     uint64_t tune_class() const;
 
     int upload();  // from `host` and `cc`

@@ -1,0 +1,36 @@
+"""When the warps are tried.  A lattice whose samples they left does not rule them
+out for a short graph of the same size and degree (both to a power of two).  Each
+test has an engine of its own by a slot count that no other test asks for; results
+do not depend on the choice (Sp_sampler::random_path,
+silvan/src/Sp_sampler.cpp:41-238)."""
+import pytest
+
+from test_gpu_modes import assert_same_run
+from conftest import port_graph
+
+pytestmark = pytest.mark.gpu
+
+ONE_PATH = dict(alpha=0.0, alpha_given=True)
+
+
+@pytest.fixture(scope="module")
+def lattice(sb):
+    return sb.Graph.from_pairs(sb.grid(384, 0.05, 0.001, 1))
+
+
+def run(sb, g, eps, seed, slots, **kw):
+    job = sb.Probabilistic(g, eps, 0.1, seed=seed, slots=slots, **kw)
+    return job, job.run()
+
+
+def test_a_lattice_leaves_the_warps_to_short_graphs_of_its_class(sb, port, lattice):
+    hg = sb.HostGraph.from_pairs(sb.barabasi_albert(140000, 2, 1), False)
+    csr = hg.csr()
+    assert csr.n >> 17 == lattice.n >> 17 == 1
+    assert len(csr.out_adj) // csr.n == 3 and 2 <= 2 * 384 * 383 * 0.95 * 2 // lattice.n < 4
+    for seed in range(3):
+        info = run(sb, lattice, 0.1, seed, 26, **ONE_PATH)[0].sampler_info()
+    assert info["warp_tried"] == 0  # left out by now
+    job, res = run(sb, sb.Graph.from_host(hg), 0.02, 7, 26)
+    assert job.sampler_info()["warp_tried"] > 0
+    assert_same_run(job, res, port_graph(port, csr).run(csr.diameter, 0.02, 0.1, seed=7))
