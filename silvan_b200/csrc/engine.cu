@@ -752,11 +752,13 @@ int Engine::choose_block(const std::vector<Job *> &jobs, const std::vector<JobRe
 // round of a few samples per CTA not when more than an eighth was left: such a
 // round lasts as long as its slowest samples, and these would wait for the warps
 // first (23,000 random nodes, 2,100 samples in two rounds: 0.37 ms with the warps,
-// 0.23 without).
+// 0.23 without).  A class that is left out is tried again after kWarpRetry
+// launches of its graphs: its next graph may be another one, and a lattice loses a
+// quarter of a percent by it.
 bool Engine::try_warps(const DeviceGraph *G, uint32_t total) const {
     if (!G->rows_match) return false;
     auto it = warp_stats_.find(G->tune_class());
-    if (it == warp_stats_.end()) return true;
+    if (it == warp_stats_.end() || it->second.skipped >= kWarpRetry) return true;
     return (total <= 2 * slots_.slots ? 8 : 2) * it->second.left <= it->second.drawn;
 }
 
@@ -836,6 +838,9 @@ int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> 
     RK(ensure_segs((uint32_t)idx.size()));
     uint32_t all = 0;
     for (uint32_t i : idx) all += reqs[i].count;
+    // decided once: a redrawn round tries what its first draw tried
+    std::vector<uint8_t> tried(jobs.size());
+    for (uint32_t i : idx) tried[i] = try_warps(jobs[i]->graph(), all);
     auto fill = [&](uint32_t s, uint32_t j, uint32_t base) {
         Job *job = jobs[j];
         const JobRequest &r = reqs[j];
@@ -859,7 +864,7 @@ int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> 
             const uint32_t ai = job->params().assist_items;
             S.assist_items = ai == 0u ? kAssistItemsAuto : (ai == 0xffffffffu ? 0u : ai);
         }
-        S.compact = !try_warps(&G, all) ? 0u : kCompactOn | (G.directed ? 0u : kCompactWindow);
+        S.compact = !tried[j] ? 0u : kCompactOn | (G.directed ? 0u : kCompactWindow);
         S.left = d_cursors_ + max_segs_ + s;
         S.first_sample = r.first_global;
         S.count = r.count;
@@ -901,7 +906,7 @@ int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> 
     // asks for levels of the CTA sampler.
     bool warp = false;
     if (warps_.warps > 0 && jobs[idx[0]]->params().form != SILVAN_FORM_PLAIN) {
-        for (uint32_t i : idx) warp = warp || try_warps(jobs[i]->graph(), all);
+        for (uint32_t i : idx) warp = warp || tried[i];
         for (uint32_t i : idx) {
             const uint32_t ai = jobs[i]->params().assist_items;
             if (ai != 0u && ai != 0xffffffffu) warp = false;
@@ -1009,7 +1014,7 @@ int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> 
             for (uint32_t s = 0; s < idx.size(); s++)
                 if (h_segs_[s].compact)
                     warp_stats_[jobs[idx[s]]->graph()->tune_class()] =
-                        WarpStats{reqs[idx[s]].count, h_cursors_[max_segs_ + s]};
+                        WarpStats{reqs[idx[s]].count, h_cursors_[max_segs_ + s], 0};
         bool redo = false;
         uint32_t base = 0;
         for (uint32_t s = 0; s < idx.size(); s++) {
@@ -1038,6 +1043,10 @@ int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> 
         h_hdr_->cycles = 0;
         h_hdr_->max_cycles = 0;
         h_hdr_->wait_polls = polls;
+    }
+    for (uint32_t i : idx) {
+        auto it = warp_stats_.find(jobs[i]->graph()->tune_class());
+        if (!tried[i] && it != warp_stats_.end()) it->second.skipped++;
     }
     for (uint32_t s = 0; s < idx.size(); s++) records[idx[s]] = h_cursors_[s];
     return SILVAN_OK;

@@ -219,10 +219,13 @@ class Engine {
         uint32_t rounds = 0;
     };
     // Samples of a class of graphs that went through the warp sampler, and those
-    // it left to the CTA sampler, in the last such launch.
+    // it left to the CTA sampler, in the last such launch, and the launches since
+    // that did not try it.
     struct WarpStats {
         uint64_t drawn = 0, left = 0;
+        uint32_t skipped = 0;
     };
+    static constexpr uint32_t kWarpRetry = 64;
     bool try_warps(const DeviceGraph *G, uint32_t total) const;
     struct Exec {
         int block;

@@ -1,8 +1,8 @@
 """When the warps are tried.  A lattice whose samples they left does not rule them
-out for a short graph of the same size and degree (both to a power of two).  Each
-test has an engine of its own by a slot count that no other test asks for; results
-do not depend on the choice (Sp_sampler::random_path,
-silvan/src/Sp_sampler.cpp:41-238)."""
+out for a short graph of the same size and degree (both to a power of two), nor for
+its own kind for good: after 64 launches they are tried again.  Each test has an
+engine of its own by a slot count that no other test asks for; results do not
+depend on the choice (Sp_sampler::random_path, silvan/src/Sp_sampler.cpp:41-238)."""
 import pytest
 
 from test_gpu_modes import assert_same_run
@@ -34,3 +34,15 @@ def test_a_lattice_leaves_the_warps_to_short_graphs_of_its_class(sb, port, latti
     job, res = run(sb, sb.Graph.from_host(hg), 0.02, 7, 26)
     assert job.sampler_info()["warp_tried"] > 0
     assert_same_run(job, res, port_graph(port, csr).run(csr.diameter, 0.02, 0.1, seed=7))
+
+
+def test_left_out_graphs_are_tried_again(sb, lattice):
+    tried, launches = [], []
+    for seed in range(80):
+        job, res = run(sb, lattice, 0.2, seed, 27, **ONE_PATH)
+        tried.append(job.sampler_info()["warp_tried"] > 0)
+        launches.append(res["sampler_launches"])
+        if tried[1:].count(True):
+            break
+    assert tried[0] and tried[-1]
+    assert sum(launches[1:-1]) <= 64 <= sum(launches)
