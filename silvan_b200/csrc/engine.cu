@@ -769,9 +769,15 @@ void Engine::fair_share(const std::vector<Job *> &jobs, std::vector<JobRequest> 
     std::vector<double> cost(n, 0.0);
     uint32_t grid = 0;
     for (int b = 0; b < kNB; b++) grid = std::max(grid, max_grid_[b]);
+    // measured in rounds that used the warps as this one will, else in the others
+    uint32_t total = 0;
+    for (const JobRequest &r : reqs) total += r.count;
+    bool warp = false;
+    for (size_t i = 0; i < n && warps_.warps > 0; i++)
+        warp = warp || (reqs[i].count > 0 && try_warps(jobs[i]->graph(), total));
     for (size_t i = 0; i < n; i++) {
-        auto it = stats_.find(stats_key(jobs[i]->graph(), true));
-        if (it == stats_.end()) it = stats_.find(stats_key(jobs[i]->graph(), false));
+        auto it = stats_.find(stats_key(jobs[i]->graph(), warp));
+        if (it == stats_.end()) it = stats_.find(stats_key(jobs[i]->graph(), !warp));
         if (it == stats_.end()) return;
         double best = 0;
         for (int b = 0; b < kNB; b++) {
