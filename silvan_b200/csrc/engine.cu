@@ -43,7 +43,8 @@ constexpr uint32_t kUncertainCap = 1u << 16;
 // freed block is reusable only after a device synchronisation (the one
 // cudaFree would have done), taken when a request finds no ready block but
 // freed ones are waiting.  On allocation failure the cached blocks of the
-// device are released and the allocation is tried once more.
+// device are released and the allocation is tried once more, then the idle
+// engines of the pool.
 class BlockCache {
   public:
     void *alloc(size_t bytes, bool host, cudaError_t *err) {
@@ -71,19 +72,20 @@ class BlockCache {
             }
         }
         void *p = nullptr;
-        {
+        const auto get = [&]() {
             std::lock_guard<std::mutex> cl(capture_mutex());
             *err = host ? cudaMallocHost(&p, cls) : cudaMalloc(&p, cls);
-        }
-        if (*err != cudaSuccess) {
-            cudaGetLastError();
+            if (*err != cudaSuccess) cudaGetLastError();
+            return *err == cudaSuccess;
+        };
+        if (!get()) {
             release(dev);
-            std::lock_guard<std::mutex> cl(capture_mutex());
-            *err = host ? cudaMallocHost(&p, cls) : cudaMalloc(&p, cls);
-            if (*err != cudaSuccess) {
-                cudaGetLastError();
-                return nullptr;
+            bool ok = get();
+            if (!ok && !host && engines_trim(dev)) {
+                release(dev);
+                ok = get();
             }
+            if (!ok) return nullptr;
         }
         std::lock_guard<std::mutex> lk(mu_);
         live_[p] = key;
@@ -199,6 +201,18 @@ int device_alloc(void **p, size_t bytes) {
 }
 
 void device_free(void *p) { block_cache().free(p); }
+
+namespace {
+// Free device memory, counting the blocks this process freed and keeps for reuse
+// (an engine created after another one would otherwise see half of the previous
+// budget, and so on).
+cudaError_t free_bytes(int dev, uint64_t *bytes) {
+    size_t fr = 0, tot = 0;
+    const cudaError_t e = cudaMemGetInfo(&fr, &tot);
+    if (e == cudaSuccess) *bytes = fr + block_cache().idle_bytes(dev);
+    return e;
+}
+}  // namespace
 
 void set_error(const std::string &msg) { g_err = msg; }
 const char *last_error_cstr() { return g_err.c_str(); }
@@ -586,6 +600,11 @@ Engine::~Engine() {
     if (stream_) cudaStreamDestroy(stream_);
 }
 
+uint64_t Engine::device_bytes() const {
+    return slots_.slots * SlotPool::bytes_per_slot(slots_.n) +
+           (warps_.own ? WarpPool::bytes(warps_.warps, warps_.s.cap) : 0);
+}
+
 int Engine::init(uint64_t n_max, uint32_t slots, uint64_t mem_budget) {
     CK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
     {
@@ -608,19 +627,20 @@ int Engine::init(uint64_t n_max, uint32_t slots, uint64_t mem_budget) {
         most = std::max(most, resident[b]);
     }
     if (slots == 0) slots = std::max<uint32_t>(most, 1);
+    const uint64_t per_slot = std::max<uint64_t>(SlotPool::bytes_per_slot(n_max), 1);
     if (mem_budget == 0) {
-        // half of the free memory, counting the blocks this process freed
-        // and keeps for reuse (an engine created after another one would
-        // otherwise see half of the previous budget, and so on)
-        size_t fr = 0, tot = 0;
+        // half of the free memory; where that bounds the slots, the pool's idle
+        // engines give way (what a batch of large graphs took would otherwise
+        // halve a server that is started after it)
         int dev = 0;
+        uint64_t bytes = 0;
         CK(cudaGetDevice(&dev));
-        CK(cudaMemGetInfo(&fr, &tot));
-        mem_budget = (fr + block_cache().idle_bytes(dev)) / 2;
+        CK(free_bytes(dev, &bytes));
+        if (bytes / 2 / per_slot < slots && engines_trim(dev)) CK(free_bytes(dev, &bytes));
+        mem_budget = bytes / 2;
     }
     // the slots first, then the warp sampler's state in what they leave, at most
     // an eighth of the budget
-    const uint64_t per_slot = std::max<uint64_t>(SlotPool::bytes_per_slot(n_max), 1);
     const uint64_t fit = mem_budget / per_slot;
     if (fit < slots) slots = (uint32_t)std::max<uint64_t>(fit, 1);
     RK(slots_.alloc(slots, n_max, stream_));
@@ -1143,66 +1163,96 @@ struct PooledEngine {
 std::mutex g_pool_mu;
 std::vector<PooledEngine> g_pool_free;
 std::vector<PooledEngine> g_pool_busy;
+
+// Takes the idle engines of a device that `pick` chooses out of the pool.
+template <typename F>
+std::vector<PooledEngine> take_idle(int dev, F pick) {
+    std::vector<PooledEngine> out;
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    for (size_t i = 0; i < g_pool_free.size();)
+        if (g_pool_free[i].device == dev && pick(g_pool_free[i])) {
+            out.push_back(g_pool_free[i]);
+            g_pool_free.erase(g_pool_free.begin() + i);
+        } else {
+            i++;
+        }
+    return out;
+}
+
+// More slots first (a larger engine may hold fewer), then fewer nodes.
+bool better_fit(const PooledEngine &a, const PooledEngine &b) {
+    return a.eng->slots() != b.eng->slots() ? a.eng->slots() > b.eng->slots()
+                                            : a.eng->n_max() < b.eng->n_max();
+}
 }  // namespace
 
+bool engines_trim(int device) {
+    const std::vector<PooledEngine> idle = take_idle(device, [](const PooledEngine &) {
+        return true;
+    });
+    for (const PooledEngine &p : idle) delete p.eng;
+    return !idle.empty();
+}
+
+// Idle engines for smaller graphs make room for a new one, which serves their
+// requests too and starts from what they have measured.  One of them stays where
+// memory leaves the new one fewer slots and it is small beside what is free:
+// small graphs go on with all the slots that the GPU can run.
 Engine *engine_acquire(uint64_t n, uint32_t slots, int *rc) {
     int dev = 0;
     cudaGetDevice(&dev);
     {
         std::lock_guard<std::mutex> lk(g_pool_mu);
+        size_t best = g_pool_free.size();
         for (size_t i = 0; i < g_pool_free.size(); i++) {
-            PooledEngine &p = g_pool_free[i];
-            if (p.device == dev && p.eng->n_max() >= n && p.requested_slots == slots) {
-                PooledEngine q = p;
-                g_pool_free.erase(g_pool_free.begin() + i);
-                g_pool_busy.push_back(q);
-                *rc = SILVAN_OK;
-                return q.eng;
-            }
+            const PooledEngine &p = g_pool_free[i];
+            if (p.device == dev && p.eng->n_max() >= n && p.requested_slots == slots &&
+                (best == g_pool_free.size() || better_fit(p, g_pool_free[best])))
+                best = i;
+        }
+        if (best < g_pool_free.size()) {
+            const PooledEngine q = g_pool_free[best];
+            g_pool_free.erase(g_pool_free.begin() + best);
+            g_pool_busy.push_back(q);
+            *rc = SILVAN_OK;
+            return q.eng;
         }
     }
-    // Idle engines for smaller graphs make room for the new one, which serves
-    // their requests too and takes over what they have measured.
-    std::vector<Engine *> old;
-    {
-        std::lock_guard<std::mutex> lk(g_pool_mu);
-        for (size_t i = 0; i < g_pool_free.size();)
-            if (g_pool_free[i].device == dev && g_pool_free[i].requested_slots == slots) {
-                old.push_back(g_pool_free[i].eng);
-                g_pool_free.erase(g_pool_free.begin() + i);
-            } else {
-                i++;
-            }
-    }
+    std::vector<PooledEngine> old = take_idle(dev, [&](const PooledEngine &p) {
+        return p.requested_slots == slots;
+    });
     Engine *e = new Engine();
-    for (Engine *o : old) {
-        e->adopt(*o);
-        delete o;
+    for (const PooledEngine &p : old) e->adopt(*p.eng);
+    PooledEngine stay{};
+    uint64_t bytes = 0;
+    if (!old.empty() && free_bytes(dev, &bytes) == cudaSuccess) {
+        const PooledEngine &p = *std::max_element(
+            old.begin(), old.end(), [](const PooledEngine &a, const PooledEngine &b) {
+                return std::make_pair(a.eng->slots(), a.eng->n_max()) <
+                       std::make_pair(b.eng->slots(), b.eng->n_max());
+            });
+        if (p.eng->device_bytes() <= bytes / 8) stay = p;
     }
+    for (const PooledEngine &p : old)
+        if (p.eng != stay.eng) delete p.eng;
     *rc = e->init(n, slots, 0);
-    if (*rc != SILVAN_OK) {
-        // release idle engines of this device and try once more
-        std::vector<Engine *> drop;
-        {
-            std::lock_guard<std::mutex> lk(g_pool_mu);
-            for (size_t i = 0; i < g_pool_free.size();)
-                if (g_pool_free[i].device == dev) {
-                    drop.push_back(g_pool_free[i].eng);
-                    g_pool_free.erase(g_pool_free.begin() + i);
-                } else {
-                    i++;
-                }
-        }
-        for (Engine *d : drop) delete d;
+    if (*rc != SILVAN_OK && stay.eng) {  // once more without it
         delete e;
+        delete stay.eng;
+        stay.eng = nullptr;
         e = new Engine();
         *rc = e->init(n, slots, 0);
-        if (*rc != SILVAN_OK) {
-            delete e;
-            return nullptr;
-        }
+    }
+    if (*rc != SILVAN_OK) {
+        delete e;
+        return nullptr;
+    }
+    if (stay.eng && stay.eng->slots() <= e->slots()) {
+        delete stay.eng;
+        stay.eng = nullptr;
     }
     std::lock_guard<std::mutex> lk(g_pool_mu);
+    if (stay.eng) g_pool_free.push_back(stay);
     g_pool_busy.push_back(PooledEngine{dev, slots, e});
     return e;
 }

@@ -151,6 +151,8 @@ class Engine;
 // run, so repeated jobs do not re-allocate and re-initialise the slots.
 Engine *engine_acquire(uint64_t n, uint32_t slots, int *rc);
 void engine_release(Engine *e);
+// Gives back what the device's idle engines hold; whether there were any.
+bool engines_trim(int device);
 
 class Engine {
   public:
@@ -177,13 +179,15 @@ class Engine {
     // used, when its second pass kept alpha (0: none recorded)
     uint64_t job_hint(const DeviceGraph *G, const silvan_params_t &p) const;
     void note_job(const DeviceGraph *G, const silvan_params_t &p, uint64_t used, bool alpha_kept);
-    // takes over another engine's measurements of graph classes and job kinds
-    void adopt(Engine &o) {
-        stats_.merge(o.stats_);
-        last_.merge(o.last_);
-        warp_stats_.merge(o.warp_stats_);
-        job_total_.merge(o.job_total_);
+    // starts from another engine's measurements of graph classes and job kinds
+    void adopt(const Engine &o) {
+        stats_.insert(o.stats_.begin(), o.stats_.end());
+        last_.insert(o.last_.begin(), o.last_.end());
+        warp_stats_.insert(o.warp_stats_.begin(), o.warp_stats_.end());
+        job_total_.insert(o.job_total_.begin(), o.job_total_.end());
     }
+    // the device memory of the slots and the warps
+    uint64_t device_bytes() const;
     static uint64_t job_kind(const DeviceGraph *G, const silvan_params_t &p);
     uint64_t launches() const { return launches_; }
     float sample_ms() const { return sample_ms_; }
