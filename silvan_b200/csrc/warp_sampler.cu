@@ -28,8 +28,8 @@
 // Why one warp.  The CTA sampler pays about 25 us for a sample of a hundred
 // entries (8 CTAs of 128 threads an SM): five barriers and as many dependent
 // trips to L2 a level, most of its warps waiting.  Here a level costs two
-// trips (rows, adjacency) and no barrier, and 22 samples run on an SM.  One
-// B200, sampler time of a run with 22 warps an SM against the CTA sampler alone:
+// trips (rows, adjacency) and no barrier, and 21 samples run on an SM.  One
+// B200, sampler time of a run with 21 warps an SM against the CTA sampler alone:
 // 2.3 k samples on a Barabasi-Albert graph of 600 nodes 0.06 ms, before 0.11;
 // 14 k on one of 10 k nodes 0.43 ms, before 0.82; 263 k on R-MAT 14 9.6 ms,
 // before 10.3.  It is bound by instruction issue (0.3 a cycle and scheduler with
@@ -47,9 +47,11 @@ namespace silvan {
 namespace {
 
 // Table entries of a warp: the resident warps of an SM share its shared memory.
-// 1024 entries (10 KB, 22 warps an SM) draw R-MAT 14 samples faster than 2048
+// 1024 entries (10 KB, 21 warps an SM) draw R-MAT 14 samples faster than 2048
 // (18 KB, 12 warps, 5 % longer, sampler time of a top-10 run) and 4096 (7 %).
-constexpr int kWarpTable = 1024;
+constexpr uint32_t kWarpTable = 1024;
+// The warps of an SM that the registers allow for; shared memory holds 21 of them.
+constexpr int kWarpsPerSm = 22;
 constexpr int kMaxProbe = 32;  // buckets looked at for one node
 constexpr uint32_t kNoKey = 0xffffffffu;
 // A table value: kSettled | (side V ? kSettledV : 0) | queue position; below
@@ -62,16 +64,15 @@ constexpr uint32_t kNearTouched = 128;  // path-map positions kept in shared mem
 constexpr uint32_t kWarpPaths = 2048;  // paths of a sample drawn here
 constexpr uint32_t kScreenMax = 32;   // samples screened at once, one lane each
 
-// T table entries, in buckets of four keys (one 16-byte load).
-template <int T>
+constexpr uint32_t kBuckets = kWarpTable / 4;       // of four keys (one 16-byte load)
+constexpr uint32_t kTableLimit = kWarpTable * 3 / 4;  // entries in use
+// A frontier of more adjacency entries than this is left to the CTA sampler at
+// once: its nodes would not fit the table.
+constexpr uint32_t kFrontierItems = 4 * kWarpTable;
+
 struct WarpSmem {
-    static constexpr uint32_t kBuckets = T / 4;
-    static constexpr uint32_t kLimit = T * 3 / 4;  // entries in use
-    // A frontier of more adjacency entries than this is left to the CTA
-    // sampler at once: its nodes would not fit the table.
-    static constexpr uint32_t kItems = 4 * T;
-    uint4 key[T / 4];
-    uint32_t val[T];
+    uint4 key[kBuckets];
+    uint32_t val[kWarpTable];
     unsigned long long mpre[kNearMeets];
     uint2 meet[kNearMeets];
     uint32_t touched[kNearTouched];
@@ -107,11 +108,10 @@ struct View {
 // bucket together, without branches on single lanes: false when some lane has
 // not found its place after kMaxProbe looks.  The values are read after the
 // warp has come together again.
-template <int T>
-__device__ __forceinline__ bool table_slots(WarpSmem<T> &s, uint32_t y, bool act, uint32_t &h,
+__device__ __forceinline__ bool table_slots(WarpSmem &s, uint32_t y, bool act, uint32_t &h,
                                             bool &won) {
-    constexpr int kShift = T == 512 ? 25 : T == 1024 ? 24 : T == 2048 ? 23 : 22;
-    static_assert((1u << (32 - kShift)) == WarpSmem<T>::kBuckets, "table size");
+    constexpr int kShift = 24;
+    static_assert((1u << (32 - kShift)) == kBuckets, "table size");
     uint32_t b = (y * 2654435769u) >> kShift;
     uint32_t *keys = reinterpret_cast<uint32_t *>(s.key);
     won = false;
@@ -131,18 +131,17 @@ __device__ __forceinline__ bool table_slots(WarpSmem<T> &s, uint32_t y, bool act
         won = won || mine;
         const bool there = act && to < 4u && (at < 4u || o == kNoKey || o == y);
         if (there) h = 4u * b + to;
-        if (to == 4u) b = (b + 1u) & (WarpSmem<T>::kBuckets - 1u);
+        if (to == 4u) b = (b + 1u) & (kBuckets - 1u);
         act = act && !there;
         if (!__any_sync(kFull, act)) return true;
     }
     return false;
 }
 
-template <int T>
-__device__ __forceinline__ void table_clear(WarpSmem<T> &s) {
+__device__ __forceinline__ void table_clear(WarpSmem &s) {
     const uint4 e = make_uint4(kNoKey, kNoKey, kNoKey, kNoKey);
 #pragma unroll 4
-    for (uint32_t i = threadIdx.x & 31; i < WarpSmem<T>::kBuckets; i += 32) s.key[i] = e;
+    for (uint32_t i = threadIdx.x & 31; i < kBuckets; i += 32) s.key[i] = e;
 }
 
 template <typename T>
@@ -161,7 +160,7 @@ struct Found {
     uint32_t nmeet;   // meeting edges (0: the ends are not connected)
     uint32_t end;     // visited nodes
     uint32_t hits;    // predecessor entries
-    uint32_t vis;     // adjacency entries scanned (below 2^32: kWarpItems a level)
+    uint32_t vis;     // adjacency entries scanned (below 2^32: kFrontierItems a level)
     uint32_t depth;   // level of the first end of a meeting edge
     uint32_t wide;    // adjacency entries of the larger frontier, when it does not fit
     bool fits;        // false: the CTA sampler has to draw this sample
@@ -169,8 +168,7 @@ struct Found {
 
 // The balanced bidirectional BFS (silvan/src/Sp_sampler.cpp:89-144) between
 // u and v, whose rows (out of u, into v) are row_u and row_v.
-template <int T>
-__device__ __forceinline__ Found search(const SegDesc &A, WarpSmem<T> &s, const View &W,
+__device__ __forceinline__ Found search(const SegDesc &A, WarpSmem &s, const View &W,
                                         uint32_t u, uint32_t v, uint2 row_u, uint2 row_v) {
     const uint32_t lane = threadIdx.x & 31;
     const uint2 *rows_u = A.out_rows, *rows_v = A.in_rows;
@@ -204,11 +202,11 @@ __device__ __forceinline__ Found search(const SegDesc &A, WarpSmem<T> &s, const 
             depth ? (side_u ? sum_u : sum_v)
                   : (side_u ? row_u.y - row_u.x : row_v.y - row_v.x);
         f.wide = max(max(sum_u, sum_v), items);
-        if (items > WarpSmem<T>::kItems || depth + 2u >= kWarpLevels) {
+        if (items > kFrontierItems || depth + 2u >= kWarpLevels) {
             f.fits = false;
             return f;
         }
-        if (window && keys > (uint32_t)T / 2u) {
+        if (window && keys > kWarpTable / 2u) {
             // forget all but the last two levels of either side
             uint2 prev = make_uint2(0u, 0u);
             const uint32_t pd = lane ? depth_v : depth_u;
@@ -216,7 +214,7 @@ __device__ __forceinline__ Found search(const SegDesc &A, WarpSmem<T> &s, const 
             const uint32_t pu0 = __shfl_sync(kFull, prev.x, 0), pu1 = __shfl_sync(kFull, prev.y, 0);
             const uint32_t pv0 = __shfl_sync(kFull, prev.x, 1), pv1 = __shfl_sync(kFull, prev.y, 1);
             const uint32_t live = (hi_u - lo_u) + (hi_v - lo_v) + (pu1 - pu0) + (pv1 - pv0);
-            if (live <= (uint32_t)T / 2u) {
+            if (live <= kWarpTable / 2u) {
                 keys = live;
                 table_clear(s);
                 __syncwarp();
@@ -311,7 +309,7 @@ __device__ __forceinline__ Found search(const SegDesc &A, WarpSmem<T> &s, const 
                 }
                 const uint32_t J = __popc(jm);
                 keys += J;
-                if (!placed || keys > WarpSmem<T>::kLimit || end + J > W.cap) {
+                if (!placed || keys > kTableLimit || end + J > W.cap) {
                     f.fits = false;
                     return f;
                 }
@@ -442,8 +440,7 @@ __device__ uint32_t ranked_pred(const SegDesc &A, const View &W, uint32_t a, uin
 
 // Draws one sample and writes its outputs; false: left to the CTA sampler,
 // with nothing written.
-template <int T>
-__device__ __forceinline__ bool draw_sample(const SegDesc &A, WarpSmem<T> &s, const View &W,
+__device__ __forceinline__ bool draw_sample(const SegDesc &A, WarpSmem &s, const View &W,
                                             uint32_t sl, uint32_t u, uint32_t v,
                                             uint32_t draw_base, uint2 row_u, uint2 row_v,
                                             uint32_t &wide) {
@@ -645,9 +642,8 @@ __device__ __forceinline__ bool draw_sample(const SegDesc &A, WarpSmem<T> &s, co
     return true;
 }
 
-template <int T>
-__global__ void __launch_bounds__(32, 22528 / T) warp_sampler_kernel(WarpLaunch L) {
-    __shared__ WarpSmem<T> s;
+__global__ void __launch_bounds__(32, kWarpsPerSm) warp_sampler_kernel(WarpLaunch L) {
+    __shared__ WarpSmem s;
     const uint32_t lane = threadIdx.x;
     const uint64_t slot = blockIdx.x;
     const View W{L.slots.ball + slot * L.slots.cap,    L.slots.rows + slot * L.slots.cap,
@@ -730,13 +726,13 @@ __global__ void __launch_bounds__(32, 22528 / T) warp_sampler_kernel(WarpLaunch 
 
 cudaError_t warp_sampler_launch(const WarpLaunch &L, uint32_t grid, cudaStream_t stream) {
     if (grid == 0) return cudaSuccess;
-    warp_sampler_kernel<kWarpTable><<<grid, 32, 0, stream>>>(L);
+    warp_sampler_kernel<<<grid, 32, 0, stream>>>(L);
     return cudaGetLastError();
 }
 
 int warp_sampler_per_sm() {
     int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, warp_sampler_kernel<kWarpTable>, 32, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, warp_sampler_kernel, 32, 0);
     return n;
 }
 
