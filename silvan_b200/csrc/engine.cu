@@ -739,6 +739,12 @@ int Engine::choose_block(const std::vector<Job *> &jobs, const std::vector<JobRe
     if (p0.block) return (int)p0.block;
     if (p0.form == SILVAN_FORM_PLAIN) return kSamplerBlock;
     static const int order[kNB] = {2, 1, 0, 3};  // 512, 256, 128, 1024
+    if (!warp && idx.size() == 1) {  // first without the warps: the size that is best with them
+        auto w = warp_stats_.find(jobs[idx[0]]->graph()->tune_class());
+        if (w != warp_stats_.end() && w->second.cost[0].samples == 0 &&
+            w->second.cost[1].samples)
+            return kSamplerBlocks[w->second.cost[1].size];
+    }
     for (int oi = 0; oi < kNB; oi++) {
         const int b = order[oi];
         if (!max_grid_[b]) continue;
@@ -772,14 +778,33 @@ int Engine::choose_block(const std::vector<Job *> &jobs, const std::vector<JobRe
 // round of a few samples per CTA not when more than an eighth was left: such a
 // round lasts as long as its slowest samples, and these would wait for the warps
 // first (23,000 random nodes, 2,100 samples in two rounds: 0.37 ms with the warps,
-// 0.23 without).  A class that is left out is tried again after kWarpRetry
-// launches of its graphs: its next graph may be another one, and a lattice loses a
-// quarter of a percent by it.
-bool Engine::try_warps(const DeviceGraph *G, uint32_t total) const {
+// 0.23 without).  Between the two, where the warps leave more than a 64th, what
+// they leave does not say whether trying pays: of undirected R-MAT 18 they leave
+// 34 % and save 10 % of a run (the long samples are known then and start first),
+// of a 120 x 120 lattice 39 % and lose 18 %.  There one launch goes without them,
+// and they are left out while that is a tenth faster than the best with them (the
+// tails of single launches differ by as much).  A class that is left out is
+// tried again after kWarpRetry launches of its graphs: its next graph may be
+// another one, and a lattice loses a quarter of a percent by it.
+bool Engine::try_warps(const DeviceGraph *G, uint32_t total, bool one_job) const {
     if (!G->rows_match) return false;
     auto it = warp_stats_.find(G->tune_class());
-    if (it == warp_stats_.end() || it->second.skipped >= kWarpRetry) return true;
-    return (total <= 2 * slots_.slots ? 8 : 2) * it->second.left <= it->second.drawn;
+    if (it == warp_stats_.end()) return true;
+    const WarpStats &w = it->second;
+    if (w.skipped >= kWarpRetry) return true;
+    if ((total <= 2 * slots_.slots ? 8 : 2) * w.left > w.drawn) return false;
+    if (64 * w.left <= w.drawn || w.cost[1].samples == 0) return true;
+    if (w.cost[0].samples == 0) return !one_job || !sizes_tried(G, true);
+    return !w.cost[0].faster(w.cost[1], 1.1);
+}
+
+// Whether every CTA size has been measured on the class of G.
+bool Engine::sizes_tried(const DeviceGraph *G, bool warp) const {
+    auto it = stats_.find(stats_key(G, warp));
+    if (it == stats_.end()) return false;
+    for (int b = 0; b < kNB; b++)
+        if (max_grid_[b] && it->second[b].rounds == 0) return false;
+    return true;
 }
 
 void Engine::fair_share(const std::vector<Job *> &jobs, std::vector<JobRequest> &reqs,
@@ -794,7 +819,7 @@ void Engine::fair_share(const std::vector<Job *> &jobs, std::vector<JobRequest> 
     for (const JobRequest &r : reqs) total += r.count;
     bool warp = false;
     for (size_t i = 0; i < n && warps_.warps > 0; i++)
-        warp = warp || (reqs[i].count > 0 && try_warps(jobs[i]->graph(), total));
+        warp = warp || (reqs[i].count > 0 && try_warps(jobs[i]->graph(), total, false));
     for (size_t i = 0; i < n; i++) {
         auto it = stats_.find(stats_key(jobs[i]->graph(), warp));
         if (it == stats_.end()) it = stats_.find(stats_key(jobs[i]->graph(), !warp));
@@ -866,7 +891,7 @@ int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> 
     for (uint32_t i : idx) all += reqs[i].count;
     // decided once: a redrawn round tries what its first draw tried
     std::vector<uint8_t> tried(jobs.size());
-    for (uint32_t i : idx) tried[i] = try_warps(jobs[i]->graph(), all);
+    for (uint32_t i : idx) tried[i] = try_warps(jobs[i]->graph(), all, idx.size() == 1);
     auto fill = [&](uint32_t s, uint32_t j, uint32_t base) {
         Job *job = jobs[j];
         const JobRequest &r = reqs[j];
@@ -1029,18 +1054,31 @@ int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> 
                 // the slowest sample of a launch grows with the launch's size
                 // and is rare: the estimate follows a longer tail at once and
                 // a shorter one slowly
+                const bool settled = sizes_tried(jobs[i]->graph(), warp);  // before this launch
                 BlockStats &st = stats_[stats_key(jobs[i]->graph(), warp)][bi];
                 st.cta_ms = st.rounds ? 0.5 * (st.cta_ms + cta_ms) : cta_ms;
                 st.tail_ms = (!st.rounds || tail_ms > st.tail_ms) ? tail_ms
                                                                   : 0.75 * st.tail_ms + 0.25 * tail_ms;
                 st.rounds++;
+                const silvan_params_t &p = jobs[i]->params();
+                if (idx.size() > 1 || total <= 2 * slots_.slots ||
+                    p.form == SILVAN_FORM_PLAIN || p.block || p.assist_items)
+                    continue;
+                WarpStats::Cost &best = warp_stats_[jobs[i]->graph()->tune_class()].cost[warp];
+                WarpStats::Cost c{ms, total, bi};
+                const bool mean = !warp && settled;
+                if (mean && best.size == bi) c.ms = 0.5 * (best.ms * total / best.samples + ms);
+                if (mean || best.samples == 0 || c.faster(best, 1.0)) best = c;
             }
         }
         if (warp)
             for (uint32_t s = 0; s < idx.size(); s++)
-                if (h_segs_[s].compact)
-                    warp_stats_[jobs[idx[s]]->graph()->tune_class()] =
-                        WarpStats{reqs[idx[s]].count, h_cursors_[max_segs_ + s], 0};
+                if (h_segs_[s].compact) {
+                    WarpStats &w = warp_stats_[jobs[idx[s]]->graph()->tune_class()];
+                    w.drawn = reqs[idx[s]].count;
+                    w.left = h_cursors_[max_segs_ + s];
+                    w.skipped = 0;
+                }
         bool redo = false;
         uint32_t base = 0;
         for (uint32_t s = 0; s < idx.size(); s++) {

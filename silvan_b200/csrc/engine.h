@@ -228,9 +228,22 @@ class Engine {
     struct WarpStats {
         uint64_t drawn = 0, left = 0;
         uint32_t skipped = 0;
+        // launches of one job and many samples: without the warps under the CTA
+        // size in use, with them the best one so far
+        struct Cost {
+            double ms = 0;
+            uint32_t samples = 0;  // 0: not measured
+            int size = -1;         // index into kSamplerBlocks
+            // a launch of more samples lasts longer, of fewer longer per sample:
+            // a is faster for sure when it is so at its own number of samples
+            bool faster(const Cost &b, double by) const {
+                return by * ms * std::max(1.0, (double)b.samples / samples) < b.ms;
+            }
+        } cost[2];
     };
     static constexpr uint32_t kWarpRetry = 64;
-    bool try_warps(const DeviceGraph *G, uint32_t total) const;
+    bool try_warps(const DeviceGraph *G, uint32_t total, bool one_job) const;
+    bool sizes_tried(const DeviceGraph *G, bool warp) const;
     struct Exec {
         int block;
         uint32_t grid;

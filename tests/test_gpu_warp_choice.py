@@ -1,7 +1,8 @@
 """When the warps are tried.  A lattice whose samples they left does not rule them
 out for a short graph of the same size and degree (both to a power of two), nor for
-its own kind for good: after 64 launches they are tried again.  Each test has an
-engine of its own by a slot count that no other test asks for; results do not
+its own kind for good: after 64 launches they are tried again.  Where they leave
+some of the samples, what a launch takes with and without them decides.  Each test
+has an engine of its own by a slot count that no other test asks for; results do not
 depend on the choice (Sp_sampler::random_path, silvan/src/Sp_sampler.cpp:41-238)."""
 import pytest
 
@@ -46,3 +47,22 @@ def test_left_out_graphs_are_tried_again(sb, lattice):
             break
     assert tried[0] and tried[-1]
     assert sum(launches[1:-1]) <= 64 <= sum(launches)
+
+
+def test_the_time_decides_where_some_samples_are_left(sb, port):
+    """Of a 120 x 120 lattice the warps leave four samples in ten and cost a quarter
+    of the sampling; of 10,000 nodes of Barabasi-Albert one in fourteen, and without
+    them the sampling is half as long again."""
+    hg = sb.HostGraph.from_pairs(sb.grid(120, 0.05, 0.001, 1), False)
+    g, infos = sb.Graph.from_host(hg), []
+    for seed in range(14):
+        job, res = run(sb, g, 0.03, seed, 1183, **ONE_PATH)
+        infos.append(job.sampler_info())
+    assert 64 * infos[0]["warp_left"] > infos[0]["warp_tried"] > 2 * infos[0]["warp_left"]
+    assert [i["warp_tried"] for i in infos[-3:]] == [0, 0, 0]
+    csr = hg.csr()
+    assert_same_run(job, res, port_graph(port, csr).run(csr.diameter, 0.03, 0.1, seed=13,
+                                                        **ONE_PATH))
+    small = sb.Graph.from_pairs(sb.barabasi_albert(10000, 5, 1))
+    infos = [run(sb, small, 0.01, seed, 1183)[0].sampler_info() for seed in range(14)]
+    assert all(i["warp_tried"] > 0 for i in infos[-3:])
