@@ -1043,9 +1043,10 @@ int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> 
                 warp ? (double)h_hdr_->warp_cycles / clock_khz_ / warps_.warps : 0.0;
             const double cta_ms =
                 ((double)h_hdr_->cycles / clock_khz_ + warp_ms * grid) / h_hdr_->total;
-            // where warps draw most of a launch, drawing on meanwhile is not free (5,000
-            // random nodes: 5,200 samples drawn for 2,200 used, 0.28 ms of sampling)
-            const double slowest_ms = warp ? 0.0 : (double)h_hdr_->max_cycles / clock_khz_;
+            // where the warps take most of a launch, drawing on meanwhile is not free
+            // (5,000 random nodes: 5,200 samples drawn for 2,200 used, 0.28 ms of sampling)
+            const bool by_warps = (double)h_hdr_->cycles / clock_khz_ < warp_ms * grid;
+            const double slowest_ms = by_warps ? 0.0 : (double)h_hdr_->max_cycles / clock_khz_;
             const double tail_ms = (double)h_hdr_->max_cycles / clock_khz_ + warp_ms;
             for (uint32_t i : idx)
                 last_[jobs[i]->graph()->tune_class()] =

@@ -4,6 +4,7 @@ its own kind for good: after 64 launches they are tried again.  Where they leave
 some of the samples, what a launch takes with and without them decides.  Each test
 has an engine of its own by a slot count that no other test asks for; results do not
 depend on the choice (Sp_sampler::random_path, silvan/src/Sp_sampler.cpp:41-238)."""
+import numpy as np
 import pytest
 
 from test_gpu_modes import assert_same_run
@@ -66,3 +67,13 @@ def test_the_time_decides_where_some_samples_are_left(sb, port):
     small = sb.Graph.from_pairs(sb.barabasi_albert(10000, 5, 1))
     infos = [run(sb, small, 0.01, seed, 1183)[0].sampler_info() for seed in range(14)]
     assert all(i["warp_tried"] > 0 for i in infos[-3:])
+
+
+def test_draws_ahead_where_the_ctas_take_the_time(sb):
+    """Sparse directed random graphs: nearly all samples are void, and the others are
+    long ones of the CTA sampler's.  The slots that are free while the slowest is
+    drawn draw ahead, so that the first pass and the second take a launch each."""
+    pairs = np.random.RandomState(1).randint(0, 200000, (220000, 2)).astype(np.uint32)
+    g = sb.Graph.from_pairs(pairs, True)
+    res = [run(sb, g, 0.005, seed, 1182)[1] for seed in range(10)]
+    assert min(r["sampler_launches"] for r in res[-5:]) <= 2
