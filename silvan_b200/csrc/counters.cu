@@ -97,7 +97,8 @@ __device__ void bucket_count(const RoundBuffers &rb, const ApplyArgs &a) {
 // Bucket space of every touched node, taken from a cursor (the buckets need
 // no order among themselves): one atomic per warp for the warp's nodes, the
 // lanes' offsets by a warp scan.  The node's count becomes its scatter
-// cursor; buckets of more than 32 entries are listed for the CTA-wide fold.
+// cursor; buckets of more than 32 entries are listed for fold_large, of more than
+// kHugeBucket for order_huge.
 __device__ void bucket_alloc(const RoundBuffers &rb, uint32_t T) {
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
     const uint32_t lane = threadIdx.x & 31;

@@ -1121,7 +1121,7 @@ int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> 
 // same accuracy, confidence, mode and sampling rate.  The class alone is too
 // wide: a top-k job's 227,000 samples on a 384 x 384 lattice had the next
 // absolute job on a 511 x 511 one (the same class) draw 65,536 samples where
-// it uses 1,900: 158 ms, against 7 alone.
+// it uses 4,000: 158 ms, against 7 alone.
 uint64_t Engine::job_kind(const DeviceGraph *G, const silvan_params_t &p) {
     uint64_t h = G->tune_class();
     auto mix = [&](uint64_t v) {  // 64-bit FNV-1a over words, then a shift

@@ -12,20 +12,23 @@
 // predecessor lists are appended in scan order, and meeting edges are
 // collected in scan order.  Here the items of a level are numbered
 // g = 0, 1, ... in exactly that order and processed in tiles of ascending g:
-//   phase 1  every item reads the state of its neighbour y; every item that
-//            reaches a node of the new level (unvisited, or joined earlier in
-//            this level) records itself with atomicMin/atomicMax of
-//            (g << 32 | x) (the first and the last predecessor), a count and
-//            sigma += sigma(x) (a wrapping sum, order-free);
-//   phase 2  after a barrier the items whose g equals their node's minimum are
-//            the joining hits; they mark their node as visited and, with the
-//            meeting items, are compacted in g order (warp ballots plus one
-//            block scan), which appends new nodes to the queue and meeting
-//            edges to the list in the reference order.
-// A later tile can never lower a node's minimum below an earlier tile's g, so
-// each tile is final once its own phase 1 is done.  A wide level may instead
-// be expanded by several CTAs, tile by tile with the same numbering (the help
-// board, below).
+//   phase 1  every item reads the state of its neighbour y; the unvisited ones
+//            go through a table in shared memory that finds the lowest item of
+//            each node; nodes joined by an earlier tile have their record and
+//            take the hit there (count, last predecessor, sigma += sigma(x), a
+//            wrapping sum: order-free);
+//   phase 2  after a barrier the items found are the joining hits: they mark
+//            their node as visited, write its record with one store and, with
+//            the meeting items, are compacted in g order (warp ballots plus
+//            sums over the warps' counts), which appends new nodes to the queue
+//            and meeting edges to the list in the reference order; the tile's
+//            other hits on those nodes follow after a barrier.
+// A later tile can never lower a node's first item below an earlier tile's g, so
+// each tile is final once its own phase 1 is done.  Once a level has a meeting
+// edge it is the search's last, and its later tiles only mark and count
+// (last_tile).  A wide level may instead be expanded by several CTAs, tile by
+// tile with the same numbering (the help board, below): there the items of a
+// tile find their node's first and last by atomicMin/atomicMax on its record.
 //
 // The backtrack needs pred(y)[t] with t = min(r mod sigma(y), |pred(y)| - 1)
 // (Sp_sampler.cpp:241-265: the walk adds n_paths[v] == 1 per entry).  t == 0
