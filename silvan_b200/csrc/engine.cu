@@ -739,10 +739,12 @@ int Engine::choose_block(const std::vector<Job *> &jobs, const std::vector<JobRe
     if (p0.block) return (int)p0.block;
     if (p0.form == SILVAN_FORM_PLAIN) return kSamplerBlock;
     static const int order[kNB] = {2, 1, 0, 3};  // 512, 256, 128, 1024
-    if (!warp && idx.size() == 1) {  // first without the warps: the size that is best with them
-        auto w = warp_stats_.find(jobs[idx[0]]->graph()->tune_class());
-        if (w != warp_stats_.end() && w->second.cost[0].samples == 0 &&
-            w->second.cost[1].samples)
+    // a class measured with the warps: without them the size that was best with them
+    if (!warp && idx.size() == 1) {
+        const DeviceGraph *G = jobs[idx[0]]->graph();
+        auto w = warp_stats_.find(G->tune_class());
+        if (w != warp_stats_.end() && w->second.cost[1].samples && sizes_tried(G, true) &&
+            !sizes_tried(G, false))
             return kSamplerBlocks[w->second.cost[1].size];
     }
     for (int oi = 0; oi < kNB; oi++) {
@@ -782,8 +784,8 @@ int Engine::choose_block(const std::vector<Job *> &jobs, const std::vector<JobRe
 // they leave does not say whether trying pays: of undirected R-MAT 18 they leave
 // 34 % and save 10 % of a run (the long samples are known then and start first),
 // of a 120 x 120 lattice 39 % and lose 18 %.  There one launch goes without them,
-// and they are left out while that is a tenth faster than the best with them (the
-// tails of single launches differ by as much).  A class that is left out is
+// and they are left out while that is a tenth faster than the best of at least
+// kWarpSettled with them (single launches differ by as much).  A class that is left out is
 // tried again after kWarpRetry launches of its graphs: its next graph may be
 // another one, and a lattice loses a quarter of a percent by it.
 bool Engine::try_warps(const DeviceGraph *G, uint32_t total, bool one_job) const {
@@ -794,7 +796,7 @@ bool Engine::try_warps(const DeviceGraph *G, uint32_t total, bool one_job) const
     if (w.skipped >= kWarpRetry) return true;
     if ((total <= 2 * slots_.slots ? 8 : 2) * w.left > w.drawn) return false;
     if (64 * w.left <= w.drawn || w.cost[1].samples == 0) return true;
-    if (w.cost[0].samples == 0) return !one_job || !sizes_tried(G, true);
+    if (w.cost[0].samples == 0) return !one_job || w.settled < kWarpSettled;
     return !w.cost[0].faster(w.cost[1], 1.1);
 }
 
@@ -1065,11 +1067,12 @@ int Engine::round(const std::vector<Job *> &jobs, const std::vector<JobRequest> 
                 if (idx.size() > 1 || total <= 2 * slots_.slots ||
                     p.form == SILVAN_FORM_PLAIN || p.block || p.assist_items)
                     continue;
-                WarpStats::Cost &best = warp_stats_[jobs[i]->graph()->tune_class()].cost[warp];
+                WarpStats &w = warp_stats_[jobs[i]->graph()->tune_class()];
+                WarpStats::Cost &best = w.cost[warp];
                 WarpStats::Cost c{ms, total, bi};
-                const bool mean = !warp && settled;
-                if (mean && best.size == bi) c.ms = 0.5 * (best.ms * total / best.samples + ms);
-                if (mean || best.samples == 0 || c.faster(best, 1.0)) best = c;
+                if (warp && settled) w.settled++;
+                if (!warp && best.size == bi) c.ms = 0.5 * (best.ms * total / best.samples + ms);
+                if (!warp || best.samples == 0 || c.faster(best, 1.0)) best = c;
             }
         }
         if (warp)

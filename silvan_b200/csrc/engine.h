@@ -228,6 +228,7 @@ class Engine {
     struct WarpStats {
         uint64_t drawn = 0, left = 0;
         uint32_t skipped = 0;
+        uint32_t settled = 0;  // launches with them after every CTA size was tried
         // launches of one job and many samples: without the warps under the CTA
         // size in use, with them the best one so far
         struct Cost {
@@ -241,7 +242,7 @@ class Engine {
             }
         } cost[2];
     };
-    static constexpr uint32_t kWarpRetry = 64;
+    static constexpr uint32_t kWarpRetry = 64, kWarpSettled = 8;
     bool try_warps(const DeviceGraph *G, uint32_t total, bool one_job) const;
     bool sizes_tried(const DeviceGraph *G, bool warp) const;
     struct Exec {
