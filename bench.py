@@ -846,7 +846,7 @@ def main():
         t_samp = sum(r["time_sampling_s"] for r in results)
         achieved = alg / t_samp / 1e9 if t_samp > 0 else 0.0
         # DRAM bytes per launch: bytes per sample from an ncu capture of the
-        # same kernel on this workload (profiles/), times samples per launch
+        # samplers on this workload (profiles/), times samples per launch
         traffic = None
         tp = os.path.join(ROOT, "profiles", "sampler_traffic.json")
         if os.path.exists(tp):

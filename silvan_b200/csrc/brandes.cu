@@ -26,7 +26,7 @@
 // memory.  A row is scanned by as many lanes as the mean degree asks for, a
 // long one by its whole warp.  Barabasi-Albert graph of 10,000 nodes, 5 edges
 // per new node, one B200: 14.1 ms (with all of it in global memory and one thread a
-// node in the backward pass: 50.5 ms); issue slots 52 % busy, 24 edges a warp step.
+// node in the backward pass: 50.5 ms); issue slots 55 % busy.
 #include "brandes.h"
 
 #include <algorithm>

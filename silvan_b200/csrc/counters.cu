@@ -48,7 +48,7 @@ namespace {
 //
 // Once per draw, not per commit round: an estimation commits a draw in about
 // ten rounds, and the three barriers and their phases were more than half of
-// each (R-MAT 20, a million nodes: 14 of 31-35 us; a round is now 27 and the draw 55 once).
+// each (R-MAT 20, a million nodes: 14 of 31-35 us; a round is now 20 and the draw 66 once).
 // ---------------------------------------------------------------------------
 constexpr int kCommitThreads = 1024;
 

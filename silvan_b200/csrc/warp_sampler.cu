@@ -32,8 +32,10 @@
 // B200, sampler time of a run with 21 warps an SM against the CTA sampler alone:
 // 2.3 k samples on a Barabasi-Albert graph of 600 nodes 0.06 ms, before 0.11;
 // 14 k on one of 10 k nodes 0.43 ms, before 0.82; 263 k on R-MAT 14 9.6 ms,
-// before 10.3.  It is bound by instruction issue (0.3 a cycle and scheduler with
-// 3 warps; about 190 instructions per 32 entries), not by memory: DRAM 5 %.
+// before 10.3.  It is bound by instruction issue and latency, not by bandwidth: with
+// samples for all warps 0.54 instructions a cycle and scheduler, five warps on each,
+// an instruction waiting as long for the one before as for memory; DRAM 14 %
+// (R-MAT 16).
 // A CTA of four warps around the same table was slower than the general
 // search: its fixed cost per level is paid by every warp.
 #include <algorithm>
